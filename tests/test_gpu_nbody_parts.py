@@ -1,0 +1,76 @@
+"""The far-field N-body walkers over sheet parts against the FP64 oracle (B200).
+
+Sheets whose rows and columns leave remainders in every direction of a part
+(2, 4 or 6 node rows x 32 segment columns, up to 8 narrow parts per strip), at
+targets that are near, between near and far, and far, on nodes and along the
+extension of segments, where the reference's cut-off |r1 x r2|^2 < 1e-10
+decides.  Tolerances are those of the other N-body tests: FP64 1e-12 of
+max |v|; FP32 2e-5 of the local velocity + 1e-6 of max |v|.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1, 1), (1, 1, 33), (2, 3, 32), (1, 4, 65), (1, 7, 8), (5, 2, 3), (40, 1, 1), (1, 26, 31), (1, 13, 130)]
+
+
+def _sheet(num, rows, cols, seed, wobble):
+    rng = np.random.default_rng(seed)
+    x, y = np.meshgrid(0.15 * np.arange(rows + 1), 0.06 * np.arange(cols + 1), indexing="ij")
+    pos = np.stack([np.stack([x, y + 0.3 * n, 0.2 * n + 0 * x], -1) for n in range(num)])
+    return pos + wobble * rng.standard_normal(pos.shape), rng.standard_normal((num, rows, cols))
+
+
+def _targets(pos, seed):
+    """Nodes, points at every distance, and points along the extension of both kinds of segments at offsets on
+    both sides of the cut-off (|r1 x r2| = |r0| offset against 1e-5)."""
+    rng = np.random.default_rng(seed)
+    flat = pos.reshape(-1, 3)
+    d = rng.standard_normal((300, 3))
+    d *= (10.0 ** rng.uniform(-3, 1.5, 300) / np.linalg.norm(d, axis=1))[:, None]
+    out = [flat[rng.integers(0, len(flat), 64)], flat[rng.integers(0, len(flat), 300)] + d]
+    for a, b in ((pos[:, :-1], pos[:, 1:]), (pos[:, :, :-1], pos[:, :, 1:])):
+        a, b = a.reshape(-1, 3), b.reshape(-1, 3)
+        k = rng.integers(0, len(a), 120)
+        r0 = b[k] - a[k]
+        length = np.linalg.norm(r0, axis=1)
+        side = np.cross(r0, rng.standard_normal(r0.shape))
+        side /= np.linalg.norm(side, axis=1)[:, None]
+        away = rng.choice([-1.0, 1.0], 120) * 10.0 ** rng.uniform(-0.5, 1.3, 120)
+        factor = rng.choice([0.0, 0.5, 0.8, 1.25, 2.0, 100.0], 120)  # of the cut-off
+        out.append(b[k] + r0 / length[:, None] * away[:, None] + side * (factor * 1e-5 / length)[:, None])
+    return np.concatenate(out)
+
+
+@pytest.mark.parametrize("wobble", [0.0, 0.004])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_parts_match_oracle(shape, wobble):
+    import pyoracle as o
+
+    import uvlm_b200 as U
+
+    pos, gamma = _sheet(*shape, seed=sum(shape), wobble=wobble)
+    targets = _targets(pos, seed=7 + shape[1])
+    ref = o.sheet_induced_velocity(pos, gamma, targets)
+    scale, mag = np.max(np.abs(ref)), np.linalg.norm(ref, axis=1)
+    got = U.InducedVelocity(targets, pos, gamma)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * scale
+    got = U.InducedVelocity(targets, pos, gamma, precision="mixed")
+    assert np.all(np.abs(got - ref).max(axis=1) <= 2e-5 * mag + 1e-6 * scale)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_strengths_scale_exactly(precision):
+    """Powers of two of the circulations scale the velocities exactly, and zero circulations give zeros."""
+    import uvlm_b200 as U
+
+    pos, gamma = _sheet(1, 9, 40, seed=3, wobble=0.003)
+    t = _targets(pos, seed=4)
+    v = U.InducedVelocity(t, pos, gamma, precision)
+    for e in (-20, 10):
+        np.testing.assert_array_equal(U.InducedVelocity(t, pos, gamma * 2.0 ** e, precision), v * 2.0 ** e)
+    np.testing.assert_array_equal(U.InducedVelocity(t, pos, gamma * 0, precision), 0)
+    # circulations so small that their squares leave the FP32 range
+    small = U.InducedVelocity(t, pos, gamma * 2.0 ** -60, precision) * 2.0 ** 60
+    np.testing.assert_allclose(small, v, rtol=0, atol=(1e-12 if precision == "fp64" else 2e-5) * np.max(np.abs(v)))

@@ -105,10 +105,11 @@ struct uvlm_ctx {
   bool have_factors = false;
   bool refresh_next = false;  // refactor at the next solve (GMRES reached gmres_refresh_iter)
   // N-body tile variant per stage (kStageRhs, kStageLoads, kStageAdvect) and
-  // precision ([0] FP32, [1] FP64); defaults fp32_h3_t2_b128_x2f and
-  // fp64_h2_t1_b128_m3, each autotuned on that stage's first large evaluation
-  // unless the configuration pins one
-  int stage_variant[3][2] = {{16, 9}, {16, 9}, {16, 9}};
+  // precision ([0] FP32, [1] FP64), each autotuned on that stage's first large
+  // evaluation unless the configuration pins one
+  int stage_variant[3][2] = {{kDefaultVariantF32, kDefaultVariantF64},
+                             {kDefaultVariantF32, kDefaultVariantF64},
+                             {kDefaultVariantF32, kDefaultVariantF64}};
   bool stage_pinned[3][2] = {};        // the configuration chose the tile
   double stage_tuned_pairs[3][2] = {};  // pairs of the evaluation the tile was tuned on (0: not yet)
   // learned warm start: network (borrowed), per-step features, collected data
@@ -311,7 +312,7 @@ Error uvlm_ctx::eval(const SourceBlock* blocks, int nblocks, long long nt, NBody
     float best_ms = 1e30f;
     int best = chosen;
     for (int v = 0; v < nbody_num_variants(); ++v) {
-      if (nbody_variant_prec(v) != prec) continue;
+      if (nbody_variant_prec(v) != prec || !nbody_variant_far(v)) continue;
       if (prec == kNBodyFP32 && cfg.nbody_near_fp64 && !nbody_variant_near64(v)) continue;  // keep the FP64 near field
       float ms = 0;
       for (int rep = 0; rep < 2; ++rep) {

@@ -30,7 +30,8 @@
 // (= r1 x r2 of src/vortex.cpp:24-28) without the cancellation of two long,
 // nearly parallel vectors.  Sources are walked in "strips" of H owned node
 // rows x up to kStripCols node columns, staged through shared memory by
-// cp.async double buffering.
+// cp.async double buffering; the far-field walkers of nbody_parts.cuh walk parts
+// of a sheet instead.
 #pragma once
 
 #include "common.cuh"
@@ -198,6 +199,108 @@ __device__ inline StripInfo decode_strip(const Blocks& B, long long s) {
   return si;
 }
 
+// ------------------------------------------------------------ sheet parts
+// What the far-field walkers (nbody_parts.cuh) walk: a sheet is cut into parts
+// of H owned node rows (plus the row below) x at most kPartCols segment
+// columns, and a strip is a run of consecutive parts of one block.
+constexpr int kPartCols = 32;    // segment columns of a part at most
+constexpr int kStripSlots = 66;  // node columns of a strip at most (two full parts)
+constexpr int kMaxParts = 8;     // parts of a strip at most
+
+// Source blocks cut into parts and strips.
+struct PartBlocks {
+  SourceBlock b[4];
+  int n;
+  int chunks[4];  // parts per row group
+  int width[4];   // segment columns of a part (the last of a row group may have fewer)
+  int groups[4];  // row groups per sheet
+  int per[4];     // parts per strip
+  long long strip_begin[5];
+};
+
+// Fills B from the blocks that carry segments, H node rows per part and at
+// most max_parts parts per strip; returns the strip count.
+__host__ __device__ inline long long fill_parts(PartBlocks& B, const SourceBlock* blocks, int n_blocks, int H,
+                                                int max_parts) {
+  B.n = 0;
+  long long strips = 0;
+  for (int i = 0; i < n_blocks && B.n < 4; ++i) {
+    const SourceBlock& sb = blocks[i];
+    if (sb.num <= 0 || sb.node_rows < 2 || sb.cols <= 0) continue;  // no rings -> no segments
+    const int q = B.n++;
+    B.b[q] = sb;
+    B.chunks[q] = (sb.cols + kPartCols - 1) / kPartCols;
+    B.width[q] = (sb.cols + B.chunks[q] - 1) / B.chunks[q];
+    B.chunks[q] = (sb.cols + B.width[q] - 1) / B.width[q];
+    B.groups[q] = (sb.node_rows + H - 1) / H;
+    int per = kStripSlots / (B.width[q] + 1);
+    if (per > max_parts) per = max_parts;
+    if (per < 1) per = 1;
+    B.per[q] = per;
+    B.strip_begin[q] = strips;
+    const long long parts = (long long)sb.num * B.groups[q] * B.chunks[q];
+    strips += (parts + per - 1) / per;
+  }
+  B.strip_begin[B.n] = strips;
+  return strips;
+}
+
+// One part: its first node's record, its shape and what it owns.
+struct PartInfo {
+  long long first;  // record of node (i0, j0)
+  int stride;       // records per node row of the sheet
+  int nr;           // node rows present (owned rows and the one below them)
+  int nc;           // node columns
+  int last_h;       // owns the chordwise segments of its last column
+};
+
+// Parts of strip s; returns how many (0 past the last).
+template <int H>
+__device__ inline int decode_part(const PartBlocks& B, long long s, int p, PartInfo& pi, int& width1) {
+  int bi = 0;
+  while (bi + 1 < B.n && s >= B.strip_begin[bi + 1]) ++bi;
+  const SourceBlock& sb = B.b[bi];
+  const int chunks = B.chunks[bi], groups = B.groups[bi], per = B.per[bi], w = B.width[bi];
+  width1 = w + 1;
+  const long long total = (long long)sb.num * groups * chunks;
+  const long long k = (s - B.strip_begin[bi]) * per + p;
+  const long long left = total - (s - B.strip_begin[bi]) * per;
+  const int count = left < per ? (int)left : per;
+  if (p < count) {
+    int c, n, g;
+    if (total <= 0x7fffffff) {  // 32-bit divisions
+      const unsigned row = (unsigned)k / (unsigned)chunks;
+      c = (int)((unsigned)k - row * chunks);
+      n = (int)(row / (unsigned)groups);
+      g = (int)(row - (unsigned)n * groups);
+    } else {
+      const long long row = k / chunks;
+      c = (int)(k - row * chunks);
+      n = (int)(row / groups);
+      g = (int)(row - (long long)n * groups);
+    }
+    const int i0 = g * H, j0 = c * w;
+    const int owned = min(H, sb.node_rows - i0);
+    pi.nr = owned + (i0 + owned < sb.node_rows ? 1 : 0);
+    pi.nc = min(w, sb.cols - j0) + 1;
+    pi.last_h = j0 + pi.nc - 1 == sb.cols;
+    pi.stride = sb.cols + 1;
+    pi.first = sb.rec_off + ((long long)n * sb.node_rows + i0) * (sb.cols + 1) + j0;
+  }
+  return count;
+}
+
+// The source strips of a target tile are dealt into `classes` (strip s to
+// class s mod classes) and split y of the tile takes the classes begin[y] ..
+// begin[y + 1] - 1.  Neighbouring strips fall into different classes, so the
+// strips near a tile (the newest wake rows, next to the wing) and their
+// costlier near-field work are spread over its splits.
+constexpr int kMaxSplits = 64;
+struct SplitTable {
+  int n, classes;
+  unsigned char begin[kMaxSplits + 1];
+};
+
 // ------------------------------------------------------ batched evaluation
 // Many independent problems in one persistent launch: problem c has its own
 // source blocks (records already built) and targets [tgt_off, tgt_off+n_tgt)
@@ -205,7 +308,7 @@ __device__ inline StripInfo decode_strip(const Blocks& B, long long s) {
 // Work items = (problem, target tile, source split) with at most
 // kBatchStripsPerItem strips each; every CTA strides over the items, so the
 // launch shape is fixed while the problem sizes change from step to step.
-constexpr int kBatchStripsPerItem = 8;
+constexpr int kBatchStripsPerItem = 3;
 
 struct NBodyBatchInput {
   SourceBlock blocks[2];
@@ -214,36 +317,18 @@ struct NBodyBatchInput {
 };
 
 struct NBodyBatchPlan {
-  Blocks B;
+  PartBlocks B;
   long long n_strips, tgt_off, n_tgt;
   long long tiles, splits, item_off, part_off, tgt_prefix;
 };
 
-// A problem whose sheets fill at least 3/4 of the staged strip columns is
-// walked as whole padded strips by the packed FP32x2 walker (FP32 only); the
-// others by the general walker.  FP32 evaluations therefore run as two
-// persistent launches, one per class.
-__host__ __device__ inline bool batch_input_padded(const NBodyBatchInput& x) {
-  bool any = false;
-  for (int i = 0; i < x.n_blocks; ++i) {
-    const SourceBlock& b = x.blocks[i];
-    if (b.num <= 0 || b.node_rows < 2 || b.cols <= 0) continue;
-    const long long chunks = (b.cols + kStripCols - 1) / kStripCols;
-    if (4 * (b.cols + chunks) < 3 * chunks * (kStripCols + 1)) return false;
-    any = true;
-  }
-  return any;
-}
-
-// Strip height of the batched tile of a precision and class.
-int nbody_batch_rows(NBodyPrec prec, bool padded);
 // Upper bound of the partial-sum doubles for the given inputs (host copy).
 long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in, int n);
 // Persistent grid sizes used by nbody_batch_eval on this device, and the
 // FP32 tile (strip height) the batch runs: tiles[t] is the grid of tile t.
 constexpr int kNumBatchTilesF = 3;
 struct NBodyBatchGrids {
-  int general = 0, padded = 0;
+  int fp64 = 0;
   int tiles[kNumBatchTilesF] = {0, 0, 0};
   int tile = 0;
 };
@@ -263,7 +348,14 @@ int nbody_num_variants();
 int nbody_variant_prec(int v);
 // Whether a variant evaluates the FP32 form's near pairs in FP64 when NBodyWork::near64 is set.
 bool nbody_variant_near64(int v);
+// Whether a variant is one of the far-field walkers (nbody_parts.cuh), the only ones the autotuners time.
+bool nbody_variant_far(int v);
 const char* nbody_variant_name(int v);
+// The variant an evaluation takes where nothing has chosen one: the lowest
+// parts, which leave the fewest pairs to the near walkers (whole step at a
+// 50-row wake: fp32 h2 0.72, h3 0.78 ms; fp64 h2_t1 0.74, h2_t2 0.77, h3 0.79;
+// on long wakes the autotuner chooses).
+constexpr int kDefaultVariantF32 = 17, kDefaultVariantF64 = 18;  // fp32_h2_t2_b128_x2f, fp64_h2_t1_b128_m3f
 
 // Build the source records of `n_views` sheets into work.records (blocks are
 // appended in order) and fill blocks[].  Returns total records.
