@@ -303,6 +303,12 @@ int uvlm_sheet_induced_velocity_noalloc(const double* pos, const double* gamma, 
                                         int64_t gcols, const double* targets, int64_t n_targets, double* out,
                                         int32_t precision, void* stream);
 
+/* No counterpart in the reference.  The context-free calls take their device
+ * arrays from a pool that keeps at most 256 MiB per device between calls; this
+ * gives all of it back (calls of other threads that are still running keep what
+ * they use). */
+int uvlm_release_workspace(int32_t device);
+
 /* advect::Advection strategy object (src/advect.h:48-59) from
  * AdvectFactory(name) (src/advect_factory.cpp:43-60): "euler", "RK2",
  * "RK4", "AB2".  AB2 keeps its velocity history between calls. */

@@ -1,0 +1,55 @@
+"""The workspace of the context-free calls: shared by threads, given back (B200)."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(seed):
+    rng = np.random.default_rng(seed)
+    rows, cols = 3 + seed, 5 + 2 * seed
+    x, y = np.meshgrid(0.2 * np.arange(rows + 1), 0.1 * np.arange(cols + 1), indexing="ij")
+    pos = np.stack([x, y, 0.02 * rng.standard_normal(x.shape)], -1)[None]
+    return pos, rng.standard_normal((1, rows, cols)), rng.uniform(-1, 2, (200 + 900 * seed, 3))
+
+
+def test_threads_share_the_workspace_and_it_is_given_back():
+    """Calls of several threads at once, of different sizes and kinds, give what each gives alone; so do calls after
+    the workspace was released, between and during them."""
+    import uvlm_b200 as U
+
+    def work(seed):
+        pos, gamma, t = _case(seed)
+        A = np.eye(40 + 30 * seed) * 3 + np.random.default_rng(seed).standard_normal((40 + 30 * seed,) * 2) * 0.1
+        b = np.arange(len(A), dtype=float)
+        return [U.InducedVelocity(t, pos, gamma), U.InducedVelocity(t, pos, gamma, "mixed"), U.dense_solve(A, b)[0],
+                U.dense_solve(A, b, "tf32")[0]]
+
+    alone = [work(s) for s in range(4)]
+    got, errors = [[] for _ in range(4)], []
+
+    def run(s):
+        try:
+            for _ in range(6):
+                got[s].append(work(s))
+        except Exception as e:  # noqa: BLE001 (reported below)
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    U.release_workspace()
+    for t in threads:
+        t.join()
+    assert not errors
+    for s in range(4):
+        for rep in got[s]:
+            for a, b in zip(rep, alone[s]):
+                np.testing.assert_array_equal(a, b)
+    U.release_workspace()
+    for a, b in zip(work(2), alone[2]):
+        np.testing.assert_array_equal(a, b)
+    with pytest.raises(U.UVLMError):
+        U.release_workspace(63)

@@ -29,7 +29,7 @@ from .wing import NACA00XXGenerator, NACA4digitGenerator, RectGenerator, WholeWi
 
 __all__ = ["SimpleSimulator", "Morphing", "WingGenerator", "RectGenerator", "NACA4digitGenerator",
            "NACA00XXGenerator", "WholeWing", "AdvectFactory", "Advection", "InducedVelocity", "UVLMError",
-           "dense_solve", "rings", "lib"]
+           "dense_solve", "release_workspace", "rings", "lib"]
 
 _P = C.POINTER(C.c_double)
 
@@ -438,6 +438,11 @@ def InducedVelocity(x, pos, gamma, precision: str = "fp64") -> np.ndarray:  # no
     check(lib().uvlm_sheet_induced_velocity(_p(pos), _p(gamma) if gamma.size else None, num, gr, gc, _p(xs),
                                             xs.shape[0], _p(out), PRECISION[precision]))
     return out[0] if single else out
+
+
+def release_workspace(device: int = 0) -> None:
+    """Give back the device memory that the context-free calls keep between calls (at most 256 MiB)."""
+    check(lib().uvlm_release_workspace(int(device)))
 
 
 def dense_solve(A, b, method: str = "fp64"):

@@ -1,5 +1,6 @@
 // gmres.cu -- FP64 GMRES(m) with an FP32 LU preconditioner.
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
 #include "gmres.cuh"
@@ -89,28 +90,48 @@ Error matvec(const float* A32, const double* A64, int n, const double* x, double
   return ok();
 }
 
-Error gmres_work_alloc(GmresWork* g, int n, int m) {
+Error gmres_work_alloc(GmresWork* g, int n, int m, Scratch* scratch) {
   gmres_work_free(g);
   g->n = n;
   g->m = m;
-  UVLM_CUDA_TRY(cudaMalloc(&g->V, sizeof(double) * (size_t)(m + 1) * n));
-  UVLM_CUDA_TRY(cudaMalloc(&g->Z, sizeof(double) * (size_t)m * n));
-  UVLM_CUDA_TRY(cudaMalloc(&g->w, sizeof(double) * n));
-  UVLM_CUDA_TRY(cudaMalloc(&g->h, sizeof(double) * 2 * (m + 2)));
-  UVLM_CUDA_TRY(cudaMalloc(&g->y, sizeof(double) * (m + 1)));
-  UVLM_CUDA_TRY(cudaMalloc(&g->ptmp, sizeof(float) * 2 * n));
-  UVLM_CUDA_TRY(cudaMallocHost(&g->hh, sizeof(double) * 2 * (m + 2)));
+  auto aligned = [](size_t bytes) { return (bytes + 255) & ~(size_t)255; };
+  const size_t size[6] = {aligned(sizeof(double) * (size_t)(m + 1) * n), aligned(sizeof(double) * (size_t)m * n),
+                          aligned(sizeof(double) * n), aligned(sizeof(double) * 2 * (m + 2)),
+                          aligned(sizeof(double) * (m + 1)), aligned(sizeof(float) * 2 * n)};
+  size_t bytes = 0;
+  for (size_t q : size) bytes += q;
+  void* base = nullptr;
+  if (scratch) {
+    UVLM_TRY(scratch->bytes(&base, bytes));
+    g->hh = static_cast<double*>(std::malloc(sizeof(double) * 2 * (m + 2)));
+    if (!g->hh) return fail(kErrCapacity, "out of host memory");
+  } else {
+    UVLM_CUDA_TRY(cudaMalloc(&base, bytes));
+    g->own = base;
+    UVLM_CUDA_TRY(cudaMallocHost(&g->hh, sizeof(double) * 2 * (m + 2)));
+  }
+  char* p = static_cast<char*>(base);
+  void* at[6];
+  for (int q = 0; q < 6; ++q) {
+    at[q] = p;
+    p += size[q];
+  }
+  g->V = static_cast<double*>(at[0]);
+  g->Z = static_cast<double*>(at[1]);
+  g->w = static_cast<double*>(at[2]);
+  g->h = static_cast<double*>(at[3]);
+  g->y = static_cast<double*>(at[4]);
+  g->ptmp = static_cast<float*>(at[5]);
   return ok();
 }
 
 void gmres_work_free(GmresWork* g) {
-  cudaFree(g->V);
-  cudaFree(g->Z);
-  cudaFree(g->w);
-  cudaFree(g->h);
-  cudaFree(g->y);
-  cudaFree(g->ptmp);
-  if (g->hh) cudaFreeHost(g->hh);
+  if (g->own) {
+    cudaFree(g->own);
+    if (g->hh) cudaFreeHost(g->hh);
+  } else {
+    std::free(g->hh);
+  }
   *g = GmresWork{};
 }
 

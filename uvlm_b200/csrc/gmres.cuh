@@ -14,11 +14,12 @@ namespace uvlm {
 
 struct GmresWork {
   int n = 0, m = 0;
+  void* own = nullptr;   // the block of the device arrays (NULL when it is a Scratch's)
   double* V = nullptr;   // [m+1][n]
   double* Z = nullptr;   // [m][n]   preconditioned directions
   double* w = nullptr;   // [n]
   double* h = nullptr;   // [2][m+1] device dot products
-  double* hh = nullptr;  // pinned host copy
+  double* hh = nullptr;  // host copy (pinned where the device arrays are the GmresWork's own)
   float* ptmp = nullptr; // [2n] preconditioner scratch
   double* y = nullptr;   // [m] device
 };
@@ -31,7 +32,7 @@ struct GmresResult {
   bool nonfinite_guess = false;  // the initial guess gave a non-finite residual (nothing iterated)
 };
 
-Error gmres_work_alloc(GmresWork* g, int n, int m);
+Error gmres_work_alloc(GmresWork* g, int n, int m, Scratch* scratch = nullptr);
 void gmres_work_free(GmresWork* g);
 
 // Solves A x = b.  Exactly one of A32 / A64 is non-null (the residual matrix,

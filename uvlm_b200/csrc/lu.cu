@@ -1481,51 +1481,59 @@ Error lu_inverse_f32(const float* LU, int n, LuUpdate upd, LuWork* w, float* X, 
   return ok();
 }
 
-Error lu_work_alloc(LuWork* w, int n, int elem_size, int num_sms) {
+namespace {
+// The arrays of a LuWork laid out in one block from `base` (NULL: only counts);
+// returns its size.
+size_t lu_work_place(LuWork* w, char* base) {
+  size_t at = 0;
+  auto put = [&](auto** p, size_t bytes) {
+    if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + at);
+    at += (bytes + 255) & ~(size_t)255;
+  };
+  const size_t n = (size_t)w->n, e = (size_t)w->elem_size, nblk = (size_t)ceil_div(w->n, kTriB);
+  put(&w->err, sizeof(int) * 4);
+  put(&w->flags, sizeof(unsigned) * 2 * kLuMaxCtas);
+  put(&w->ipiv, sizeof(int) * 2 * n);
+  put(&w->bar, sizeof(unsigned) * 2);
+  put(&w->cand_val, sizeof(double) * 2 * kLuMaxCtas);
+  put(&w->cand_row, sizeof(int) * 2 * kLuMaxCtas);
+  put(&w->cand_data, e * 2 * kLuMaxCtas * kLuNB);
+  put(&w->diag_data, e * 2 * kLuNB);
+  put(&w->dinv_l, e * nblk * kTriB * kTriB);
+  put(&w->dinv_u, e * nblk * kTriB * kTriB);
+  if (e == 4) {
+    put(&w->ut, sizeof(float) * n * kLuNB);
+    put(&w->a3, sizeof(float) * n * 3 * kTriB);
+    put(&w->b3, sizeof(float) * n * 3 * kTriB);
+    put(&w->opA, 2 * n * kLuNB);
+    put(&w->opB, 2 * n * kLuNB);
+  }
+  return at;
+}
+}  // namespace
+
+Error lu_work_alloc(LuWork* w, int n, int elem_size, int num_sms, Scratch* scratch) {
   lu_work_free(w);
   w->n = n;
   w->elem_size = elem_size;
   w->num_sms = num_sms;
-  const int nblk = ceil_div(n, kTriB);
-  UVLM_CUDA_TRY(cudaMalloc(&w->ipiv, sizeof(int) * 2 * n));
-  UVLM_CUDA_TRY(cudaMalloc(&w->err, sizeof(int) * 4));
-  UVLM_CUDA_TRY(cudaMalloc(&w->bar, sizeof(unsigned) * 2));
-  UVLM_CUDA_TRY(cudaMalloc(&w->cand_val, sizeof(double) * 2 * kLuMaxCtas));
-  UVLM_CUDA_TRY(cudaMalloc(&w->cand_row, sizeof(int) * 2 * kLuMaxCtas));
-  UVLM_CUDA_TRY(cudaMalloc(&w->cand_data, (size_t)elem_size * 2 * kLuMaxCtas * kLuNB));
-  UVLM_CUDA_TRY(cudaMalloc(&w->diag_data, (size_t)elem_size * 2 * kLuNB));
-  UVLM_CUDA_TRY(cudaMalloc(&w->dinv_l, (size_t)elem_size * nblk * kTriB * kTriB));
-  UVLM_CUDA_TRY(cudaMalloc(&w->dinv_u, (size_t)elem_size * nblk * kTriB * kTriB));
-  UVLM_CUDA_TRY(cudaMalloc(&w->flags, sizeof(unsigned) * 2 * kLuMaxCtas));
+  const size_t bytes = lu_work_place(w, nullptr);
+  void* base = nullptr;
+  if (scratch) {
+    UVLM_TRY(scratch->bytes(&base, bytes));
+  } else {
+    UVLM_CUDA_TRY(cudaMalloc(&base, bytes));
+    w->own = base;
+  }
+  lu_work_place(w, static_cast<char*>(base));
   UVLM_CUDA_TRY(cudaMemset(w->flags, 0, sizeof(unsigned) * 2 * kLuMaxCtas));
   UVLM_CUDA_TRY(cudaMemset(w->err, 0, sizeof(int) * 4));
-  if (elem_size == 4) {
-    UVLM_CUDA_TRY(cudaMalloc(&w->ut, sizeof(float) * (size_t)n * kLuNB));
-    UVLM_CUDA_TRY(cudaMalloc(&w->a3, sizeof(float) * (size_t)n * 3 * kTriB));
-    UVLM_CUDA_TRY(cudaMalloc(&w->b3, sizeof(float) * (size_t)n * 3 * kTriB));
-    UVLM_CUDA_TRY(cudaMalloc(&w->opA, 2 * (size_t)n * kLuNB));
-    UVLM_CUDA_TRY(cudaMalloc(&w->opB, 2 * (size_t)n * kLuNB));
-  }
   w->epoch = 0;
   return ok();
 }
 
 void lu_work_free(LuWork* w) {
-  cudaFree(w->ipiv);
-  cudaFree(w->err);
-  cudaFree(w->bar);
-  cudaFree(w->cand_val);
-  cudaFree(w->cand_row);
-  cudaFree(w->cand_data);
-  cudaFree(w->diag_data);
-  cudaFree(w->dinv_l);
-  cudaFree(w->dinv_u);
-  cudaFree(w->flags);
-  cudaFree(w->ut);
-  cudaFree(w->a3);
-  cudaFree(w->b3);
-  cudaFree(w->opA);
-  cudaFree(w->opB);
+  cudaFree(w->own);
   *w = LuWork{};
 }
 

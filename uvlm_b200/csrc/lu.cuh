@@ -28,6 +28,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "workspace.cuh"
 
 namespace uvlm {
 
@@ -38,6 +39,7 @@ enum LuUpdate { kLuUpdateSimt = 0, kLuUpdateTF32 = 1, kLuUpdateBF16 = 2 };
 
 struct LuWork {
   int n = 0;
+  void* own = nullptr;        // the block of all arrays (NULL when it is a Scratch's)
   int* ipiv = nullptr;        // [n]
   int* err = nullptr;         // [1]: 0 ok, 1 barrier timeout, 2 zero pivot, 3 solve timeout
   unsigned* bar = nullptr;    // [2] grid barrier state
@@ -63,7 +65,9 @@ struct LuWork {
 
 constexpr int kLuMaxCtas = 148;
 
-Error lu_work_alloc(LuWork* w, int n, int elem_size, int num_sms);
+// scratch: the arrays come from it and live as long as it does, else they are
+// the LuWork's own until lu_work_free.
+Error lu_work_alloc(LuWork* w, int n, int elem_size, int num_sms, Scratch* scratch = nullptr);
 void lu_work_free(LuWork* w);
 
 // In-place factorisation PA = LU of a row-major n x n matrix.

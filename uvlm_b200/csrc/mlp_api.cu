@@ -10,6 +10,7 @@
 
 #include "../../include/uvlm_b200.h"
 #include "mlp.cuh"
+#include "workspace.cuh"
 
 using namespace uvlm;
 
@@ -34,11 +35,6 @@ __global__ void gather_rows(const float* src, int width, const long long* idx, l
     dst[q] = src[idx[r] * width + q % width];
   }
 }
-
-struct DevBuf {
-  void* p = nullptr;
-  ~DevBuf() { cudaFree(p); }
-};
 
 }  // namespace
 
@@ -97,12 +93,12 @@ int uvlm_mlp_forward(uvlm_mlp* h, const float* x, int64_t n, float* y) {
   if (!h || !x || !y || n < 0) return report(fail(kErrInvalid, "invalid argument"));
   if (n == 0) return UVLM_OK;
   auto run = [&]() -> Error {
-    DevBuf dx, dy;
-    UVLM_CUDA_TRY(cudaMalloc(&dx.p, sizeof(float) * n * kMlpIn));
-    UVLM_CUDA_TRY(cudaMalloc(&dy.p, sizeof(float) * n));
-    UVLM_CUDA_TRY(cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
-    UVLM_TRY(mlp_forward(&h->m, (const float*)dx.p, n, (float*)dy.p, 0));
-    UVLM_CUDA_TRY(cudaMemcpy(y, dy.p, sizeof(float) * n, cudaMemcpyDeviceToHost));
+    Scratch S;
+    float *dx, *dy;
+    UVLM_TRY(S.up(&dx, x, (size_t)n * kMlpIn));
+    UVLM_TRY(S.get(&dy, (size_t)n));
+    UVLM_TRY(mlp_forward(&h->m, dx, n, dy, 0));
+    UVLM_CUDA_TRY(cudaMemcpy(y, dy, sizeof(float) * n, cudaMemcpyDeviceToHost));
     return ok();
   };
   return report(run());
@@ -113,13 +109,13 @@ int uvlm_mlp_forward_tc(uvlm_mlp* h, const float* x, int64_t n, float* y) {
   if (n == 0) return UVLM_OK;
   if (!mlp_tc_available()) return report(fail(kErrUnsupported, "tcgen05 inference needs an sm_100 device"));
   auto run = [&]() -> Error {
-    DevBuf dx, dy;
-    UVLM_CUDA_TRY(cudaMalloc(&dx.p, sizeof(float) * n * kMlpIn));
-    UVLM_CUDA_TRY(cudaMalloc(&dy.p, sizeof(float) * n));
-    UVLM_CUDA_TRY(cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
-    UVLM_TRY(mlp_forward_tc(&h->m, (const float*)dx.p, n, (float*)dy.p, 0));
+    Scratch S;
+    float *dx, *dy;
+    UVLM_TRY(S.up(&dx, x, (size_t)n * kMlpIn));
+    UVLM_TRY(S.get(&dy, (size_t)n));
+    UVLM_TRY(mlp_forward_tc(&h->m, dx, n, dy, 0));
     UVLM_TRY(mlp_tc_check(&h->m, 0));
-    UVLM_CUDA_TRY(cudaMemcpy(y, dy.p, sizeof(float) * n, cudaMemcpyDeviceToHost));
+    UVLM_CUDA_TRY(cudaMemcpy(y, dy, sizeof(float) * n, cudaMemcpyDeviceToHost));
     return ok();
   };
   return report(run());
@@ -128,13 +124,12 @@ int uvlm_mlp_forward_tc(uvlm_mlp* h, const float* x, int64_t n, float* y) {
 int uvlm_mlp_gradients(uvlm_mlp* h, const float* x, const float* target, int64_t n, float* grads, double* loss) {
   if (!h || !x || !target || !grads || n < 1) return report(fail(kErrInvalid, "invalid argument"));
   auto run = [&]() -> Error {
-    DevBuf dx, dt;
-    UVLM_CUDA_TRY(cudaMalloc(&dx.p, sizeof(float) * n * kMlpIn));
-    UVLM_CUDA_TRY(cudaMalloc(&dt.p, sizeof(float) * n));
-    UVLM_CUDA_TRY(cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
-    UVLM_CUDA_TRY(cudaMemcpy(dt.p, target, sizeof(float) * n, cudaMemcpyHostToDevice));
+    Scratch S;
+    float *dx, *dt;
+    UVLM_TRY(S.up(&dx, x, (size_t)n * kMlpIn));
+    UVLM_TRY(S.up(&dt, target, (size_t)n));
     double l = 0;
-    UVLM_TRY(mlp_loss_backward(&h->m, (const float*)dx.p, (const float*)dt.p, n, &l, 0));
+    UVLM_TRY(mlp_loss_backward(&h->m, dx, dt, n, &l, 0));
     UVLM_CUDA_TRY(cudaMemcpy(grads, h->m.grad, sizeof(float) * h->m.n_params, cudaMemcpyDeviceToHost));
     if (loss) *loss = l;
     return ok();
@@ -147,33 +142,33 @@ int uvlm_mlp_train(uvlm_mlp* h, const float* x, const float* target, int64_t n, 
   if (!h || !x || !target || n < 1 || epochs < 1 || batch < 1 || !(lr > 0))
     return report(fail(kErrInvalid, "invalid argument"));
   auto run = [&]() -> Error {
-    DevBuf dx, dt, bx, bt, didx;
-    UVLM_CUDA_TRY(cudaMalloc(&dx.p, sizeof(float) * n * kMlpIn));
-    UVLM_CUDA_TRY(cudaMalloc(&dt.p, sizeof(float) * n));
-    UVLM_CUDA_TRY(cudaMalloc(&bx.p, sizeof(float) * (size_t)batch * kMlpIn));
-    UVLM_CUDA_TRY(cudaMalloc(&bt.p, sizeof(float) * (size_t)batch));
-    UVLM_CUDA_TRY(cudaMalloc(&didx.p, sizeof(long long) * n));
-    UVLM_CUDA_TRY(cudaMemcpy(dx.p, x, sizeof(float) * n * kMlpIn, cudaMemcpyHostToDevice));
-    UVLM_CUDA_TRY(cudaMemcpy(dt.p, target, sizeof(float) * n, cudaMemcpyHostToDevice));
+    Scratch S;
+    float *dx, *dt, *bx, *bt;
+    long long* didx;
+    UVLM_TRY(S.up(&dx, x, (size_t)n * kMlpIn));
+    UVLM_TRY(S.up(&dt, target, (size_t)n));
+    UVLM_TRY(S.get(&bx, (size_t)batch * kMlpIn));
+    UVLM_TRY(S.get(&bt, (size_t)batch));
+    UVLM_TRY(S.get(&didx, (size_t)n));
     std::vector<long long> idx(n);
     std::iota(idx.begin(), idx.end(), 0LL);
     std::mt19937_64 rng(seed);
     double epoch_loss = 0;
     for (int e = 0; e < epochs; ++e) {
       std::shuffle(idx.begin(), idx.end(), rng);
-      UVLM_CUDA_TRY(cudaMemcpy(didx.p, idx.data(), sizeof(long long) * n, cudaMemcpyHostToDevice));
+      UVLM_CUDA_TRY(cudaMemcpy(didx, idx.data(), sizeof(long long) * n, cudaMemcpyHostToDevice));
       epoch_loss = 0;
       long long nb = 0;
       for (long long b0 = 0; b0 + batch <= n || (b0 == 0 && n < batch); b0 += batch) {
         const long long B = std::min<long long>(batch, n - b0);
-        const long long* ib = (const long long*)didx.p + b0;
-        gather_rows<<<std::min<long long>((B * kMlpIn + 255) / 256, 4096), 256>>>((const float*)dx.p, kMlpIn, ib, B,
-                                                                                (float*)bx.p);
+        const long long* ib = didx + b0;
+        gather_rows<<<std::min<long long>((B * kMlpIn + 255) / 256, 4096), 256>>>(dx, kMlpIn, ib, B,
+                                                                                bx);
         UVLM_LAUNCH_CHECK();
-        gather_rows<<<std::min<long long>((B + 255) / 256, 4096), 256>>>((const float*)dt.p, 1, ib, B, (float*)bt.p);
+        gather_rows<<<std::min<long long>((B + 255) / 256, 4096), 256>>>(dt, 1, ib, B, bt);
         UVLM_LAUNCH_CHECK();
         double l = 0;
-        UVLM_TRY(mlp_loss_backward(&h->m, (const float*)bx.p, (const float*)bt.p, B, &l, 0));
+        UVLM_TRY(mlp_loss_backward(&h->m, bx, bt, B, &l, 0));
         UVLM_TRY(mlp_adam_step(&h->m, (float)lr, 0));
         epoch_loss += l;
         ++nb;

@@ -16,14 +16,13 @@
 // the same call, and the empty-sheet case clears the velocities it returns).
 // Calls that overlap on the GPU (for example on two streams) race on the
 // array: serialise them.
-#include <cuda.h>
-
 #include <climits>
 #include <mutex>
 
 #include "../../include/uvlm_b200.h"
 #include "device_once.h"
 #include "nbody.cuh"
+#include "workspace.cuh"
 
 namespace uvlm {
 namespace {
@@ -37,32 +36,6 @@ __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 std::mutex g_mu;
 void* g_scratch_ptr[kMaxDevices] = {};
 unsigned long long g_scratch_ctx[kMaxDevices] = {};  // context the address belongs to
-
-// Unique id of the context current on this thread (0 if the driver entry
-// points are unavailable).  A cudaDeviceReset destroys the primary context and
-// the module with it; the next primary context has another id, so the address
-// is looked up again instead of reusing a stale one.
-unsigned long long current_context_id() {
-  using GetCurrent = CUresult (*)(CUcontext*);
-  using GetId = CUresult (*)(CUcontext, unsigned long long*);
-  static GetCurrent get_current = nullptr;
-  static GetId get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<GetCurrent>(fn);
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<GetId>(fn);
-  });
-  CUcontext ctx = nullptr;
-  unsigned long long id = 0;
-  if (get_current && get_id && get_current(&ctx) == CUDA_SUCCESS && ctx) get_id(ctx, &id);
-  return id;
-}
 
 // Set-up, once per device (and again only if that device's context was
 // reset), with that device current: the device address of the scratch array.

@@ -140,7 +140,7 @@ Error solve_rings(const double* bound_rings, const double* bound_rings0, int64_t
   }
   UVLM_TRY(launch_legacy_rhs(dk, dko, dr0, n, cen, nrm, freestream, t, wv, b, 0));
   LuWork lu;
-  UVLM_TRY(lu_work_alloc(&lu, n, 8, sms()));
+  UVLM_TRY(lu_work_alloc(&lu, n, 8, sms(), &S));
   Error e = lu_factor_f64(A, n, &lu, 0);
   if (!e.code) e = lu_check(&lu, 0);
   if (!e.code) e = lu_solve_f64(A, n, &lu, b, x, tmp, 0);
@@ -230,7 +230,7 @@ int uvlm_advection_advect(uvlm_advection* adv, double* next, const double* wing_
   const int C = (int)cols, nodes = (int)wake_rows + 1;
   const size_t wn = (size_t)num * nodes * (C + 1) * 3;
   auto run = [&]() -> Error {
-    double *dwing, *dwg, *x, *pos2, *k1, *k2, *k3, *vprev, *dwg2, *vx, *vy, *vz, *targets;
+    double *dwing, *dwg, *x, *pos2, *k1, *k2, *k3, *vprev, *dwg2, *vx, *vy, *vz, *tx, *ty, *tz;
     UVLM_TRY(S.up(&dwing, wing_pos, (size_t)num * (rows + 1) * (cols + 1) * 3));
     UVLM_TRY(S.up(&dwg, wing_gamma, (size_t)num * rows * cols));
     UVLM_TRY(S.up(&x, wake_pos, wn));
@@ -249,24 +249,24 @@ int uvlm_advection_advect(uvlm_advection* adv, double* next, const double* wing_
     UVLM_TRY(S.get(&vx, std::max<long long>(nt, 1)));
     UVLM_TRY(S.get(&vy, std::max<long long>(nt, 1)));
     UVLM_TRY(S.get(&vz, std::max<long long>(nt, 1)));
-    UVLM_TRY(S.get(&targets, 3 * std::max<long long>(nt, 1)));
+    UVLM_TRY(S.get(&tx, std::max<long long>(nt, 1)));
+    UVLM_TRY(S.get(&ty, std::max<long long>(nt, 1)));
+    UVLM_TRY(S.get(&tz, std::max<long long>(nt, 1)));
     const WakeLayout L{(int)num, C, nodes, 0, nodes};
-    auto vel = [&](const double* P) -> Error {
-      if (nt == 0) return ok();
-      double *tx, *ty, *tz;
-      UVLM_TRY(S.get(&tx, nt));
-      UVLM_TRY(S.get(&ty, nt));
-      UVLM_TRY(S.get(&tz, nt));
-      UVLM_TRY(launch_gather_wake(L, P, tx, ty, tz, 0));
-      soa_to_aos<<<gfor(nt), 256>>>(tx, ty, tz, nt, targets, nullptr, nullptr, 1.0);
-      UVLM_LAUNCH_CHECK();
+    // velocities at the wake rows first_row.. of the wake at P
+    auto vel = [&](const double* P, int first_row = 1) -> Error {
+      const long long n_tgt = (long long)num * std::max(0, nodes - first_row) * (C + 1);
+      if (n_tgt == 0) return ok();
+      UVLM_TRY(launch_gather_wake(L, P, tx, ty, tz, 0, first_row));
       SheetView views[2] = {
           SheetView{dwing, (int)rows + 1, 0, dwg, (int)rows, 0, (int)num, (int)rows + 1, C},
           SheetView{P, nodes, 0, dwg2, nodes, 0, (int)num, nodes, C}};
       const int nv = wake_rows > 0 ? 2 : 1;
-      return velocity_at(views, nv, prec, targets, nt, vx, vy, vz, S);
+      return velocity_soa(views, nv, prec, tx, ty, tz, n_tgt, vx, vy, vz, S);
     };
     const int ign = 5;
+    // the last evaluation of RK2 and RK4 only feeds the rows past `ign` (src/advect.cpp:71-79, :167-178)
+    const int late = ign + 1;
     switch (adv->scheme) {
       case UVLM_ADVECT_EULER:
         UVLM_TRY(vel(x));
@@ -275,16 +275,16 @@ int uvlm_advection_advect(uvlm_advection* adv, double* next, const double* wing_
       case UVLM_ADVECT_RK2:
         UVLM_TRY(vel(x));
         UVLM_TRY(launch_advect(kAdvRK2K1, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0));
-        UVLM_TRY(vel(pos2));
-        UVLM_TRY(launch_advect(kAdvRK2Upd, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0));
+        UVLM_TRY(vel(pos2, late));
+        UVLM_TRY(launch_advect(kAdvRK2Upd, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0, late));
         break;
       case UVLM_ADVECT_RK4:
         UVLM_TRY(vel(x));
         UVLM_TRY(launch_advect(kAdvRK4K1, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0));
         UVLM_TRY(vel(pos2));
         UVLM_TRY(launch_advect(kAdvRK4K2, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0));
-        UVLM_TRY(vel(pos2));
-        UVLM_TRY(launch_advect(kAdvRK4Upd, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0));
+        UVLM_TRY(vel(pos2, late));
+        UVLM_TRY(launch_advect(kAdvRK4Upd, L, x, pos2, k1, k2, k3, vprev, false, vx, vy, vz, ff, dt, ign, 0, late));
         break;
       case UVLM_ADVECT_AB2: {
         // v_prev(n, i-1, j) of the previous call pairs with v(n, i, j)
@@ -446,7 +446,7 @@ int uvlm_lu_factor_f32(const float* A, int64_t n, int32_t update, float* LU, int
     float* dA;
     UVLM_TRY(S.up(&dA, A, (size_t)N * N));
     LuWork lu;
-    UVLM_TRY(lu_work_alloc(&lu, N, 4, sms()));
+    UVLM_TRY(lu_work_alloc(&lu, N, 4, sms(), &S));
     const LuUpdate u = update == 0 ? kLuUpdateSimt : (update == 1 ? kLuUpdateTF32 : kLuUpdateBF16);
     Error e = lu_factor_f32(dA, N, u, &lu, 0);
     if (!e.code) e = lu_check(&lu, 0);
@@ -473,7 +473,7 @@ int uvlm_dense_solve(const double* A, int64_t n, const double* b, double* x, int
     LuWork lu;
     Error e;
     if (method == 0) {
-      UVLM_TRY(lu_work_alloc(&lu, N, 8, sms()));
+      UVLM_TRY(lu_work_alloc(&lu, N, 8, sms(), &S));
       e = lu_factor_f64(dA, N, &lu, 0);
       if (!e.code) e = lu_check(&lu, 0);
       if (!e.code) e = lu_solve_f64(dA, N, &lu, db, dx, tmp, 0);
@@ -484,13 +484,13 @@ int uvlm_dense_solve(const double* A, int64_t n, const double* b, double* x, int
       UVLM_TRY(S.get(&F, (size_t)N * N));
       f64_to_f32<<<gfor((long long)N * N), 256>>>(dA, (long long)N * N, F);
       UVLM_LAUNCH_CHECK();
-      UVLM_TRY(lu_work_alloc(&lu, N, 4, sms()));
+      UVLM_TRY(lu_work_alloc(&lu, N, 4, sms(), &S));
       const LuUpdate upd = method == 2 ? kLuUpdateBF16 : kLuUpdateTF32;
       e = lu_factor_f32(F, N, gemm_tc_available() ? upd : kLuUpdateSimt, &lu, 0);
       if (!e.code) e = lu_check(&lu, 0);
       GmresWork gw;
       GmresResult r;
-      if (!e.code) e = gmres_work_alloc(&gw, N, 20);
+      if (!e.code) e = gmres_work_alloc(&gw, N, 20, &S);
       if (!e.code) {
         UVLM_CUDA_TRY(cudaMemset(dx, 0, sizeof(double) * N));
         e = gmres_solve(nullptr, dA, N, F, &lu, nullptr, db, dx, 1e-13, 200, &gw, &r, 0);

@@ -1,15 +1,14 @@
 // refapi_util.cuh -- helpers shared by the context-free C-ABI entry points
-// (refapi.cu, legacy.cu): scoped device scratch, AoS/SoA conversion, AoS
+// (refapi.cu, legacy.cu): AoS/SoA conversion, AoS
 // rings as 1 x 1 sheets, the FP64/FP32 N-body at arbitrary targets and a
 // fixed-order block sum.
 #pragma once
 
 #include <algorithm>
-#include <vector>
-
 #include "../../include/uvlm_b200.h"
 #include "common.cuh"
 #include "nbody.cuh"
+#include "workspace.cuh"
 
 using namespace uvlm;
 
@@ -26,28 +25,6 @@ int sms() {
   cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d);
   return v;
 }
-
-// Device buffers freed at scope exit.
-struct Scratch {
-  std::vector<void*> p;
-  ~Scratch() {
-    for (void* q : p) cudaFree(q);
-  }
-  template <class T>
-  Error get(T** out, size_t count) {
-    *out = nullptr;
-    if (count == 0) return ok();
-    UVLM_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(out), sizeof(T) * count));
-    p.push_back(*out);
-    return ok();
-  }
-  template <class T>
-  Error up(T** out, const T* host, size_t count) {
-    UVLM_TRY(get(out, count));
-    if (count) UVLM_CUDA_TRY(cudaMemcpy(*out, host, sizeof(T) * count, cudaMemcpyHostToDevice));
-    return ok();
-  }
-};
 
 __global__ void aos_to_soa(const double* a, long long n, double* x, double* y, double* z) {
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
@@ -102,6 +79,23 @@ __device__ inline d3 block_sum3(d3 v, double* sh) {
 
 inline int gfor(long long n) { return (int)std::min<long long>(std::max<long long>((n + 255) / 256, 1), 65535); }
 
+// Velocities of the sheets at SoA targets.  The partial sums get room for 64
+// splits of few target tiles; from 64 tiles on fewer splits fill the device.
+Error velocity_soa(const SheetView* views, int nv, NBodyPrec prec, const double* tx, const double* ty,
+                   const double* tz, long long nt, double* vx, double* vy, double* vz, Scratch& S) {
+  NBodyWork w;
+  long long recs = 0;
+  for (int i = 0; i < nv; ++i) recs += (long long)views[i].num * views[i].node_rows * (views[i].cols + 1);
+  w.records_cap = std::max<long long>(recs, 1) * (long long)(prec == kNBodyFP32 ? sizeof(RecF) : sizeof(RecD));
+  UVLM_TRY(S.get(reinterpret_cast<char**>(&w.records), (size_t)w.records_cap));
+  w.partial_cap = 3 * std::max<long long>(nt, 1) * (nt > 64 * 256 ? 24 : kMaxSplits);
+  UVLM_TRY(S.get(&w.partial, (size_t)w.partial_cap));
+  SourceBlock blocks[4];
+  UVLM_TRY(nbody_build_sources(views, nv, prec, &w, blocks, 0));
+  const int variant = prec == kNBodyFP32 ? kDefaultVariantF32 : kDefaultVariantF64;
+  return nbody_eval(blocks, nv, prec, tx, ty, tz, nt, vx, vy, vz, &w, variant, sms(), 0);
+}
+
 Error velocity_at(const SheetView* views, int nv, NBodyPrec prec, const double* d_targets_aos, long long nt,
                   double* vx, double* vy, double* vz, Scratch& S) {
   double *tx, *ty, *tz;
@@ -110,18 +104,7 @@ Error velocity_at(const SheetView* views, int nv, NBodyPrec prec, const double* 
   UVLM_TRY(S.get(&tz, nt));
   aos_to_soa<<<gfor(nt), 256>>>(d_targets_aos, nt, tx, ty, tz);
   UVLM_LAUNCH_CHECK();
-  NBodyWork w;
-  long long recs = 0;
-  for (int i = 0; i < nv; ++i) recs += (long long)views[i].num * views[i].node_rows * (views[i].cols + 1);
-  w.records_cap = std::max<long long>(recs, 1) * (long long)sizeof(RecD);
-  UVLM_TRY(S.get(reinterpret_cast<char**>(&w.records), (size_t)w.records_cap));
-  w.partial_cap = 3 * std::max<long long>(nt, 1) * 64;
-  UVLM_TRY(S.get(&w.partial, (size_t)w.partial_cap));
-  SourceBlock blocks[4];
-  UVLM_TRY(nbody_build_sources(views, nv, prec, &w, blocks, 0));
-  const int variant = prec == kNBodyFP32 ? kDefaultVariantF32 : kDefaultVariantF64;
-  UVLM_TRY(nbody_eval(blocks, nv, prec, tx, ty, tz, nt, vx, vy, vz, &w, variant, sms(), 0));
-  return ok();
+  return velocity_soa(views, nv, prec, tx, ty, tz, nt, vx, vy, vz, S);
 }
 
 }  // namespace

@@ -1,0 +1,64 @@
+// workspace.cuh -- device memory for the length of a context-free call.
+#pragma once
+
+#include <vector>
+
+#include "common.cuh"
+
+namespace uvlm {
+
+// Stream-ordered on the legacy default stream of the current device.
+Error workspace_alloc(void** p, size_t bytes);
+void workspace_free(void* p);
+// Unique id of the context current on this thread (0 if the driver entry
+// points are unavailable).  A cudaDeviceReset destroys the primary context and
+// what belongs to it; the next primary context has another id.
+unsigned long long current_context_id();
+
+// Device buffers of one call, freed at scope exit.  Small ones share slabs.
+struct Scratch {
+  std::vector<void*> p;
+  char* slab = nullptr;
+  size_t left = 0;
+  Scratch() = default;
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  ~Scratch() {
+    for (void* q : p) workspace_free(q);
+  }
+  Error bytes(void** out, size_t count) {
+    constexpr size_t kSlab = 1u << 20;
+    *out = nullptr;
+    if (count == 0) return ok();
+    const size_t need = (count + 255) & ~(size_t)255;
+    if (need < count) return fail(kErrCapacity, "buffer size out of range");
+    if (need <= kSlab / 2) {
+      if (need > left) {
+        void* s = nullptr;
+        UVLM_TRY(workspace_alloc(&s, kSlab));
+        p.push_back(s);
+        slab = static_cast<char*>(s);
+        left = kSlab;
+      }
+      *out = slab;
+      slab += need;
+      left -= need;
+      return ok();
+    }
+    UVLM_TRY(workspace_alloc(out, need));
+    p.push_back(*out);
+    return ok();
+  }
+  template <class T>
+  Error get(T** out, size_t count) {
+    return bytes(reinterpret_cast<void**>(out), sizeof(T) * count);
+  }
+  template <class T>
+  Error up(T** out, const T* host, size_t count) {
+    UVLM_TRY(get(out, count));
+    if (count) UVLM_CUDA_TRY(cudaMemcpy(*out, host, sizeof(T) * count, cudaMemcpyHostToDevice));
+    return ok();
+  }
+};
+
+}  // namespace uvlm
