@@ -245,3 +245,32 @@ def test_every_batch_tile_agrees_with_the_fp64_batch():
     for t in range(3):
         got = run("mixed", t)
         assert np.max(np.abs(got[:, :, 1:] - ref[:, :, 1:])) <= 1e-6 * scale, t
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_per_case_solve_at_its_block_edges(precision):
+    """Cases whose N = rows x cols sits at and between the edges of the per-case solver (panels of 32 or 16 columns,
+    32-row diagonal blocks, 64 x 256 and 64 x 128 update tiles, the largest N = 1024) against single-case FP64
+    simulators: loads within the batch tolerances."""
+    import uvlm_b200 as U
+    from uvlm_b200.batch import BatchSimulator
+
+    shapes = [(1, 2), (1, 16), (1, 18), (2, 16), (3, 10), (3, 22), (4, 16), (5, 26), (8, 32), (9, 30), (16, 64)]
+    steps, dt = 4, 0.15
+    sim = BatchSimulator(precision=precision, max_steps=steps, nbody_tile=0 if precision == "mixed" else -1)
+    for k, (r, c) in enumerate(shapes):
+        m = U.Morphing().set_alpha(0.05).set_plug(0.1 + 0.01 * k, 1.0).set_twist(0.1, 1.0, math.pi / 2)
+        sim.add_case(m, 1.0, 3.0 + 0.2 * k, r, c, dt)
+    sim.run(steps)
+    rows = sim.loads()
+    sim.close()
+    tol = 1e-9 if precision == "fp64" else 1e-6
+    for k, (r, c) in enumerate(shapes):
+        one = U.SimpleSimulator()
+        m = U.Morphing().set_alpha(0.05).set_plug(0.1 + 0.01 * k, 1.0).set_twist(0.1, 1.0, math.pi / 2)
+        one.AddWing(U.RectGenerator(), m, 1.0, 3.0 + 0.2 * k, r, c)
+        one.set_forward_flight([-1.0, 0.0, 0.0])
+        one.set_advection("euler")
+        ref = one.Run(steps - 1, dt)
+        one.close()
+        assert np.max(np.abs(rows[:, k, 1:] - ref[:, 1:])) <= tol * np.max(np.abs(ref[:, 1:])), (r, c)

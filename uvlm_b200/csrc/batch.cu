@@ -22,6 +22,8 @@
 // and ring row i at the same physical row as node row i (a prepend without a
 // memmove, as SimpleSimulator::Shed prepends, simple_simulator.cpp:171-188).
 #include <algorithm>
+#include <type_traits>
+#include <utility>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -39,7 +41,7 @@ namespace {
 struct BCase {
   int R, C, N, lines;
   long long node_off, ring_off, line_off, mat_off;
-  long long wnode_off, wring_off, wtgt_off, rec_off;
+  long long wnode_off, wring_off, wtgt_off, rec_off, dinv_off;
   double ff[3];
   double dt, area_ref;
   uvlm_kinematics kin;
@@ -288,287 +290,377 @@ __global__ void b_rhs_kernel(const BCase* __restrict__ cs, BPrefix P, int n, con
 
 // ------------------------------------------------------------- dense solve
 // Threads of the per-case solve CTA: the FP32-factor form (refinement sweeps,
-// latency-bound streaming on the largest cases) takes 16 warps; the FP64
-// form, which factors every step, 8 (its panel code keeps its registers).
+// which stream the largest cases' matrices through one SM) takes 16 warps; the
+// FP64 form, which factors every step, 8 (its update tiles fill their
+// registers).
 template <class T>
 struct SolveCfg {
   static constexpr int kThreads = sizeof(T) == 4 ? 512 : 256;
-};
-
-// Panel width of the shared-memory LU: 32 FP32 / 16 FP64 columns, so that
-// the whole panel of the largest case (1024 rows) stays in shared memory.
-template <class T>
-struct PanelCfg {
+  // panel width of the LU: the whole panel of the largest case (1024 rows)
+  // stays in shared memory
   static constexpr int NB = sizeof(T) == 4 ? 32 : 16;
-  static constexpr int LD = NB + 1;  // padded row (conflict-free column walks)
 };
+constexpr int kSolveBlock = 32;  // diagonal block of the triangular solves
 
-inline size_t panel_smem_bytes(int max_N, int elem) {
-  const int nb = elem == 4 ? 32 : 16;
-  return (size_t)max_N * (nb + 1) * elem;
+// Leading dimension of the column-major panel: 16-byte aligned columns with room
+// for the rows that an update tile reads past the last one.
+__host__ __device__ inline int panel_ld(int N) { return ((N + 3) & ~3) + 8; }
+
+// Dynamic shared memory of the solve: x and r, the panel (the solves' vector
+// afterwards), the panel's row map and the row permutation.
+template <class T>
+size_t solve_smem_bytes(int max_N) {
+  return sizeof(double) * 2 * (size_t)max_N + sizeof(T) * SolveCfg<T>::NB * (size_t)panel_ld(max_N) +
+         sizeof(int) * 2 * (size_t)max_N;
+}
+
+// (|v|, i) of the largest |v| over the block, ties to the lowest i (i < 2^16;
+// a thread without a candidate has v < 0).  One barrier: every warp reduces the
+// warps' results itself.
+template <int NT>
+__device__ int block_pivot(double v, int i, unsigned (*s_key)[NT / 32], bool& nonzero) {
+  // the bits of a non-negative double order as the value does
+  const unsigned long long b = v < 0 ? 0ull : (unsigned long long)__double_as_longlong(v);
+  const unsigned idx = v < 0 ? 0xffffu : (unsigned)i;
+  unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
+  auto reduce = [](unsigned& h, unsigned& l, unsigned& id) {
+    const unsigned mh = __reduce_max_sync(0xffffffffu, h);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, h == mh ? l : 0u);
+    const unsigned mi = __reduce_min_sync(0xffffffffu, h == mh && l == ml ? id : 0xffffu);
+    h = mh;
+    l = ml;
+    id = mi;
+  };
+  unsigned id = idx;
+  reduce(hi, lo, id);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) {
+    s_key[0][wid] = hi;
+    s_key[1][wid] = lo;
+    s_key[2][wid] = id;
+  }
+  __syncthreads();
+  hi = lane < NT / 32 ? s_key[0][lane] : 0u;
+  lo = lane < NT / 32 ? s_key[1][lane] : 0u;
+  id = lane < NT / 32 ? s_key[2][lane] : 0xffffu;
+  reduce(hi, lo, id);
+  nonzero = (hi | lo) != 0u;
+  return (int)id;
+}
+
+__device__ __forceinline__ void ld16(const float* p, float* o) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  o[0] = v.x, o[1] = v.y, o[2] = v.z, o[3] = v.w;
+}
+__device__ __forceinline__ void ld16(const double* p, double* o) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  o[0] = v.x, o[1] = v.y;
 }
 
 // Right-looking blocked LU with partial pivoting of the row-major N x N
-// matrix A by one CTA.  Each panel of NB columns is held in shared memory
-// while it is factored (the pivot of column j is the largest |a| at or below
-// the diagonal, ties to the lower index; pivot search, swaps, scaling and the
-// rank-1 updates walk shared memory instead of strided rows in L2).  The
-// panel's row swaps are then applied to the other columns (LAPACK order),
-// U12 = L11^-1 A12 is solved column per thread with L11 from shared memory,
-// and A22 -= L21 U12 reads L21 from shared memory.  piv[j] = row swapped
-// with j.  P: (N - k0) x LD panel buffer in dynamic shared memory.
+// matrix A by one CTA (N even).  Each panel of NB columns is held column-major
+// in shared memory while it is factored, one row per thread (two barriers per
+// column: the pivot search, the exchange of the pivot row).  The panel's row
+// exchanges are then applied to every other column at once: a thread takes a
+// column, loads the rows that come to the top and the rows that are displaced
+// (up to 2 NB independent loads), stores the displaced ones, and right of the
+// panel solves U12 = L11^-1 A12 in registers first.  A22 -= L21 U12 runs in
+// tiles of 8 x 4 values per thread, L21 read as 16-byte
+// pieces of the panel's columns.  perm[i]: the row of the original matrix at
+// row i.  The largest case of a sweep (N = 1024), against a row-major panel with
+// four barriers per column, row exchanges one after another and 4 x 4 tiles:
+// FP32 10 -> 6.2 ms, FP64 with its solve 30 -> 11.8 ms.
 template <class T>
-__device__ void cta_lu_panel_smem(T* A, int N, int* piv, int* status, T* P) {
-  constexpr int NB = PanelCfg<T>::NB, LD = PanelCfg<T>::LD;
-  constexpr int NT = SolveCfg<T>::kThreads;
-  constexpr int TR = NT / 16 * 4;  // rows of an A22 tile (16 threads x 4 columns across, 4 rows each)
-  __shared__ double s_val[NT / 32];
-  __shared__ int s_idx[NT / 32];
+__device__ void cta_lu_factor(T* A, int N, int* perm_out, int* status, T* P, int* map, int* perm) {
+  constexpr int NB = SolveCfg<T>::NB, NT = SolveCfg<T>::kThreads;
+  constexpr int kRows = 8, kCols = 4;                 // values of a thread in an update tile
+  constexpr int TR = NT / 16 * kRows;                 // 16 threads across
+  constexpr int TC = 16 * kCols;
+  const int LD = panel_ld(N);
+  __shared__ unsigned s_key[2][3][NT / 32];
   __shared__ int s_piv[NB];
-  __shared__ T Bs[NB][64];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  __shared__ T s_u[NB];
+  __shared__ __align__(16) T Bs[NB][TC];
+  const int tid = threadIdx.x;
+  for (int i = tid; i < N; i += NT) perm[i] = i;
   for (int k0 = 0; k0 < N; k0 += NB) {
     const int kb = min(NB, N - k0);
     const int m = N - k0;
+    __syncthreads();  // the last panel's readers are done
     for (int q = tid; q < m * NB; q += NT) {
       const int r = q / NB, c = q % NB;
-      P[r * LD + c] = c < kb ? A[(long long)(k0 + r) * N + k0 + c] : (T)0;
+      P[c * LD + r] = c < kb ? A[(long long)(k0 + r) * N + k0 + c] : (T)0;
     }
+    for (int i = tid; i < m; i += NT) map[i] = i;
     __syncthreads();
     for (int jj = 0; jj < kb; ++jj) {
       double best = -1.0;
-      int bi = jj;
-      for (int i = jj + tid; i < m; i += NT) {
-        const double v = fabs((double)P[i * LD + jj]);
+      int bi = 0;
+      for (int i = tid; i < m; i += NT) {
+        if (i < jj) continue;
+        const double v = fabs((double)P[jj * LD + i]);
         if (v > best) {
           best = v;
           bi = i;
         }
       }
-      for (int off = 16; off; off >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, best, off);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-        if (ov > best || (ov == best && oi < bi)) {
-          best = ov;
-          bi = oi;
-        }
+      bool nonzero;
+      int p = block_pivot<NT>(best, bi, s_key[jj & 1], nonzero);
+      if (!nonzero) p = jj;  // zero (or NaN) column
+      if (tid < NB) {
+        // exchange rows jj and p; row jj is published for the elimination
+        const T u = P[tid * LD + p], w = P[tid * LD + jj];
+        P[tid * LD + p] = w;
+        P[tid * LD + jj] = u;
+        s_u[tid] = u;
       }
-      if (lane == 0) {
-        s_val[wid] = best;
-        s_idx[wid] = bi;
-      }
-      __syncthreads();
-      if (tid == 0) {
-        double bv = s_val[0];
-        int ii = s_idx[0];
-        for (int w = 1; w < NT / 32; ++w)
-          if (s_val[w] > bv || (s_val[w] == bv && s_idx[w] < ii)) {
-            bv = s_val[w];
-            ii = s_idx[w];
-          }
-        s_piv[jj] = ii;
-        piv[k0 + jj] = k0 + ii;
-        if (!(bv > 0)) status[1] = 1;
+      if (tid == NB) {
+        s_piv[jj] = p;
+        const int a = map[jj];
+        map[jj] = map[p];
+        map[p] = a;
+        if (!nonzero) status[1] = 1;
       }
       __syncthreads();
-      const int p = s_piv[jj];
-      if (p != jj && tid < NB) {
-        const T t = P[jj * LD + tid];
-        P[jj * LD + tid] = P[p * LD + tid];
-        P[p * LD + tid] = t;
+      const T d = s_u[jj];
+      for (int i = tid; i < m; i += NT) {
+        if (i <= jj) continue;
+        const T l = P[jj * LD + i] / d;
+        P[jj * LD + i] = l;
+#pragma unroll 4
+        for (int c = jj + 1; c < kb; ++c) P[c * LD + i] -= l * s_u[c];
       }
-      __syncthreads();
-      const T d = P[jj * LD + jj];
-      for (int i = jj + 1 + tid; i < m; i += NT) {
-        T* row = P + i * LD;
-        const T l = row[jj] / d;
-        row[jj] = l;
-        for (int c = jj + 1; c < kb; ++c) row[c] -= l * P[jj * LD + c];
-      }
-      __syncthreads();
+      // the next column's search reads rows this thread wrote; its barrier
+      // orders the others' rows before the next exchange, and s_u's readers
     }
-    // panel back to global memory
+    __syncthreads();
     for (int q = tid; q < m * NB; q += NT) {
       const int r = q / NB, c = q % NB;
-      if (c < kb) A[(long long)(k0 + r) * N + k0 + c] = P[r * LD + c];
+      if (c < kb) A[(long long)(k0 + r) * N + k0 + c] = P[c * LD + r];
     }
-    // the panel's swaps on the columns left and right of it, in order
-    for (int jj = 0; jj < kb; ++jj) {
-      const int p = s_piv[jj];
-      if (p != jj) {
-        T* ra = A + (long long)(k0 + jj) * N;
-        T* rb = A + (long long)(k0 + p) * N;
-        for (int c = tid; c < N - kb; c += NT) {
-          const int col = c < k0 ? c : c + kb;
-          const T t = ra[col];
-          ra[col] = rb[col];
-          rb[col] = t;
-        }
+    // the permutation so far, in place through registers
+    {
+      int top = 0, low = 0;
+      if (tid < kb) {
+        top = perm[k0 + map[tid]];
+        low = perm[k0 + map[s_piv[tid]]];
       }
       __syncthreads();
+      if (tid < kb) {
+        perm[k0 + tid] = top;
+        if (s_piv[tid] >= kb) perm[k0 + s_piv[tid]] = low;
+      }
     }
     const int c0 = k0 + kb;
-    if (c0 >= N) break;
-    // U12 = L11^-1 A12: column per thread, the column in registers
-    for (int c = c0 + tid; c < N; c += NT) {
-      T u[NB];
+    for (int q = tid; q < N - kb; q += NT) {
+      const int c = q < k0 ? q : q + kb;
+      T* col = A + (long long)k0 * N + c;
+      T u[NB], w[NB];
 #pragma unroll
-      for (int i = 0; i < NB; ++i) u[i] = i < kb ? A[(long long)(k0 + i) * N + c] : (T)0;
+      for (int i = 0; i < NB; ++i) u[i] = i < kb ? col[(long long)map[i] * N] : (T)0;
 #pragma unroll
-      for (int i = 1; i < NB; ++i) {
-        T s = u[i];
+      for (int i = 0; i < NB; ++i) w[i] = i < kb && s_piv[i] >= kb ? col[(long long)map[s_piv[i]] * N] : (T)0;
 #pragma unroll
-        for (int l = 0; l < i; ++l) s -= P[i * LD + l] * u[l];
-        u[i] = s;
+      for (int i = 0; i < NB; ++i)
+        if (i < kb && s_piv[i] >= kb) col[(long long)s_piv[i] * N] = w[i];
+      if (c >= c0) {
+#pragma unroll
+        for (int i = 1; i < NB; ++i) {
+          T s = u[i];
+#pragma unroll
+          for (int l = 0; l < i; ++l) s -= P[l * LD + i] * u[l];
+          u[i] = s;
+        }
       }
 #pragma unroll
-      for (int i = 1; i < NB; ++i)
-        if (i < kb) A[(long long)(k0 + i) * N + c] = u[i];
+      for (int i = 0; i < NB; ++i)
+        if (i < kb) col[(long long)i * N] = u[i];
     }
+    if (c0 >= N) break;
     __syncthreads();
-    // A22 -= L21 U12 in TR x 64 tiles, L21 = panel rows kb.. (shared memory)
-    const int mt = N - c0;
-    const int rtiles = (mt + TR - 1) / TR, ctiles = (mt + 63) / 64;
-    const int tx = tid & 15, ty = tid >> 4;
-    for (int t = 0; t < rtiles * ctiles; ++t) {
-      const int r0 = (t / ctiles) * TR, q0 = c0 + (t % ctiles) * 64;  // r0 counts from row c0
-      for (int q = tid; q < NB * 64; q += NT) {
-        const int l = q / 64, cc = q % 64;
-        Bs[l][cc] = (q0 + cc < N && l < kb) ? A[(long long)(k0 + l) * N + q0 + cc] : (T)0;
+    // A22 -= L21 U12 (kb == NB here); two neighbouring columns of a row load
+    // and store as one (N and the tile's columns are even)
+    const int mt = N - c0, tx = tid & 15, ty = tid >> 4;
+    using V2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+    for (int q0 = c0; q0 < N; q0 += TC) {
+      __syncthreads();
+      for (int q = tid; q < NB * TC; q += NT) {
+        const int l = q / TC, cc = q % TC;
+        Bs[l][cc] = q0 + cc < N ? A[(long long)(k0 + l) * N + q0 + cc] : (T)0;
       }
       __syncthreads();
-      T acc[4][4];
+      for (int r0 = 0; r0 < mt; r0 += TR) {
+        const int rr = r0 + ty * kRows;
+        if (rr >= mt) continue;
+        T* Cp = A + (long long)(c0 + rr) * N + q0 + tx * kCols;
+        // the products are summed on their own and subtracted once (started
+        // from A22, an FP32 sum would round 32 times at A22's magnitude); A22
+        // is requested first
+        V2 cv[kRows][kCols / 2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < kRows; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = (T)0;
-      if (r0 + ty * 4 < mt) {
-        const T* Lp = P + (kb + r0 + ty * 4) * LD;
+          for (int j = 0; j < kCols; j += 2)
+            if (rr + i < mt && q0 + tx * kCols + j < N)
+              cv[i][j / 2] = *reinterpret_cast<const V2*>(Cp + (long long)i * N + j);
+        T acc[kRows][kCols];
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+#pragma unroll
+          for (int j = 0; j < kCols; ++j) acc[i][j] = (T)0;
+        const T* Lp = P + NB + rr;
 #pragma unroll 4
-        for (int l = 0; l < kb; ++l) {
-          T a[4], bb[4];
+        for (int l = 0; l < NB; ++l) {
+          constexpr int kV = 16 / sizeof(T);  // values of a 16-byte load
+          T a[kRows], b[kCols];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) a[i] = (r0 + ty * 4 + i < mt) ? Lp[i * LD + l] : (T)0;
+          for (int i = 0; i < kRows; i += kV) ld16(Lp + l * LD + i, a + i);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) bb[j] = Bs[l][tx * 4 + j];
+          for (int j = 0; j < kCols; j += kV) ld16(&Bs[l][tx * kCols + j], b + j);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
+          for (int i = 0; i < kRows; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * bb[j];
+            for (int j = 0; j < kCols; ++j) acc[i][j] += a[i] * b[j];
         }
-      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = c0 + r0 + ty * 4 + i;
-        if (r >= N) continue;
+        for (int i = 0; i < kRows; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int cc = q0 + tx * 4 + j;
-          if (cc < N) A[(long long)r * N + cc] -= acc[i][j];
-        }
+          for (int j = 0; j < kCols; j += 2)
+            if (rr + i < mt && q0 + tx * kCols + j < N)
+              *reinterpret_cast<V2*>(Cp + (long long)i * N + j) =
+                  V2{cv[i][j / 2].x - acc[i][j], cv[i][j / 2].y - acc[i][j + 1]};
       }
-      __syncthreads();
     }
   }
+  __syncthreads();
+  for (int i = tid; i < N; i += NT) perm_out[i] = perm[i];
 }
 
-// x <- (LU)^-1 P x in place (x in shared memory, FP64 arithmetic): the row
-// swaps, then unit-lower and upper block substitution (32-row diagonal blocks
-// by warp 0 with shuffles, the rest by all threads).
+// Inverses of the 32 x 32 diagonal blocks of L and of U, one warp per block,
+// one column of the inverse per lane; D[2 b + (U)][l][q] = inverse[q][l], so
+// that a lane per row reads them in order.  FP64 although the factors are FP32:
+// rounded to FP32 they cost some cases a third refinement sweep.  Rows past N
+// act as the identity.
 template <class T>
-__device__ void cta_lu_solve(const T* LU, int N, const int* piv, double* x) {
-  if (threadIdx.x == 0)
-    for (int k = 0; k < N; ++k) {
-      const int p = piv[k];
-      if (p != k) {
-        const double t = x[k];
-        x[k] = x[p];
-        x[p] = t;
-      }
-    }
-  __syncthreads();
-  // Full 32-column blocks take unrolled loops (the same operations in the
-  // same order): the loads of a row segment, which do not depend on the
-  // substitution chain, then issue together instead of a few at a time.
-  for (int J0 = 0; J0 < N; J0 += 32) {
-    const int nb = min(32, N - J0);
-    if (threadIdx.x < 32) {
-      const int q = threadIdx.x;
-      double v = q < nb ? x[J0 + q] : 0.0;
-      if (nb == 32) {
-        const T* a = LU + (long long)(J0 + q) * N + J0;
+__device__ void cta_diag_inverses(const T* LU, int N, double* D) {
+  constexpr int B = kSolveBlock;
+  const int lane = threadIdx.x & 31, blocks = (N + B - 1) / B;
+  for (int k = threadIdx.x >> 5; k < 2 * blocks; k += (int)blockDim.x / 32) {
+    const int J0 = (k >> 1) * B;
+    const bool upper = k & 1;
+    auto at = [&](int r, int c) -> double {
+      return J0 + r < N && J0 + c < N ? (double)LU[(long long)(J0 + r) * N + J0 + c] : (r == c ? 1.0 : 0.0);
+    };
+    double x[B];
+    if (!upper) {
 #pragma unroll
-        for (int l = 0; l < 32; ++l) {
-          const double xl = __shfl_sync(0xffffffffu, v, l);
-          if (q > l) v -= (double)a[l] * xl;
-        }
-      } else {
-        for (int l = 0; l < nb; ++l) {
-          const double xl = __shfl_sync(0xffffffffu, v, l);
-          if (q > l && q < nb) v -= (double)LU[(long long)(J0 + q) * N + J0 + l] * xl;
-        }
-      }
-      if (q < nb) x[J0 + q] = v;
-    }
-    __syncthreads();
-    if (nb == 32) {
-#pragma unroll 2
-      for (int i = J0 + 32 + threadIdx.x; i < N; i += blockDim.x) {
-        const T* a = LU + (long long)i * N + J0;
-        double s = x[i];
+      for (int i = 0; i < B; ++i) {
+        double s = i == lane ? 1.0 : 0.0;
 #pragma unroll
-        for (int l = 0; l < 32; ++l) s -= (double)a[l] * x[J0 + l];
+        for (int l = 0; l < i; ++l) s -= at(i, l) * x[l];
         x[i] = s;
       }
     } else {
-      for (int i = J0 + nb + threadIdx.x; i < N; i += blockDim.x) {
-        double s = x[i];
-        for (int l = 0; l < nb; ++l) s -= (double)LU[(long long)i * N + J0 + l] * x[J0 + l];
-        x[i] = s;
+#pragma unroll
+      for (int i = B - 1; i >= 0; --i) {
+        double s = i == lane ? 1.0 : 0.0;
+#pragma unroll
+        for (int l = i + 1; l < B; ++l) s -= at(i, l) * x[l];
+        x[i] = s / at(i, i);
       }
     }
-    __syncthreads();
+    double* d = D + (long long)k * B * B;
+#pragma unroll
+    for (int i = 0; i < B; ++i) d[lane * B + i] = x[i];
   }
-  for (int J1 = N; J1 > 0; J1 -= 32) {
-    const int J0 = max(0, J1 - 32), nb = J1 - J0;
-    if (threadIdx.x < 32) {
-      const int q = threadIdx.x;
-      double v = q < nb ? x[J0 + q] : 0.0;
-      if (nb == 32) {
-        const T* a = LU + (long long)(J0 + q) * N + J0;
+  __syncthreads();
+}
+
+// y <- (LU)^-1 y in place (y in shared memory, already permuted, FP64
+// arithmetic), block row by block row: every warp forms the products of two or
+// four rows with the part of y that is known, along the rows (coalesced pairs; a
+// thread per row touched a line per value, and one thread replayed the row
+// exchanges before each solve: a step's solve launch with its two sweeps and
+// three FP64 residuals went from 2.07 to 0.72 ms), then one warp solves the 32 x 32 diagonal block: with the
+// block's inverse (D, FP32 factors) or by substitution (FP64 factors).
+template <class T>
+__device__ void cta_lu_solve(const T* LU, int N, const double* D, double* y) {
+  constexpr int NT = SolveCfg<T>::kThreads, kW = NT / 32, B = kSolveBlock, kR = B / kW;
+  using V2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // y[J0 + r] -= sum over columns [a, b) for the block's rows
+  auto products = [&](int J0, int nb, int a, int b) {
+    double s[kR];
+    const T* row[kR];
 #pragma unroll
-        for (int l = 31; l >= 0; --l) {
-          if (q == l) v /= (double)a[l];
-          const double xl = __shfl_sync(0xffffffffu, v, l);
-          if (q < l) v -= (double)a[l] * xl;
-        }
+    for (int k = 0; k < kR; ++k) {
+      const int r = min(wid + k * kW, nb - 1);
+      row[k] = LU + (long long)(J0 + r) * N;
+      s[k] = 0.0;
+    }
+#pragma unroll 4
+    for (int j = a + 2 * lane; j < b; j += 64) {
+      const double y0 = y[j], y1 = j + 1 < b ? y[j + 1] : 0.0;
+#pragma unroll
+      for (int k = 0; k < kR; ++k) {
+        const V2 v = *reinterpret_cast<const V2*>(row[k] + j);
+        s[k] += (double)v.x * y0 + (double)v.y * y1;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+      for (int off = 16; off; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+      if (lane == 0 && wid + k * kW < nb) y[J0 + wid + k * kW] -= s[k];
+    }
+  };
+  auto diagonal = [&](int J0, int nb, bool upper) {
+    if (wid == 0) {
+      double v = lane < nb ? y[J0 + lane] : 0.0;
+      if constexpr (sizeof(T) == 4) {
+        const double* d = D + (long long)(2 * (J0 / B) + (upper ? 1 : 0)) * B * B + lane;
+        double s = 0.0;
+#pragma unroll
+        for (int l = 0; l < B; ++l) s += d[l * B] * __shfl_sync(0xffffffffu, v, l);
+        v = s;
       } else {
-        for (int l = nb - 1; l >= 0; --l) {
-          if (q == l) v /= (double)LU[(long long)(J0 + l) * N + J0 + l];
-          const double xl = __shfl_sync(0xffffffffu, v, l);
-          if (q < l) v -= (double)LU[(long long)(J0 + q) * N + J0 + l] * xl;
+        T a[B];
+#pragma unroll
+        for (int l = 0; l < B; ++l)
+          a[l] = lane < nb && l < nb ? LU[(long long)(J0 + lane) * N + J0 + l] : (T)(l == lane ? 1 : 0);
+        if (!upper) {
+#pragma unroll
+          for (int l = 0; l < B; ++l) {
+            const double xl = __shfl_sync(0xffffffffu, v, l);
+            if (lane > l) v -= a[l] * xl;
+          }
+        } else {
+#pragma unroll
+          for (int l = B - 1; l >= 0; --l) {
+            if (lane == l) v /= a[l];
+            const double xl = __shfl_sync(0xffffffffu, v, l);
+            if (lane < l) v -= a[l] * xl;
+          }
         }
       }
-      if (q < nb) x[J0 + q] = v;
+      if (lane < nb) y[J0 + lane] = v;
     }
     __syncthreads();
-    if (nb == 32) {
-#pragma unroll 2
-      for (int i = threadIdx.x; i < J0; i += blockDim.x) {
-        const T* a = LU + (long long)i * N + J0;
-        double s = x[i];
-#pragma unroll
-        for (int l = 0; l < 32; ++l) s -= (double)a[l] * x[J0 + l];
-        x[i] = s;
-      }
-    } else {
-      for (int i = threadIdx.x; i < J0; i += blockDim.x) {
-        double s = x[i];
-        for (int l = 0; l < nb; ++l) s -= (double)LU[(long long)i * N + J0 + l] * x[J0 + l];
-        x[i] = s;
-      }
+  };
+  for (int J0 = 0; J0 < N; J0 += B) {
+    const int nb = min(B, N - J0);
+    if (J0 > 0) {
+      products(J0, nb, 0, J0);
+      __syncthreads();
     }
-    __syncthreads();
+    diagonal(J0, nb, false);
+  }
+  for (int J0 = (N - 1) / B * B; J0 >= 0; J0 -= B) {
+    const int nb = min(B, N - J0);
+    if (J0 + nb < N) {
+      products(J0, nb, J0 + nb, N);
+      __syncthreads();
+    }
+    diagonal(J0, nb, true);
   }
 }
 
@@ -599,14 +691,14 @@ constexpr double kStaleContraction = 0.5;
 // (each case decides for itself; refac counts the factorisations).
 template <class T>
 __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BCase* __restrict__ cs, double* A64, float* F32,
-                                                                int* piv_all, const double* rhs, double* gamma,
+                                                                int* perm_all, double* dinv_all, const double* rhs, double* gamma,
                                                                 const double* gamma_hist, const long long* d_step,
                                                                 int max_sweeps, double tol, int stale,
                                                                 int* has_factor, unsigned long long* refac,
                                                                 int* sweeps_out, double* res_out, int* status,
                                                                 const int* __restrict__ order) {
   constexpr int NT = SolveCfg<T>::kThreads;
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   // CTA i takes the i-th largest case: with more cases than SMs the largest
   // start first instead of forming the launch's last wave
   const int ci = order[blockIdx.x];
@@ -615,13 +707,16 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
   double* x = sm;
   double* r = sm + N;
   T* panel = reinterpret_cast<T*>(sm + 2 * N);
+  double* y = sm + 2 * N;  // the solves' vector, once the panel is done with
+  int* map = reinterpret_cast<int*>(panel + SolveCfg<T>::NB * panel_ld(N));
   double* A = A64 + b.mat_off;
-  int* piv = piv_all + b.ring_off;
+  int* perm = perm_all + b.ring_off;
   const double* bb = rhs + b.ring_off;
   int sweeps = 0;
   double rel = 0;
   if constexpr (sizeof(T) == 4) {
     T* LU = F32 + b.mat_off;
+    double* dinv = dinv_all + b.dinv_off;
     double bn = 0;
     for (int i = threadIdx.x; i < N; i += NT) bn += bb[i] * bb[i];
     bn = sqrt(cta_sum<NT>(bn));
@@ -638,13 +733,15 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
         const double* a2 = v2 ? a0 + 2LL * kW * N : a0;
         const double* a3 = v3 ? a0 + 3LL * kW * N : a0;
         double c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-#pragma unroll 8
-        for (int j = lane; j < N; j += 32) {
-          const double xj = x[j];
-          c0 += a0[j] * xj;
-          c1 += a1[j] * xj;
-          c2 += a2[j] * xj;
-          c3 += a3[j] * xj;
+#pragma unroll 4
+        for (int j = 2 * lane; j < N; j += 64) {  // N is even: 16-byte loads
+          const double2 xj = *reinterpret_cast<const double2*>(x + j);
+          const double2 v0 = *reinterpret_cast<const double2*>(a0 + j), v1_ = *reinterpret_cast<const double2*>(a1 + j);
+          const double2 v2_ = *reinterpret_cast<const double2*>(a2 + j), v3_ = *reinterpret_cast<const double2*>(a3 + j);
+          c0 += v0.x * xj.x + v0.y * xj.y;
+          c1 += v1_.x * xj.x + v1_.y * xj.y;
+          c2 += v2_.x * xj.x + v2_.y * xj.y;
+          c3 += v3_.x * xj.x + v3_.y * xj.y;
         }
         for (int off = 16; off; off >>= 1) {
           c0 += __shfl_down_sync(0xffffffffu, c0, off);
@@ -666,8 +763,10 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
       return bn > 0 ? rn / bn : 0.0;
     };
     auto sweep = [&]() {
-      cta_lu_solve<T>(LU, N, piv, r);
-      for (int i = threadIdx.x; i < N; i += NT) x[i] += r[i];
+      for (int i = threadIdx.x; i < N; i += NT) y[i] = r[perm[i]];
+      __syncthreads();
+      cta_lu_solve<T>(LU, N, dinv, y);
+      for (int i = threadIdx.x; i < N; i += NT) x[i] += y[i];
       __syncthreads();
     };
     bool done = false;
@@ -691,14 +790,18 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
     if (!done) {
       for (long long q = threadIdx.x; q < (long long)N * N; q += NT) LU[q] = (float)A[q];
       __syncthreads();
-      cta_lu_panel_smem<T>(LU, N, piv, status, panel);
+      cta_lu_factor<T>(LU, N, perm, status, panel, map, map + N);
+      __syncthreads();
+      cta_diag_inverses<T>(LU, N, dinv);
       if (threadIdx.x == 0) {
         has_factor[ci] = 1;
         atomicAdd(refac, 1ull);
       }
-      for (int i = threadIdx.x; i < N; i += NT) x[i] = bb[i];
+      for (int i = threadIdx.x; i < N; i += NT) y[i] = bb[perm[i]];
       __syncthreads();
-      cta_lu_solve<T>(LU, N, piv, x);
+      cta_lu_solve<T>(LU, N, dinv, y);
+      for (int i = threadIdx.x; i < N; i += NT) x[i] = y[i];
+      __syncthreads();
       sweeps = 0;
       while (true) {
         rel = residual();
@@ -709,11 +812,12 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
     }
     if (threadIdx.x == 0 && !(rel <= tol)) status[3] = 1;
   } else {
-    cta_lu_panel_smem<T>(A, N, piv, status, panel);
+    cta_lu_factor<T>(A, N, perm, status, panel, map, map + N);
     if (threadIdx.x == 0) atomicAdd(refac, 1ull);
-    for (int i = threadIdx.x; i < N; i += NT) x[i] = bb[i];
     __syncthreads();
-    cta_lu_solve<T>(A, N, piv, x);
+    for (int i = threadIdx.x; i < N; i += NT) x[i] = bb[perm[i]];
+    __syncthreads();
+    cta_lu_solve<T>(A, N, nullptr, x);
   }
   bool finite = true;
   for (int i = threadIdx.x; i < N; i += NT) {
@@ -913,7 +1017,8 @@ struct uvlm_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int64_t launches_per_step = 0;
-  // device
+  // device (all arrays lie in `block`)
+  void* block = nullptr;
   BCase* d_cases = nullptr;
   long long* d_pre = nullptr;  // 7 prefix arrays of n + 1
   long long* d_step = nullptr;
@@ -927,7 +1032,9 @@ struct uvlm_batch {
   double *d_vx = nullptr, *d_vy = nullptr, *d_vz = nullptr;
   double* d_A64 = nullptr;
   float* d_F32 = nullptr;
-  int* d_piv = nullptr;
+  int* d_perm = nullptr;   // per case: the row of its matrix at each row of its factors
+  double* d_dinv = nullptr;  // per case: inverses of the factors' diagonal blocks (FP32 factors)
+  long long tot_dinv = 0;
   AsmTile* d_tiles = nullptr;
   int n_tiles = 0;
   void* d_rec = nullptr;
@@ -962,16 +1069,6 @@ struct uvlm_batch {
   Error nbody(int stage, const double* tx, const double* ty, const double* tz);
   void release();
 };
-
-namespace {
-template <class T>
-Error balloc(T** p, size_t count) {
-  *p = nullptr;
-  if (count == 0) count = 1;
-  UVLM_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(p), sizeof(T) * count));
-  return ok();
-}
-}  // namespace
 
 Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   cap = (int)cfg.max_steps + 1;
@@ -1009,6 +1106,8 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
     }
     off[7] += (long long)cap * b.C;
     tot_mat += (long long)b.N * b.N;
+    b.dinv_off = tot_dinv;
+    tot_dinv += 2LL * ((b.N + kSolveBlock - 1) / kSolveBlock) * kSolveBlock * kSolveBlock;
     max_N = std::max(max_N, b.N);
     uvlm_wing_desc w{};
     w.chord = u.chord;
@@ -1036,43 +1135,49 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   const long long tot_wring = off[7];
   n_tiles = (int)tiles.size();
 
-  UVLM_TRY(balloc(&d_cases, n));
-  UVLM_TRY(balloc(&d_pre, 7 * (size_t)(n + 1)));
-  UVLM_TRY(balloc(&d_step, 1));
-  UVLM_TRY(balloc(&d_pos_init, 3 * tot_nodes));
-  UVLM_TRY(balloc(&d_pos, 3 * tot_nodes));
-  UVLM_TRY(balloc(&d_gamma, tot_rings));
-  UVLM_TRY(balloc(&d_gamma_prev, tot_rings));
-  UVLM_TRY(balloc(&d_gamma_hist, tot_rings));
-  UVLM_TRY(balloc(&d_cx, tot_rings));
-  UVLM_TRY(balloc(&d_cy, tot_rings));
-  UVLM_TRY(balloc(&d_cz, tot_rings));
-  UVLM_TRY(balloc(&d_normal, 3 * tot_rings));
-  UVLM_TRY(balloc(&d_area, tot_rings));
-  UVLM_TRY(balloc(&d_uls, 3 * tot_rings));
-  UVLM_TRY(balloc(&d_rhs, tot_rings));
-  UVLM_TRY(balloc(&d_lx, tot_lines));
-  UVLM_TRY(balloc(&d_ly, tot_lines));
-  UVLM_TRY(balloc(&d_lz, tot_lines));
-  UVLM_TRY(balloc(&d_line_uls, 3 * tot_lines));
-  UVLM_TRY(balloc(&d_wpos, 3 * tot_wnode));
-  UVLM_TRY(balloc(&d_wgamma, tot_wring));
+  // every array in one block (fifty allocations took 5 to 300 ms)
+  std::vector<std::pair<void**, size_t>> wanted;
+  auto want = [&](auto** p, size_t count) {
+    wanted.emplace_back(reinterpret_cast<void**>(p), sizeof(**p) * std::max<size_t>(count, 1));
+  };
+  want(&d_cases, n);
+  want(&d_pre, 7 * (size_t)(n + 1));
+  want(&d_step, 1);
+  want(&d_pos_init, 3 * tot_nodes);
+  want(&d_pos, 3 * tot_nodes);
+  want(&d_gamma, tot_rings);
+  want(&d_gamma_prev, tot_rings);
+  want(&d_gamma_hist, tot_rings);
+  want(&d_cx, tot_rings);
+  want(&d_cy, tot_rings);
+  want(&d_cz, tot_rings);
+  want(&d_normal, 3 * tot_rings);
+  want(&d_area, tot_rings);
+  want(&d_uls, 3 * tot_rings);
+  want(&d_rhs, tot_rings);
+  want(&d_lx, tot_lines);
+  want(&d_ly, tot_lines);
+  want(&d_lz, tot_lines);
+  want(&d_line_uls, 3 * tot_lines);
+  want(&d_wpos, 3 * tot_wnode);
+  want(&d_wgamma, tot_wring);
   if (cfg.advection == UVLM_ADVECT_RK2) {
-    UVLM_TRY(balloc(&d_wpos2, 3 * tot_wnode));
-    UVLM_TRY(balloc(&d_k1, 3 * tot_wnode));
+    want(&d_wpos2, 3 * tot_wnode);
+    want(&d_k1, 3 * tot_wnode);
   }
-  UVLM_TRY(balloc(&d_wtx, tot_wtgt));
-  UVLM_TRY(balloc(&d_wty, tot_wtgt));
-  UVLM_TRY(balloc(&d_wtz, tot_wtgt));
+  want(&d_wtx, tot_wtgt);
+  want(&d_wty, tot_wtgt);
+  want(&d_wtz, tot_wtgt);
   const long long nv = std::max({tot_rings, tot_lines, tot_wtgt});
-  UVLM_TRY(balloc(&d_vx, nv));
-  UVLM_TRY(balloc(&d_vy, nv));
-  UVLM_TRY(balloc(&d_vz, nv));
-  UVLM_TRY(balloc(&d_A64, tot_mat));
-  if (mixed()) UVLM_TRY(balloc(&d_F32, tot_mat));
-  UVLM_TRY(balloc(&d_piv, tot_rings));
-  UVLM_TRY(balloc(&d_tiles, n_tiles));
-  UVLM_CUDA_TRY(cudaMalloc(&d_rec, (size_t)tot_rec * (mixed() ? sizeof(RecF) : sizeof(RecD))));
+  want(&d_vx, nv);
+  want(&d_vy, nv);
+  want(&d_vz, nv);
+  want(&d_A64, tot_mat);
+  if (mixed()) want(&d_F32, tot_mat);
+  want(&d_perm, tot_rings);
+  if (mixed()) want(&d_dinv, tot_dinv);
+  want(&d_tiles, n_tiles);
+  want(reinterpret_cast<char**>(&d_rec), (size_t)tot_rec * (mixed() ? sizeof(RecF) : sizeof(RecD)));
   // partial sums: the largest stage at the last step bounds every step
   {
     const long long s = cfg.max_steps - 1;
@@ -1098,17 +1203,26 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
       partial_cap = std::max(partial_cap, nbody_batch_partial_doubles(prec(), in.data(), n));
     }
   }
-  UVLM_TRY(balloc(&d_partial, partial_cap));
-  UVLM_TRY(balloc(&d_in, n));
-  UVLM_TRY(balloc(&d_plan, n));
-  UVLM_TRY(balloc(&d_totals, 4));
-  UVLM_TRY(balloc(&d_status, 4));
-  UVLM_TRY(balloc(&d_sweeps, n));
-  UVLM_TRY(balloc(&d_solve_order, n));
-  UVLM_TRY(balloc(&d_has_factor, n));
-  UVLM_TRY(balloc(&d_refac, 1));
-  UVLM_TRY(balloc(&d_res, n));
-  UVLM_TRY(balloc(&d_loads, (size_t)cfg.max_steps * n * 3));
+  want(&d_partial, partial_cap);
+  want(&d_in, n);
+  want(&d_plan, n);
+  want(&d_totals, 4);
+  want(&d_status, 4);
+  want(&d_sweeps, n);
+  want(&d_solve_order, n);
+  want(&d_has_factor, n);
+  want(&d_refac, 1);
+  want(&d_res, n);
+  want(&d_loads, (size_t)cfg.max_steps * n * 3);
+
+  size_t bytes = 0;
+  for (const auto& w : wanted) bytes += (w.second + 255) & ~(size_t)255;
+  UVLM_CUDA_TRY(cudaMalloc(&block, bytes));
+  char* at = static_cast<char*>(block);
+  for (const auto& w : wanted) {
+    *w.first = at;
+    at += (w.second + 255) & ~(size_t)255;
+  }
 
   std::vector<long long> flat;
   for (int k = 0; k < 7; ++k) flat.insert(flat.end(), pre[k].begin(), pre[k].end());
@@ -1133,13 +1247,12 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   UVLM_CUDA_TRY(cudaMemset(d_has_factor, 0, sizeof(int) * n));
   UVLM_CUDA_TRY(cudaMemset(d_refac, 0, sizeof(unsigned long long)));
   UVLM_CUDA_TRY(cudaMemset(d_loads, 0, sizeof(double) * (size_t)cfg.max_steps * n * 3));
-  const size_t solve_smem = sizeof(double) * 2 * (size_t)max_N + panel_smem_bytes(max_N, mixed() ? 4 : 8);
   if (mixed())
     UVLM_CUDA_TRY(cudaFuncSetAttribute(b_solve_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)solve_smem));
+                                       (int)solve_smem_bytes<float>(max_N)));
   else
     UVLM_CUDA_TRY(cudaFuncSetAttribute(b_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)solve_smem));
+                                       (int)solve_smem_bytes<double>(max_N)));
   nb_grids = nbody_batch_grids(prec(), num_sms);
   grid = num_sms * 8;
   return ok();
@@ -1238,15 +1351,14 @@ Error uvlm_batch::enqueue_step() {
   b_rhs_kernel<<<grid, 256, 0, st>>>(d_cases, P, n, d_vx, d_vy, d_vz, d_uls, d_normal, d_rhs);
   UVLM_LAUNCH_CHECK();
   // solve
-  const size_t smem = sizeof(double) * 2 * (size_t)max_N + panel_smem_bytes(max_N, mixed() ? 4 : 8);
   if (mixed())
-    b_solve_kernel<float><<<n, SolveCfg<float>::kThreads, smem, st>>>(d_cases, d_A64, d_F32, d_piv, d_rhs, d_gamma,
-                                                          d_gamma_hist, d_step, cfg.refine_max_iter, cfg.refine_tol, cfg.stale_factors,
-                                                          d_has_factor, d_refac, d_sweeps, d_res, d_status, d_solve_order);
+    b_solve_kernel<float><<<n, SolveCfg<float>::kThreads, solve_smem_bytes<float>(max_N), st>>>(
+        d_cases, d_A64, d_F32, d_perm, d_dinv, d_rhs, d_gamma, d_gamma_hist, d_step, cfg.refine_max_iter,
+        cfg.refine_tol, cfg.stale_factors, d_has_factor, d_refac, d_sweeps, d_res, d_status, d_solve_order);
   else
-    b_solve_kernel<double><<<n, SolveCfg<double>::kThreads, smem, st>>>(d_cases, d_A64, d_F32, d_piv, d_rhs, d_gamma,
-                                                           d_gamma_hist, d_step, 0, 0.0,
-                                                           0, d_has_factor, d_refac, d_sweeps, d_res, d_status, d_solve_order);
+    b_solve_kernel<double><<<n, SolveCfg<double>::kThreads, solve_smem_bytes<double>(max_N), st>>>(
+        d_cases, d_A64, d_F32, d_perm, nullptr, d_rhs, d_gamma, d_gamma_hist, d_step, 0, 0.0, 0, d_has_factor,
+        d_refac, d_sweeps, d_res, d_status, d_solve_order);
   UVLM_LAUNCH_CHECK();
   // loads: line velocities from the bound sheet (new circulation) and the wake
   b_line_prep_kernel<<<grid, 256, 0, st>>>(d_cases, P, n, d_step, d_pos, d_pos_init, d_lx, d_ly, d_lz, d_line_uls);
@@ -1285,13 +1397,8 @@ void uvlm_batch::release() {
   if (graph) cudaGraphDestroy(graph);
   exec = nullptr;
   graph = nullptr;
-  void* ptrs[] = {d_cases, d_pre, d_step, d_pos_init, d_pos, d_gamma, d_gamma_prev, d_gamma_hist, d_cx, d_cy, d_cz,
-                  d_normal,
-                  d_area, d_uls, d_rhs, d_lx, d_ly, d_lz, d_line_uls, d_wpos, d_wpos2, d_k1, d_wgamma, d_wtx,
-                  d_wty, d_wtz, d_vx, d_vy, d_vz, d_A64, d_F32, d_piv, d_tiles, d_rec, d_partial, d_in, d_plan,
-                  d_totals, d_status, d_sweeps, d_res, d_loads, d_has_factor, d_refac, d_solve_order};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  cudaFree(block);
+  block = nullptr;
   if (st) cudaStreamDestroy(st);
   st = nullptr;
 }
