@@ -225,3 +225,21 @@ def test_shipped_morphing_weights_beat_extrapolation():
     assert res["mlp"][0] < 0.5 * res["extrapolate"][0]
     scale = np.max(np.abs(res["extrapolate"][1][:, 1:]))
     np.testing.assert_allclose(res["mlp"][1][:, 1:], res["extrapolate"][1][:, 1:], rtol=0, atol=1e-6 * scale)
+
+
+@pytest.mark.parametrize("n", [1, 15, 63, 65, 2047, 2113])
+def test_mlp_gradients_at_tile_and_split_edges(n):
+    """Batches at the edges of the 64-row tiles, the 16-row inner steps and the splits of the weight gradients over the
+    batch, with the tolerances of the autograd comparison."""
+    from uvlm_b200.warmstart import MLP
+
+    rng = np.random.default_rng(n)
+    net = MLP(seed=n)
+    X = rng.standard_normal((n, 8)).astype(np.float32)
+    T = (0.3 * rng.standard_normal(n)).astype(np.float32)
+    net.set_normalization(rng.standard_normal(8) * 0.1, 0.5 + rng.random(8), 0.7)
+    g_ref, loss_ref, y_ref = _torch_reference(net, X, T)
+    np.testing.assert_allclose(net.forward(X), y_ref, rtol=1e-4, atol=1e-5 * np.max(np.abs(y_ref)))
+    g, loss = net.gradients(X, T)
+    assert abs(loss - loss_ref) <= 1e-5 * abs(loss_ref)
+    assert np.max(np.abs(g - g_ref)) <= 1e-4 * np.max(np.abs(g_ref))

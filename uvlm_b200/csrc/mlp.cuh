@@ -44,6 +44,8 @@ struct Mlp {
   float* act = nullptr;   // [depth+1][cap][hidden]: layer inputs
   float* pre = nullptr;   // [depth][cap][hidden]: pre-activations
   float* dact = nullptr;  // [2][cap][hidden]
+  double* colpart = nullptr;  // partial column sums [ceil(cap / 128)][hidden]
+  float* part = nullptr;  // partial sums of a weight gradient (training only)
   float* y = nullptr;     // [cap]
   float* dy = nullptr;    // [cap]
   double* loss = nullptr; // [1]
