@@ -121,3 +121,28 @@ def test_velocity_at_points_of_the_current_state(precision):
            + o.sheet_induced_velocity(st["wake_pos"], st["wake_gamma"], g) + np.array([1.0, 0.0, 0.0]))
     tol = 1e-12 if precision == "fp64" else 1e-6
     assert np.max(np.abs(got - ref)) <= tol * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("n", [64, 65, 127, 128, 129, 192, 257, 321, 1088, 2305, 4161])
+def test_lu_of_a_general_matrix_at_its_block_edges(n):
+    """Factors and solves of matrices whose pivots lie anywhere, at the edges of the 64-wide panels, of the 64-row and
+    64-column CTAs behind a panel and of the panel's clusters (n = 4161 starts with panels of more than one cluster).
+    Bounds: n rounding errors per entry, times a growth of n^(2/3) (random matrices with partial pivoting)."""
+    import uvlm_b200 as M
+
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n))
+    b = rng.standard_normal(n)
+    x, _ = M.dense_solve(A, b, "fp64")
+    res = np.max(np.abs(A @ x - b)) / (np.linalg.norm(A, np.inf) * np.max(np.abs(x)))
+    assert res <= n ** (5 / 3) * np.finfo(np.float64).eps
+    A32 = A.astype(np.float32)
+    LU, ipiv = M.lu_factor_f32(A32, "simt")
+    assert np.all(ipiv >= np.arange(n)) and np.all(ipiv < n)
+    PA = A32.astype(np.float64)
+    for k, p in enumerate(ipiv):
+        if p != k:
+            PA[[k, p]] = PA[[p, k]]
+    L = np.tril(LU, -1).astype(np.float64) + np.eye(n)
+    err = np.max(np.abs(PA - L @ np.triu(LU).astype(np.float64))) / np.max(np.abs(A32))
+    assert err <= n ** (5 / 3) * np.finfo(np.float32).eps

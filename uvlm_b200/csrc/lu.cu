@@ -387,7 +387,7 @@ struct TspScratch {
 
 template <class T>
 constexpr size_t tsp_smem() {
-  return sizeof(T) * ((size_t)kTspTop + (size_t)kTspRows * kTspLd) + sizeof(TspScratch);
+  return sizeof(T) * ((size_t)kTspTop + (size_t)kTspRows * kTspLd + kLuNB) + sizeof(TspScratch);
 }
 
 // One row of the panel (64 values from column k0) from A into registers;
@@ -452,6 +452,18 @@ __device__ __forceinline__ void tsp_ld8(const T* p, T (&o)[8]) {
   }
 }
 
+// Eight consecutive values to a 16-byte aligned address.
+template <class T>
+__device__ __forceinline__ void tsp_st8(T* p, const T (&o)[8]) {
+  if constexpr (sizeof(T) == 4) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(o[0], o[1], o[2], o[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(o[4], o[5], o[6], o[7]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) reinterpret_cast<double2*>(p)[q] = make_double2(o[2 * q], o[2 * q + 1]);
+  }
+}
+
 // uc[8 jc + t] = v[8 jc + t] (column c0 + 8 jc + t) for the 8-column chunks
 // that reach column c (= c0 + k) and lie left of column 64 (the shifted row's
 // entries past column 63 are dead); the chunk holding column c also writes
@@ -493,17 +505,30 @@ __device__ __forceinline__ void tsp_axpy(T (&v)[kLuNB], T l, const T* uc, int c0
   }
 }
 
-// The elimination of step c = c0 + k against the pivot row uc: l = v[k] /
-// uc[k] into *lk, then v[j] -= l uc[j] for j > k.  A zero pivot leaves the
-// row as it is and returns v[k] as its multiplier.
+// x / piv from r = 1 / piv: a product and one correction by its residual,
+// where r is far enough from the ends of the range for both; else a division.
+__device__ __forceinline__ float tsp_rcp(float x) { return __frcp_rn(x); }
+__device__ __forceinline__ double tsp_rcp(double x) { return __drcp_rn(x); }
+
 template <class T>
-__device__ __forceinline__ void tsp_eliminate(T (&v)[kLuNB], const T* uc, int c0, int k, T* lk) {
+__device__ __forceinline__ T tsp_quotient(T x, T piv, T r) {
+  constexpr T big = sizeof(T) == 8 ? (T)0x1p+900 : (T)0x1p+100f;
+  if (!(fabs(r) < big && fabs(r) > (T)1 / big)) return x / piv;
+  const T q = x * r;
+  return fma(fma(-q, piv, x), r, q);
+}
+
+// The elimination of step c = c0 + k against the pivot row uc (reciprocal of
+// the pivot in r): l = v[k] / uc[k] into *lk, then v[j] -= l uc[j] for j > k.
+// A zero pivot leaves the row as it is and returns v[k] as its multiplier.
+template <class T>
+__device__ __forceinline__ void tsp_eliminate(T (&v)[kLuNB], const T* uc, T r, int c0, int k, T* lk) {
   const T piv = uc[k];
   if (piv == (T)0) {
     *lk = v[k];
     return;
   }
-  const T l = v[k] / piv;
+  const T l = tsp_quotient<T>(v[k], piv, r);
   *lk = l;
   tsp_axpy<T>(v, l, uc, c0, k + 1);
 }
@@ -528,7 +553,7 @@ __device__ __forceinline__ void tsp_shift8(T (&v)[kLuNB]) {
 // column-by-column factorisation, in the same order.  Every thread of the
 // CTA calls it.
 template <class T>
-__device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T* Lrow, TspScratch& sc,
+__device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T* Lrow, T* Rcp, TspScratch& sc,
                           int* out) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int steps = min(kLuNB, R);
@@ -548,6 +573,9 @@ __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T*
           sc.khi[par][warp] = whi;
           sc.klo[par][warp] = wlo;
         }
+        // every row's reciprocal while the keys settle: the pivot's is then
+        // ready with its row, and no division follows the second barrier
+        const T r = tsp_rcp(v[k]);
         __syncthreads();
         const unsigned ph = lane < kTspRows / 32 ? sc.khi[par][lane] : 0u;
         const unsigned pl = lane < kTspRows / 32 ? sc.klo[par][lane] : 0u;
@@ -557,11 +585,12 @@ __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T*
         if (alive && hi == bhi && lo == blo) {
           out[c] = 0x1000 - (int)(blo & 0x1FFFu);
           sc.pivrow[c] = tid;
+          Rcp[c] = r;
           tsp_publish<T>(u, c0, k, v);
           alive = false;
         }
         __syncthreads();
-        if (alive) tsp_eliminate<T>(v, u, c0, k, lrow + c);
+        if (alive) tsp_eliminate<T>(v, u, Rcp[c], c0, k, lrow + c);
       }
     }
     tsp_shift8<T>(v);
@@ -572,31 +601,38 @@ __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T*
 
 template <class T>
 __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda, int n, int k0, int* ipiv,
-                                                                   int* err, int local) {
+                                                                   int* moves, int* err) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smraw[];
   T* Top = reinterpret_cast<T*>(smraw);  // [64][64]: the pivot rows' U parts (columns c .. 63 of row c)
   T* Lrow = Top + kTspTop;               // [256][kTspLd]: multipliers of each thread's row
-  TspScratch& sc = *reinterpret_cast<TspScratch*>(Lrow + kTspRows * kTspLd);
+  T* Rcp = Lrow + kTspRows * kTspLd;     // [64]: reciprocals of the pivots
+  TspScratch& sc = *reinterpret_cast<TspScratch*>(Rcp + kLuNB);
   const int P = (int)cl.num_blocks(), bid = (int)cl.block_rank(), tid = threadIdx.x;
   const int m = n - k0;
   const int rb = bid * kTspRows;
   const int nloc = max(0, min(kTspRows, m - rb));
   T v[kLuNB];
 
-  // ---- phase 1: this CTA's rows (with local pivoting, only the first CTA's:
+  if (bid == 0)
+    for (int q = tid; q < m && q < kTspMaxRows; q += kTspRows) {
+      sc.at[q] = (short)q;
+      sc.pos[q] = (short)q;
+    }
+
+  // ---- phase 1: this CTA's rows (with local pivoting the cluster is one CTA:
   // the pivots are chosen among the panel's top 256 rows)
-  if (!local || bid == 0) {
+  {
     const bool alive = tid < nloc;
     if (alive) tsp_load_row<T>(A, (long long)(k0 + rb + tid) * lda + k0, v);
-    const int k = tsp_factor<T>(v, alive, rb + tid, nloc, Top, Lrow, sc, sc.list);
+    const int k = tsp_factor<T>(v, alive, rb + tid, nloc, Top, Lrow, Rcp, sc, sc.list);
     if (tid == 0) sc.cnt[0] = k;
   }
 
   // ---- phase 2: 4-ary tournament tree over the cluster; the merges factor
   // the candidates' original rows
-  for (int step = 1; step < (local ? 1 : P); step *= 4) {
+  for (int step = 1; step < P; step *= 4) {
     cl.sync();  // the candidate lists of this level are final
     if ((bid % (4 * step)) == 0 && bid + step < P) {
       if (tid == 0)
@@ -615,21 +651,16 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
       }
       const bool alive = tid < R;
       if (alive) tsp_load_row<T>(A, (long long)(k0 + myid) * lda + k0, v);
-      const int k = tsp_factor<T>(v, alive, myid, R, Top, Lrow, sc, sc.list);
+      const int k = tsp_factor<T>(v, alive, myid, R, Top, Lrow, Rcp, sc, sc.list);
       if (tid == 0) sc.cnt[0] = k;
     }
   }
-  cl.sync();  // the root's Top, Lrow, pivrow and list are final
+  cl.sync();  // every read of another CTA's lists is over: all but the root may leave
+  if (bid > 0) return;
 
-  // ---- phase 3: the swap sequence (CTA 0), sent to every CTA; the row map
-  for (int q = tid; q < m; q += kTspRows) {
-    sc.at[q] = (short)q;
-    sc.pos[q] = (short)q;
-  }
-  __syncthreads();
-  const int kb = kLuNB;  // m >= 64: the launcher's condition
-  if (bid == 0 && tid == 0) {
-    for (int i = 0; i < kb; ++i) {
+  // ---- phase 3: the swap sequence and the moves it amounts to
+  if (tid == 0) {
+    for (int i = 0; i < kLuNB; ++i) {  // m >= 64: the launcher's condition
       const int r = sc.list[i];
       const int qn = sc.pos[r];
       const int ri = sc.at[i];
@@ -638,76 +669,148 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
       sc.at[qn] = (short)ri;
       sc.pos[ri] = (short)qn;
       sc.seq[i] = qn;
-      ipiv[k0 + i] = k0 + qn;
     }
   }
   __syncthreads();
-  if (bid == 0)
-    for (int q = tid; q < (P - 1) * kb; q += kTspRows) {
-      const int c = 1 + q / kb, i = q - (c - 1) * kb;
-      *cl.map_shared_rank(&sc.seq[i], c) = sc.seq[i];
-    }
-  cl.sync();
-  if (bid > 0) {
-    if (tid == 0)
-      for (int i = 0; i < kb; ++i) {
-        const int qn = sc.seq[i];
-        const short t = sc.at[i];
-        sc.at[i] = sc.at[qn];
-        sc.at[qn] = t;
-      }
-    // U11 from the root
-    const T* root = cl.map_shared_rank(Top, 0);
-    for (int q = tid; q < kLuNB * kLuNB; q += kTspRows) Top[q] = root[q];
+  if (tid < kLuNB) {
+    const int q = sc.seq[tid];
+    ipiv[k0 + tid] = k0 + q;
+    moves[tid] = sc.list[tid];
+    moves[kLuNB + tid] = q >= kLuNB ? q : -1;
+    moves[2 * kLuNB + tid] = sc.at[q];
+    if (Top[tid * kLuNB + tid] == (T)0) atomicExch(err + 1, 1);
   }
-  __syncthreads();
-  // this CTA's rows below the top block: original values by new position
-  const int p = rb + tid;
-  const bool mine = tid < nloc && p >= kb;
-  if (mine) tsp_load_row<T>(A, (long long)(k0 + sc.at[p]) * lda + k0, v);
-  cl.sync();  // every CTA holds its original rows before any row of A is overwritten
 
-  // ---- phase 4: the top block L11\U11 from the root, then L21 from l U11 = a
-  if (bid == 0) {
-    for (int q = tid; q < kb * kLuNB; q += kTspRows) {
-      const int i = q / kLuNB, c = q - i * kLuNB;
-      A[(long long)(k0 + i) * lda + k0 + c] = c < i ? Lrow[sc.pivrow[i] * kTspLd + c] : Top[q];
-    }
-    if (tid < kb && Top[tid * kLuNB + tid] == (T)0) atomicExch(err + 1, 1);
-    __syncthreads();  // the root's Lrow is read before the substitution below overwrites it
+  // ---- phase 4: the displaced rows of the panel, then its top block L11\U11
+  constexpr int kPer = kLuNB * kLuNB / kTspRows;
+  T d[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int q = tid + u * kTspRows, to = sc.seq[q >> 6];
+    d[u] = to >= kLuNB ? A[(long long)(k0 + sc.at[to]) * lda + k0 + (q & (kLuNB - 1))] : (T)0;
   }
-  if (mine) {
-    // by columns: the operations, in order, of eliminating this row against
-    // the pivot rows in a column-by-column factorisation
-    T* lrow = Lrow + tid * kTspLd;
+  __syncthreads();  // the old top rows are read
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int q = tid + u * kTspRows, i = q >> 6, c = q & (kLuNB - 1), to = sc.seq[i];
+    if (to >= kLuNB) A[(long long)(k0 + to) * lda + k0 + c] = d[u];
+    A[(long long)(k0 + i) * lda + k0 + c] = c < i ? Lrow[sc.pivrow[i] * kTspLd + c] : Top[q];
+  }
+}
+
+// After a tournament panel, in one launch of 64-thread CTAs with one row or
+// column of the matrix per thread:
+//   rows:          L21(r) from l U11 = a(r) for the rows below the top block;
+//   right columns: the panel's row moves, then U12 = L11^-1 A12 (and its
+//                  transpose into ut);
+//   left columns:  the row moves.
+// moves: for i < 64 the old row of new row i, a row below the top block that a
+// top row moves to (or -1), and that top row, relative to k0.  The row and
+// column solves are the same elimination of 64 values in registers against
+// the rows of U11 or the columns of L11 in shared memory, eight columns
+// unrolled in a run-time loop.  In the panel's cluster the rows' part kept
+// only its <= 16 SMs busy, 256 rows each (20 us a panel), and a fully
+// unrolled triangular solve per column (a kernel of its own) spent 20 us a
+// panel on fetching its instructions: APPLY_FIGURES.
+constexpr int kApplyThreads = 64;
+
+template <class T>
+__global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, int n, int k0,
+                                                                 const int* __restrict__ moves, int row_ctas,
+                                                                 int right_ctas, T* ut, int ldut) {
+  constexpr int kLd = kLuNB + 16 / sizeof(T);
+  __shared__ __align__(16) T M[kLuNB * kLd];  // row s: what step s eliminates with
+  __shared__ T Rcp[kLuNB];
+  __shared__ int mv[3 * kLuNB];
+  const int tid = threadIdx.x;
+  const bool rows = (int)blockIdx.x < row_ctas;
+  const bool right = !rows && (int)blockIdx.x < row_ctas + right_ctas;
+  for (int q = tid; q < 3 * kLuNB; q += kApplyThreads) mv[q] = moves[q];
+  if (rows || right) {
+    T t[16];
+    for (int i0 = 0; i0 < kLuNB; i0 += 16) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) t[i] = A[(long long)(k0 + i0 + i) * lda + k0 + tid];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) M[rows ? (i0 + i) * kLd + tid : tid * kLd + i0 + i] = t[i];
+    }
+  }
+  __syncthreads();
+  T v[kLuNB];
+  if (rows) {
+    Rcp[tid] = tsp_rcp(M[tid * kLd + tid]);
+    __syncthreads();
+    const int row = k0 + kLuNB + blockIdx.x * kApplyThreads + tid;
+    if (row >= n) return;
+    const long long off = (long long)row * lda + k0;
+    tsp_load_row<T>(A, off, v);
+    const bool aligned = (reinterpret_cast<uintptr_t>(A + off) & 15) == 0;
 #pragma unroll 1
     for (int c0 = 0; c0 < kLuNB; c0 += 8) {
+      T l[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        const int c = c0 + k;
-        tsp_eliminate<T>(v, Top + c * kLuNB + c0, c0, k, lrow + c);
-        if (Top[c * kLuNB + c] == (T)0) lrow[c] = (T)0;  // a zero pivot: multiplier 0 (the factor is singular)
+        const T* u = M + (c0 + k) * kLd + c0;
+        const T piv = u[k];
+        l[k] = piv == (T)0 ? (T)0 : tsp_quotient<T>(v[k], piv, Rcp[c0 + k]);  // 0: the factor is singular
+        tsp_axpy<T>(v, l[k], u, c0, k + 1);
+      }
+      if (aligned) {
+        tsp_st8<T>(A + off + c0, l);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) A[off + c0 + k] = l[k];
       }
       tsp_shift8<T>(v);
     }
+    return;
   }
-  __syncthreads();
-  for (int q = tid; q < nloc * kLuNB; q += kTspRows) {
-    const int r = q >> 6, c = q & (kLuNB - 1);
-    if (rb + r >= kb) A[(long long)(k0 + rb + r) * lda + k0 + c] = Lrow[r * kTspLd + c];
+  const int col = right ? k0 + kLuNB + ((int)blockIdx.x - row_ctas) * kApplyThreads + tid
+                        : ((int)blockIdx.x - row_ctas - right_ctas) * kApplyThreads + tid;
+  if (col >= (right ? n : k0)) return;
+  T* a = A + (long long)k0 * lda + col;
+#pragma unroll
+  for (int i = 0; i < kLuNB; ++i) v[i] = a[(long long)mv[i] * lda];
+#pragma unroll 1
+  for (int i0 = 0; i0 < kLuNB; i0 += 16) {
+    T y[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      y[i] = mv[kLuNB + i0 + i] >= 0 ? a[(long long)mv[2 * kLuNB + i0 + i] * lda] : (T)0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (mv[kLuNB + i0 + i] >= 0) a[(long long)mv[kLuNB + i0 + i] * lda] = y[i];
   }
-  // every access to another CTA's shared memory came before the last cluster
-  // barrier, so the CTAs may leave independently
+  if (!right) {
+#pragma unroll
+    for (int i = 0; i < kLuNB; ++i) a[(long long)i * lda] = v[i];
+    return;
+  }
+#pragma unroll 1
+  for (int c0 = 0; c0 < kLuNB; c0 += 8) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      tsp_axpy<T>(v, v[k], M + (c0 + k) * kLd + c0, c0, k + 1);
+      a[(long long)(c0 + k) * lda] = v[k];
+    }
+    if (ut) {
+      T o[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) o[k] = v[k];
+      tsp_st8<T>(ut + (long long)(col - k0 - kLuNB) * ldut + c0, o);  // ldut = 64
+    }
+    tsp_shift8<T>(v);
+  }
 }
 
 // Launches the tournament panel; false when it cannot run (a panel narrower
 // than 64 columns, too many rows for one cluster, or the cluster cannot be
 // formed).
 template <class T>
-bool launch_panel_tsp(T* A, int n, int k0, int kb, int* ipiv, int* err, bool local, cudaStream_t st) {
+bool launch_panel_tsp(T* A, int n, int k0, int kb, int* ipiv, int* moves, int* err, bool local, cudaStream_t st) {
   const int m = n - k0;
-  const int P = ceil_div(m, kTspRows);
-  if (P > kTspMaxCtas || kb != kLuNB || m < kLuNB) return false;
+  if (m > kTspMaxRows || kb != kLuNB || m < kLuNB) return false;
+  const int P = local ? 1 : ceil_div(m, kTspRows);
   auto kern = lu_panel_tsp_kernel<T>;
   const size_t smem = tsp_smem<T>();
   static PerDeviceOnce configured;
@@ -739,7 +842,7 @@ bool launch_panel_tsp(T* A, int n, int k0, int kb, int* ipiv, int* err, bool loc
     cudaGetLastError();
     return false;
   }
-  if (cudaLaunchKernelEx(&cfg, kern, A, n, n, k0, ipiv, err, local ? 1 : 0) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, kern, A, n, n, k0, ipiv, moves, err) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
@@ -1015,61 +1118,74 @@ __global__ void __launch_bounds__(256, 1) gemm_update_f64_kernel(double* C, int 
   }
 }
 
-// Inverses of the diagonal blocks: thread j < 64 forms column j of L_II^-1
-// (unit lower), thread 64 + j column j of U_II^-1.
-template <class T>
-__global__ void diag_inverse_kernel(const T* LU, int n, T* dinv_l, T* dinv_u) {
-  const int I = blockIdx.x;
-  const int r0 = I * kTriB;
-  const int nb = min(kTriB, n - r0);
-  T* Li = dinv_l + (long long)I * kTriB * kTriB;
-  T* Ui = dinv_u + (long long)I * kTriB * kTriB;
-  const int j = threadIdx.x & (kTriB - 1);
-  const bool upper = threadIdx.x >= kTriB;
-  if (!upper) {
-    for (int i = 0; i < kTriB; ++i) {
-      T x = (i == j) ? (T)1 : (T)0;
-      if (i < nb && j < nb && i > j) {
-        for (int s = j; s < i; ++s) x -= LU[(long long)(r0 + i) * n + r0 + s] * Li[s * kTriB + j];
-      }
-      if (i >= nb || j >= nb) x = (i == j) ? (T)1 : (T)0;
-      Li[i * kTriB + j] = (i < j) ? (T)0 : x;
-    }
-  } else {
-    for (int i = kTriB - 1; i >= 0; --i) {
-      T x = (T)0;
-      if (i < nb && j < nb && i <= j) {
-        x = (i == j) ? (T)1 : (T)0;
-        for (int s = i + 1; s <= j; ++s) x -= LU[(long long)(r0 + i) * n + r0 + s] * Ui[s * kTriB + j];
-        x = x / LU[(long long)(r0 + i) * n + r0 + i];
-      } else if (i == j) {
-        x = (T)1;
-      }
-      Ui[i * kTriB + j] = x;
-    }
-  }
-}
+// What the solves need beside the factors, one CTA of 64 threads each:
+// CTA 2 I:     L_II^-1, one column per thread;
+// CTA 2 I + 1: U_II^-1, one column per thread;
+// CTAs from 2 nblk: perm[k], the row of b that lands in row k after the swap
+// sequence, one k per thread.
+// An inverse's column stays in registers (a forward or backward elimination
+// against the block in shared memory; blocks past the matrix are padded with
+// the identity).  perm[k] is found by walking the swaps back from position k:
+// swap j <= k moves row p_j >= j to position j, so only p_j == position
+// matters; four compares per 16-byte read, independent for every k (one
+// chain of n dependent swaps took 81 us at n = 2304, the inverses from global
+// memory 108: FINISH_FIGURES).
+constexpr int kFinishThreads = kTriB;
 
-// perm[k] = row of b that lands in row k after the LAPACK-style swap sequence.
-__global__ void ipiv_to_perm_kernel(const int* ipiv, int n, int* perm) {
-  // sp: the permutation, si: the pivot sequence (both staged by every thread;
-  // the swaps themselves are one sequential chain in shared memory)
-  extern __shared__ int sp[];
-  int* si = sp + n;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    sp[k] = k;
-    si[k] = ipiv[k];
+template <class T>
+__global__ void __launch_bounds__(kFinishThreads) lu_finish_kernel(const T* LU, int n, int nblk, T* dinv_l, T* dinv_u,
+                                                                   const int* __restrict__ ipiv, int* perm) {
+  const int tid = threadIdx.x;
+  if ((int)blockIdx.x >= 2 * nblk) {
+    const int k = ((int)blockIdx.x - 2 * nblk) * kFinishThreads + tid;
+    if (k >= n) return;
+    int at = ipiv[k], j = k - 1;
+    for (; j >= 0 && (j & 3) != 3; --j)
+      if (ipiv[j] == at) at = j;
+#pragma unroll 4
+    for (; j >= 0; j -= 4) {
+      const int4 p = *reinterpret_cast<const int4*>(ipiv + j - 3);
+      if (p.w == at) at = j;
+      if (p.z == at) at = j - 1;
+      if (p.y == at) at = j - 2;
+      if (p.x == at) at = j - 3;
+    }
+    perm[k] = at;
+    return;
+  }
+  constexpr int kLd = kTriB + 16 / sizeof(T);
+  __shared__ __align__(16) T M[kTriB * kLd];  // M[s][r] = entry (r, s) of the block; rows reversed for U
+  __shared__ T Rcp[kTriB];
+  const int I = blockIdx.x >> 1, r0 = I * kTriB, nb = min(kTriB, n - r0);
+  const bool upper = blockIdx.x & 1;
+  // U reversed in both directions is lower triangular too: step s of the
+  // elimination is row 63 - s of U
+#pragma unroll 16
+  for (int i = 0; i < kTriB; ++i) {
+    const T x = i < nb && tid < nb ? LU[(long long)(r0 + i) * n + r0 + tid] : (T)(i == tid);
+    M[upper ? (kTriB - 1 - tid) * kLd + kTriB - 1 - i : tid * kLd + i] = x;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < n; ++k) {
-      const int p = si[k];
-      const int t = sp[k];
-      sp[k] = sp[p];
-      sp[p] = t;
+  if (upper) {
+    Rcp[tid] = tsp_rcp(M[tid * kLd + tid]);
+    __syncthreads();
+  }
+  T v[kTriB];
+#pragma unroll
+  for (int i = 0; i < kTriB; ++i) v[i] = (T)(i == tid);
+  T* out = (upper ? dinv_u : dinv_l) + (long long)I * kTriB * kTriB;
+#pragma unroll 1
+  for (int c0 = 0; c0 < kTriB; c0 += 8) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int s = c0 + k;
+      const T* u = M + s * kLd + c0;
+      const T x = upper ? tsp_quotient<T>(v[k], u[k], Rcp[s]) : v[k];
+      tsp_axpy<T>(v, x, u, c0, k + 1);
+      out[upper ? (kTriB - 1 - s) * kTriB + kTriB - 1 - tid : s * kTriB + tid] = x;
     }
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += blockDim.x) perm[k] = sp[k];
+    tsp_shift8<T>(v);
+  }
 }
 
 constexpr int kTriBatch = 8;  // block rows a CTA can consume in one pass
@@ -1131,6 +1247,19 @@ __global__ void __launch_bounds__(256) trsv_kernel(const T* __restrict__ LU, int
   }
   __syncthreads();
   const int deps = kLower ? I : nblk - 1 - I;
+  // what does not depend on other block rows is read ahead of the waits: the
+  // next block of the row and the inverse of the diagonal block
+  const T* rp = LU + (long long)(r0 + (row < nb ? row : 0)) * n;
+  T a[16], d[16];
+  auto fetch = [&](int pos) {
+    const int c0 = (kLower ? pos : nblk - 1 - pos) * kTriB + quarter * 16;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) a[c] = (c0 + c < n) ? rp[c0 + c] : (T)0;
+  };
+  const T* D = dinv + (long long)I * kTriB * kTriB + (long long)row * kTriB + quarter * 16;
+#pragma unroll
+  for (int c = 0; c < 16; ++c) d[c] = D[c];
+  if (deps > 0) fetch(0);
   int done = 0;
   while (done < deps) {
     const int cnt = wait_ready(flags, done, deps - done, kLower, nblk, epoch, err);
@@ -1143,17 +1272,10 @@ __global__ void __launch_bounds__(256) trsv_kernel(const T* __restrict__ LU, int
     }
     __syncthreads();
     V s = 0;
-    if (row < nb) {
-      const T* rp = LU + (long long)(r0 + row) * n;
-      for (int b = 0; b < cnt; ++b) {
-        const int J = kLower ? done + b : nblk - 1 - (done + b);
-        const int c0 = J * kTriB + quarter * 16;
-        T a[16];
+    for (int b = 0; b < cnt; ++b) {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) a[c] = (c0 + c < n) ? rp[c0 + c] : (T)0;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) s += (V)a[c] * xs[b * kTriB + quarter * 16 + c];
-      }
+      for (int c = 0; c < 16; ++c) s += (V)a[c] * xs[b * kTriB + quarter * 16 + c];
+      if (done + b + 1 < deps) fetch(done + b + 1);
     }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
@@ -1162,10 +1284,9 @@ __global__ void __launch_bounds__(256) trsv_kernel(const T* __restrict__ LU, int
     done += cnt;
   }
   // x_I = dinv_I * acc (4 threads per row)
-  const T* D = dinv + (long long)I * kTriB * kTriB + (long long)row * kTriB + quarter * 16;
   V s = 0;
 #pragma unroll
-  for (int c = 0; c < 16; ++c) s += (V)D[c] * acc[quarter * 16 + c];
+  for (int c = 0; c < 16; ++c) s += (V)d[c] * acc[quarter * 16 + c];
   s += __shfl_xor_sync(0xffffffffu, s, 1);
   s += __shfl_xor_sync(0xffffffffu, s, 2);
   if (quarter == 0) xs[row] = s;
@@ -1208,24 +1329,34 @@ Error lu_factor_impl(T* A, int n, LuUpdate upd, LuWork* w, cudaStream_t st) {
     unsigned* bar = w->bar;
     int* err = w->err;
     int nn = n, kk0 = k0, kkb = kb, rr = rpc;
+    T* ut = (upd != kLuUpdateSimt) ? reinterpret_cast<T*>(w->ut) : nullptr;
+    const int rest = n - k0 - kb;
     // tournament pivoting in one cluster; else the column-by-column cluster
     // panel; else the cooperative kernel
-    if (!(w->tournament && launch_panel_tsp<T>(A, n, k0, kb, ipiv, err, w->local_pivot, st)) &&
-        !launch_panel_cluster<T>(A, n, k0, kb, P, ipiv, err, st)) {
-      void* args[] = {&A, &lda, &nn, &kk0, &kkb, &ipiv, &cv, &cr, &cd, &dd, &bar, &err, &rr};
-      UVLM_CUDA_TRY(cudaLaunchCooperativeKernel((void*)panel, dim3(P), dim3(kPanelRows), args, smem, st));
-      note_launch();
+    const bool tsp = w->tournament && launch_panel_tsp<T>(A, n, k0, kb, ipiv, w->moves, err, w->local_pivot, st);
+    if (tsp) {
+      const int ctas = ceil_div(rest, kApplyThreads), left = ceil_div(k0, kApplyThreads);
+      if (2 * ctas + left > 0) {
+        lu_apply_kernel<T><<<2 * ctas + left, kApplyThreads, 0, st>>>(A, n, n, k0, w->moves, ctas, ctas, ut, kLuNB);
+        UVLM_LAUNCH_CHECK();
+      }
+    } else {
+      if (!launch_panel_cluster<T>(A, n, k0, kb, P, ipiv, err, st)) {
+        void* args[] = {&A, &lda, &nn, &kk0, &kkb, &ipiv, &cv, &cr, &cd, &dd, &bar, &err, &rr};
+        UVLM_CUDA_TRY(cudaLaunchCooperativeKernel((void*)panel, dim3(P), dim3(kPanelRows), args, smem, st));
+        note_launch();
+      }
+      if (n - kb > 0) {
+        const int other = n - kb;
+        laswp_kernel<T><<<std::min(ceil_div(other, 256), 1024), 256, 0, st>>>(A, n, n, k0, kb, w->ipiv);
+        UVLM_LAUNCH_CHECK();
+      }
+      if (rest > 0) {
+        trsm_kernel<T><<<ceil_div(rest, kTrsmThreads), kTrsmThreads, 0, st>>>(A, n, n, k0, kb, ut, kLuNB);
+        UVLM_LAUNCH_CHECK();
+      }
     }
-    if (n - kb > 0) {
-      const int other = n - kb;
-      laswp_kernel<T><<<std::min(ceil_div(other, 256), 1024), 256, 0, st>>>(A, n, n, k0, kb, w->ipiv);
-      UVLM_LAUNCH_CHECK();
-    }
-    const int rest = n - k0 - kb;
     if (rest > 0) {
-      T* ut = (upd != kLuUpdateSimt) ? reinterpret_cast<T*>(w->ut) : nullptr;
-      trsm_kernel<T><<<ceil_div(rest, kTrsmThreads), kTrsmThreads, 0, st>>>(A, n, n, k0, kb, ut, kLuNB);
-      UVLM_LAUNCH_CHECK();
       T* C = A + (long long)(k0 + kb) * n + (k0 + kb);
       const T* L21 = A + (long long)(k0 + kb) * n + k0;
       const T* U12 = A + (long long)k0 * n + (k0 + kb);
@@ -1245,15 +1376,9 @@ Error lu_factor_impl(T* A, int n, LuUpdate upd, LuWork* w, cudaStream_t st) {
     }
   }
   const int nblk = ceil_div(n, kTriB);
-  diag_inverse_kernel<T><<<nblk, 2 * kTriB, 0, st>>>(A, n, reinterpret_cast<T*>(w->dinv_l),
-                                                     reinterpret_cast<T*>(w->dinv_u));
-  UVLM_LAUNCH_CHECK();
   // permutation vector stored after ipiv
-  const size_t perm_smem = 2 * sizeof(int) * (size_t)n;
-  if (perm_smem > 48 * 1024)
-    UVLM_CUDA_TRY(cudaFuncSetAttribute(ipiv_to_perm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)perm_smem));
-  ipiv_to_perm_kernel<<<1, 256, perm_smem, st>>>(w->ipiv, n, w->ipiv + n);
+  lu_finish_kernel<T><<<2 * nblk + ceil_div(n, kFinishThreads), kFinishThreads, 0, st>>>(
+      A, n, nblk, reinterpret_cast<T*>(w->dinv_l), reinterpret_cast<T*>(w->dinv_u), w->ipiv, w->ipiv + n);
   UVLM_LAUNCH_CHECK();
   return ok();
 }
@@ -1494,6 +1619,7 @@ size_t lu_work_place(LuWork* w, char* base) {
   put(&w->err, sizeof(int) * 4);
   put(&w->flags, sizeof(unsigned) * 2 * kLuMaxCtas);
   put(&w->ipiv, sizeof(int) * 2 * n);
+  put(&w->moves, sizeof(int) * 3 * kLuNB);
   put(&w->bar, sizeof(unsigned) * 2);
   put(&w->cand_val, sizeof(double) * 2 * kLuMaxCtas);
   put(&w->cand_row, sizeof(int) * 2 * kLuMaxCtas);

@@ -40,7 +40,8 @@ enum LuUpdate { kLuUpdateSimt = 0, kLuUpdateTF32 = 1, kLuUpdateBF16 = 2 };
 struct LuWork {
   int n = 0;
   void* own = nullptr;        // the block of all arrays (NULL when it is a Scratch's)
-  int* ipiv = nullptr;        // [n]
+  int* ipiv = nullptr;        // [2 n]: swap sequence, then the permutation
+  int* moves = nullptr;       // [3 kLuNB]: the row moves of the current panel
   int* err = nullptr;         // [1]: 0 ok, 1 barrier timeout, 2 zero pivot, 3 solve timeout
   unsigned* bar = nullptr;    // [2] grid barrier state
   double* cand_val = nullptr; // [2][kMaxCtas]
