@@ -390,31 +390,37 @@ constexpr size_t tsp_smem() {
   return sizeof(T) * ((size_t)kTspTop + (size_t)kTspRows * kTspLd + kLuNB) + sizeof(TspScratch);
 }
 
-// One row of the panel (64 values from column k0) from A into registers;
-// vector loads when the row start is 16-byte aligned.
+// Row `id` (relative to k0) of the panel, 64 values from column k0, into the
+// registers of every thread with `alive`: each warp reads its threads' rows
+// along the rows and passes them on through the threads' rows of Lrow (a
+// thread per row touched 32 lines per load).
 template <class T>
-__device__ __forceinline__ void tsp_load_row(const T* __restrict__ A, long long off, T (&v)[kLuNB]) {
-  const T* src = A + off;
-  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) {
-    constexpr int kPer = 16 / sizeof(T);
+__device__ __forceinline__ void tsp_load_rows(const T* A, int lda, int k0, int id, bool alive, T* Lrow,
+                                              T (&v)[kLuNB]) {
+  const int lane = threadIdx.x & 31;
+  T* base = Lrow + (threadIdx.x - lane) * kTspLd;
+  const unsigned live = __ballot_sync(0xffffffffu, alive);
+#pragma unroll 1
+  for (int i0 = 0; i0 < 32; i0 += 16) {
+    T t[16][2];  // all of a batch's loads before its first store
 #pragma unroll
-    for (int q = 0; q < kLuNB / kPer; ++q) {
-      if constexpr (sizeof(T) == 8) {
-        const double2 t = reinterpret_cast<const double2*>(src)[q];
-        v[2 * q] = t.x;
-        v[2 * q + 1] = t.y;
-      } else {
-        const float4 t = reinterpret_cast<const float4*>(src)[q];
-        v[4 * q] = t.x;
-        v[4 * q + 1] = t.y;
-        v[4 * q + 2] = t.z;
-        v[4 * q + 3] = t.w;
-      }
+    for (int i = 0; i < 16; ++i) {
+      const int r = __shfl_sync(0xffffffffu, id, i0 + i);
+      const T* src = A + (long long)(k0 + r) * lda + k0 + lane;
+      const bool in = live >> (i0 + i) & 1u;
+      t[i][0] = in ? src[0] : (T)0;
+      t[i][1] = in ? src[32] : (T)0;
     }
-  } else {
 #pragma unroll
-    for (int j = 0; j < kLuNB; ++j) v[j] = src[j];
+    for (int i = 0; i < 16; ++i) {
+      base[(i0 + i) * kTspLd + lane] = t[i][0];
+      base[(i0 + i) * kTspLd + 32 + lane] = t[i][1];
+    }
   }
+  __syncwarp();
+  const T* x = Lrow + threadIdx.x * kTspLd;
+#pragma unroll
+  for (int j = 0; j < kLuNB; ++j) v[j] = x[j];
 }
 
 // Argmax key of a row: (hi, lo) compared lexicographically; 0 for a finished row.
@@ -464,47 +470,6 @@ __device__ __forceinline__ void tsp_st8(T* p, const T (&o)[8]) {
   }
 }
 
-// uc[8 jc + t] = v[8 jc + t] (column c0 + 8 jc + t) for the 8-column chunks
-// that reach column c (= c0 + k) and lie left of column 64 (the shifted row's
-// entries past column 63 are dead); the chunk holding column c also writes
-// the columns left of it, which no reader uses.
-template <class T>
-__device__ __forceinline__ void tsp_publish(T* uc, int c0, int k, const T (&v)[kLuNB]) {
-#pragma unroll
-  for (int jc = 0; jc < 8; ++jc) {
-    if (8 * jc + 7 < k) continue;
-    if (c0 + 8 * jc < kLuNB) {
-      T* p = uc + 8 * jc;
-      if constexpr (sizeof(T) == 4) {
-        reinterpret_cast<float4*>(p)[0] = make_float4(v[8 * jc], v[8 * jc + 1], v[8 * jc + 2], v[8 * jc + 3]);
-        reinterpret_cast<float4*>(p)[1] = make_float4(v[8 * jc + 4], v[8 * jc + 5], v[8 * jc + 6], v[8 * jc + 7]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          reinterpret_cast<double2*>(p)[q] = make_double2(v[8 * jc + 2 * q], v[8 * jc + 2 * q + 1]);
-      }
-    }
-  }
-}
-
-// v[j] -= l uc[j] (column c0 + j of the pivot row) for the live columns
-// j >= lo, chunk by chunk (chunks past column 63 hold dead entries of the
-// shifted row and are skipped).
-template <class T>
-__device__ __forceinline__ void tsp_axpy(T (&v)[kLuNB], T l, const T* uc, int c0, int lo) {
-#pragma unroll
-  for (int jc = 0; jc < 8; ++jc) {
-    if (8 * jc + 7 < lo) continue;
-    if (c0 + 8 * jc < kLuNB) {
-      T t8[8];
-      tsp_ld8<T>(uc + 8 * jc, t8);
-#pragma unroll
-      for (int t = 0; t < 8; ++t)
-        if (8 * jc + t >= lo) v[8 * jc + t] -= l * t8[t];
-    }
-  }
-}
-
 // x / piv from r = 1 / piv: a product and one correction by its residual,
 // where r is far enough from the ends of the range for both; else a division.
 __device__ __forceinline__ float tsp_rcp(float x) { return __frcp_rn(x); }
@@ -518,25 +483,31 @@ __device__ __forceinline__ T tsp_quotient(T x, T piv, T r) {
   return fma(fma(-q, piv, x), r, q);
 }
 
-// The elimination of step c = c0 + k against the pivot row uc (reciprocal of
-// the pivot in r): l = v[k] / uc[k] into *lk, then v[j] -= l uc[j] for j > k.
-// A zero pivot leaves the row as it is and returns v[k] as its multiplier.
+// One step of an elimination on a row kept left-aligned in registers: v[j] is
+// its value in column c + j before the step and in column c + 1 + j after it,
+// v[j] = v[j + 1] - l u[j + 1] with u[j] the pivot row's value in column c + j
+// (64 values, 16-byte aligned, in shared memory; u8: its first 8).  The next
+// chunk of u is read while one is used; chunks past column 63 hold dead values
+// and are skipped.  One body for all steps: unrolled by 8 columns with a row
+// that stays in place, the elimination's code (16 kB for FP64) took 10 % more
+// time per panel.
 template <class T>
-__device__ __forceinline__ void tsp_eliminate(T (&v)[kLuNB], const T* uc, T r, int c0, int k, T* lk) {
-  const T piv = uc[k];
-  if (piv == (T)0) {
-    *lk = v[k];
-    return;
-  }
-  const T l = tsp_quotient<T>(v[k], piv, r);
-  *lk = l;
-  tsp_axpy<T>(v, l, uc, c0, k + 1);
-}
-
-template <class T>
-__device__ __forceinline__ void tsp_shift8(T (&v)[kLuNB]) {
+__device__ __forceinline__ void tsp_step(T (&v)[kLuNB], T l, const T* u, const T (&u8)[8], int c) {
+  T cur[8];
 #pragma unroll
-  for (int j = 0; j < kLuNB - 8; ++j) v[j] = v[j + 8];
+  for (int t = 0; t < 8; ++t) cur[t] = u8[t];
+#pragma unroll
+  for (int jc = 0; jc < 8; ++jc) {
+    T nxt[8];
+    if (jc < 7) tsp_ld8<T>(u + 8 * jc + 8, nxt);
+#pragma unroll
+    for (int t = jc ? 0 : 1; t < 8; ++t) v[8 * jc + t - 1] = v[8 * jc + t] - l * cur[t];
+    if (jc < 7) {
+      if (c + 8 * jc + 8 >= kLuNB) break;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) cur[t] = nxt[t];
+    }
+  }
 }
 
 // Partial-pivoting elimination of the R <= 256 rows held by threads
@@ -559,41 +530,47 @@ __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T*
   const int steps = min(kLuNB, R);
   T* lrow = Lrow + tid * kTspLd;
 #pragma unroll 1
-  for (int c0 = 0; c0 < steps; c0 += 8) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int c = c0 + k;
-      if (c < steps) {  // uniform
-        const int par = c & 1;
-        unsigned hi, lo;
-        tsp_key<T>(v[k], myid, alive, hi, lo);
-        const unsigned whi = __reduce_max_sync(0xffffffffu, hi);
-        const unsigned wlo = __reduce_max_sync(0xffffffffu, hi == whi ? lo : 0u);
-        if (lane == 0) {
-          sc.khi[par][warp] = whi;
-          sc.klo[par][warp] = wlo;
-        }
-        // every row's reciprocal while the keys settle: the pivot's is then
-        // ready with its row, and no division follows the second barrier
-        const T r = tsp_rcp(v[k]);
-        __syncthreads();
-        const unsigned ph = lane < kTspRows / 32 ? sc.khi[par][lane] : 0u;
-        const unsigned pl = lane < kTspRows / 32 ? sc.klo[par][lane] : 0u;
-        const unsigned bhi = __reduce_max_sync(0xffffffffu, ph);
-        const unsigned blo = __reduce_max_sync(0xffffffffu, ph == bhi ? pl : 0u);
-        T* u = Top + c * kLuNB + c0;  // column c0 + j at u[j]
-        if (alive && hi == bhi && lo == blo) {
-          out[c] = 0x1000 - (int)(blo & 0x1FFFu);
-          sc.pivrow[c] = tid;
-          Rcp[c] = r;
-          tsp_publish<T>(u, c0, k, v);
-          alive = false;
-        }
-        __syncthreads();
-        if (alive) tsp_eliminate<T>(v, u, Rcp[c], c0, k, lrow + c);
-      }
+  for (int c = 0; c < steps; ++c) {
+    const int par = c & 1;
+    unsigned hi, lo;
+    tsp_key<T>(v[0], myid, alive, hi, lo);
+    const unsigned whi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned wlo = __reduce_max_sync(0xffffffffu, hi == whi ? lo : 0u);
+    if (lane == 0) {
+      sc.khi[par][warp] = whi;
+      sc.klo[par][warp] = wlo;
     }
-    tsp_shift8<T>(v);
+    // every row's reciprocal while the keys settle: the pivot's is then ready
+    // with its row, and no division follows the second barrier
+    const T r = tsp_rcp(v[0]);
+    __syncthreads();
+    const unsigned ph = lane < kTspRows / 32 ? sc.khi[par][lane] : 0u;
+    const unsigned pl = lane < kTspRows / 32 ? sc.klo[par][lane] : 0u;
+    const unsigned bhi = __reduce_max_sync(0xffffffffu, ph);
+    const unsigned blo = __reduce_max_sync(0xffffffffu, ph == bhi ? pl : 0u);
+    T* u = Top + c * kLuNB;  // column c + j at u[j]
+    if (alive && hi == bhi && lo == blo) {
+      out[c] = 0x1000 - (int)(blo & 0x1FFFu);
+      sc.pivrow[c] = tid;
+      Rcp[c] = r;
+#pragma unroll
+      for (int jc = 0; jc < 8; ++jc)
+        if (c + 8 * jc < kLuNB) {
+          T o[8];
+#pragma unroll
+          for (int t = 0; t < 8; ++t) o[t] = v[8 * jc + t];
+          tsp_st8<T>(u + 8 * jc, o);
+        }
+      alive = false;
+    }
+    __syncthreads();
+    if (alive) {
+      T u8[8];
+      tsp_ld8<T>(u, u8);
+      const T l = u8[0] == (T)0 ? (T)0 : tsp_quotient<T>(v[0], u8[0], Rcp[c]);
+      lrow[c] = l;
+      tsp_step<T>(v, l, u, u8, c);
+    }
   }
   __syncthreads();  // Top, Lrow, out and pivrow complete for every thread
   return steps;
@@ -625,7 +602,7 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
   // the pivots are chosen among the panel's top 256 rows)
   {
     const bool alive = tid < nloc;
-    if (alive) tsp_load_row<T>(A, (long long)(k0 + rb + tid) * lda + k0, v);
+    tsp_load_rows<T>(A, lda, k0, rb + tid, alive, Lrow, v);
     const int k = tsp_factor<T>(v, alive, rb + tid, nloc, Top, Lrow, Rcp, sc, sc.list);
     if (tid == 0) sc.cnt[0] = k;
   }
@@ -650,7 +627,7 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
         R += c;
       }
       const bool alive = tid < R;
-      if (alive) tsp_load_row<T>(A, (long long)(k0 + myid) * lda + k0, v);
+      tsp_load_rows<T>(A, lda, k0, myid, alive, Lrow, v);
       const int k = tsp_factor<T>(v, alive, myid, R, Top, Lrow, Rcp, sc, sc.list);
       if (tid == 0) sc.cnt[0] = k;
     }
@@ -678,7 +655,7 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
     moves[tid] = sc.list[tid];
     moves[kLuNB + tid] = q >= kLuNB ? q : -1;
     moves[2 * kLuNB + tid] = sc.at[q];
-    if (Top[tid * kLuNB + tid] == (T)0) atomicExch(err + 1, 1);
+    if (Top[tid * kLuNB] == (T)0) atomicExch(err + 1, 1);
   }
 
   // ---- phase 4: the displaced rows of the panel, then its top block L11\U11
@@ -694,7 +671,7 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
   for (int u = 0; u < kPer; ++u) {
     const int q = tid + u * kTspRows, i = q >> 6, c = q & (kLuNB - 1), to = sc.seq[i];
     if (to >= kLuNB) A[(long long)(k0 + to) * lda + k0 + c] = d[u];
-    A[(long long)(k0 + i) * lda + k0 + c] = c < i ? Lrow[sc.pivrow[i] * kTspLd + c] : Top[q];
+    A[(long long)(k0 + i) * lda + k0 + c] = c < i ? Lrow[sc.pivrow[i] * kTspLd + c] : Top[q - i];
   }
 }
 
@@ -718,8 +695,9 @@ template <class T>
 __global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, int n, int k0,
                                                                  const int* __restrict__ moves, int row_ctas,
                                                                  int right_ctas, T* ut, int ldut) {
-  constexpr int kLd = kLuNB + 16 / sizeof(T);
-  __shared__ __align__(16) T M[kLuNB * kLd];  // row s: what step s eliminates with
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T* M = reinterpret_cast<T*>(smraw);  // [64][64]: row s, from its diagonal on, is what step s eliminates with
+  T* X = M + kLuNB * kLuNB;            // [64][65]: the rows' values in and out
   __shared__ T Rcp[kLuNB];
   __shared__ int mv[3 * kLuNB];
   const int tid = threadIdx.x;
@@ -727,44 +705,56 @@ __global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, 
   const bool right = !rows && (int)blockIdx.x < row_ctas + right_ctas;
   for (int q = tid; q < 3 * kLuNB; q += kApplyThreads) mv[q] = moves[q];
   if (rows || right) {
-    T t[16];
-    for (int i0 = 0; i0 < kLuNB; i0 += 16) {
+#pragma unroll 1
+    for (int i0 = 0; i0 < kLuNB; i0 += 32) {
+      T t[32];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) t[i] = A[(long long)(k0 + i0 + i) * lda + k0 + tid];
+      for (int i = 0; i < 32; ++i) t[i] = A[(long long)(k0 + i0 + i) * lda + k0 + tid];
 #pragma unroll
-      for (int i = 0; i < 16; ++i) M[rows ? (i0 + i) * kLd + tid : tid * kLd + i0 + i] = t[i];
+      for (int i = 0; i < 32; ++i) {
+        const int d = tid - (i0 + i);  // column - row
+        if (rows && d >= 0) M[(i0 + i) * kLuNB + d] = t[i];
+        if (!rows && d <= 0) M[tid * kLuNB - d] = t[i];
+      }
     }
   }
-  __syncthreads();
   T v[kLuNB];
   if (rows) {
-    Rcp[tid] = tsp_rcp(M[tid * kLd + tid]);
-    __syncthreads();
-    const int row = k0 + kLuNB + blockIdx.x * kApplyThreads + tid;
-    if (row >= n) return;
-    const long long off = (long long)row * lda + k0;
-    tsp_load_row<T>(A, off, v);
-    const bool aligned = (reinterpret_cast<uintptr_t>(A + off) & 15) == 0;
+    const int row0 = k0 + kLuNB + blockIdx.x * kApplyThreads, nr = min(kApplyThreads, n - row0);
 #pragma unroll 1
-    for (int c0 = 0; c0 < kLuNB; c0 += 8) {
-      T l[8];
+    for (int i0 = 0; i0 < kApplyThreads; i0 += 32) {
+      T t[32];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const T* u = M + (c0 + k) * kLd + c0;
-        const T piv = u[k];
-        l[k] = piv == (T)0 ? (T)0 : tsp_quotient<T>(v[k], piv, Rcp[c0 + k]);  // 0: the factor is singular
-        tsp_axpy<T>(v, l[k], u, c0, k + 1);
-      }
-      if (aligned) {
-        tsp_st8<T>(A + off + c0, l);
-      } else {
+      for (int i = 0; i < 32; ++i) t[i] = i0 + i < nr ? A[(long long)(row0 + i0 + i) * lda + k0 + tid] : (T)0;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) A[off + c0 + k] = l[k];
-      }
-      tsp_shift8<T>(v);
+      for (int i = 0; i < 32; ++i) X[(i0 + i) * kTspLd + tid] = t[i];
     }
+    __syncthreads();
+    Rcp[tid] = tsp_rcp(M[tid * kLuNB]);
+    __syncthreads();
+    T* x = X + tid * kTspLd;
+#pragma unroll
+    for (int j = 0; j < kLuNB; ++j) v[j] = x[j];
+    T u8[8];
+    tsp_ld8<T>(M, u8);
+#pragma unroll 1
+    for (int c = 0; c < kLuNB; ++c) {
+      const T* u = M + c * kLuNB;
+      const T l = u8[0] == (T)0 ? (T)0 : tsp_quotient<T>(v[0], u8[0], Rcp[c]);  // 0: the factor is singular
+      x[c] = l;
+      T first[8];
+      tsp_ld8<T>(c + 1 < kLuNB ? u + kLuNB : u, first);
+      tsp_step<T>(v, l, u, u8, c);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) u8[t] = first[t];
+    }
+    __syncthreads();
+#pragma unroll 16
+    for (int i = 0; i < kApplyThreads; ++i)
+      if (i < nr) A[(long long)(row0 + i) * lda + k0 + tid] = X[i * kTspLd + tid];
     return;
   }
+  __syncthreads();
   const int col = right ? k0 + kLuNB + ((int)blockIdx.x - row_ctas) * kApplyThreads + tid
                         : ((int)blockIdx.x - row_ctas - right_ctas) * kApplyThreads + tid;
   if (col >= (right ? n : k0)) return;
@@ -772,13 +762,13 @@ __global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, 
 #pragma unroll
   for (int i = 0; i < kLuNB; ++i) v[i] = a[(long long)mv[i] * lda];
 #pragma unroll 1
-  for (int i0 = 0; i0 < kLuNB; i0 += 16) {
-    T y[16];
+  for (int i0 = 0; i0 < kLuNB; i0 += 32) {
+    T y[32];
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
+    for (int i = 0; i < 32; ++i)
       y[i] = mv[kLuNB + i0 + i] >= 0 ? a[(long long)mv[2 * kLuNB + i0 + i] * lda] : (T)0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i)
+    for (int i = 0; i < 32; ++i)
       if (mv[kLuNB + i0 + i] >= 0) a[(long long)mv[kLuNB + i0 + i] * lda] = y[i];
   }
   if (!right) {
@@ -786,21 +776,41 @@ __global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, 
     for (int i = 0; i < kLuNB; ++i) a[(long long)i * lda] = v[i];
     return;
   }
+  T* o = ut ? ut + (long long)(col - k0 - kLuNB) * ldut : nullptr;
+  T u8[8];
+  tsp_ld8<T>(M, u8);
 #pragma unroll 1
-  for (int c0 = 0; c0 < kLuNB; c0 += 8) {
+  for (int c = 0; c < kLuNB; ++c) {
+    const T x = v[0];
+    const T* u = M + c * kLuNB;
+    a[(long long)c * lda] = x;
+    if (o) o[c] = x;
+    T first[8];
+    tsp_ld8<T>(c + 1 < kLuNB ? u + kLuNB : u, first);
+    tsp_step<T>(v, x, u, u8, c);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      tsp_axpy<T>(v, v[k], M + (c0 + k) * kLd + c0, c0, k + 1);
-      a[(long long)(c0 + k) * lda] = v[k];
-    }
-    if (ut) {
-      T o[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = v[k];
-      tsp_st8<T>(ut + (long long)(col - k0 - kLuNB) * ldut + c0, o);  // ldut = 64
-    }
-    tsp_shift8<T>(v);
+    for (int t = 0; t < 8; ++t) u8[t] = first[t];
   }
+}
+
+template <class T>
+Error launch_apply(T* A, int n, int k0, const int* moves, T* ut, cudaStream_t st) {
+  const int ctas = ceil_div(n - k0 - kLuNB, kApplyThreads), left = ceil_div(k0, kApplyThreads);
+  if (2 * ctas + left == 0) return ok();
+  constexpr size_t smem = sizeof(T) * (kLuNB * kLuNB + kApplyThreads * kTspLd);
+  auto kern = lu_apply_kernel<T>;
+  static PerDeviceOnce configured;
+  int dev = 0;
+  UVLM_CUDA_TRY(cudaGetDevice(&dev));
+  cudaError_t e = cudaSuccess;
+  if (!once_on_device(configured, dev, [&] {
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e == cudaSuccess;
+      }))
+    UVLM_CUDA_TRY(e);
+  kern<<<2 * ctas + left, kApplyThreads, smem, st>>>(A, n, n, k0, moves, ctas, ctas, ut, kLuNB);
+  UVLM_LAUNCH_CHECK();
+  return ok();
 }
 
 // Launches the tournament panel; false when it cannot run (a panel narrower
@@ -992,8 +1002,8 @@ __global__ void __launch_bounds__(256) gemm_update_kernel(T* C, int ldc, const T
 // differs from gemm_update_kernel's (which sums the products, then subtracts
 // once) at the level of FP64 rounding.  The 16-byte copies need 16-byte
 // aligned rows: even leading dimensions and aligned bases.
-constexpr int kG64BM = 128, kG64BN = 128, kG64BK = 16, kG64Stages = 3;
-constexpr int kG64ALd = kG64BK + 2;  // 144-byte rows of the A tile: the 4-row strides fall on other banks
+constexpr int kG64BM = 64, kG64BN = 64, kG64BK = 16, kG64Stages = 3, kG64Threads = 128;
+constexpr int kG64ALd = kG64BK + 2;  // 16-byte rows of the A tile that start four banks apart
 constexpr int kG64StageA = kG64BM * kG64ALd;
 constexpr int kG64StageB = kG64BK * kG64BN;
 constexpr size_t kG64Smem = sizeof(double) * kG64Stages * (kG64StageA + kG64StageB);
@@ -1003,12 +1013,13 @@ __device__ __forceinline__ void cp_async16_zfill(void* dst, const void* src, int
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(256, 1) gemm_update_f64_kernel(double* C, int ldc, const double* __restrict__ A,
-                                                                 int lda, const double* __restrict__ B, int ldb,
-                                                                 int m, int nc, int k) {
+__global__ void __launch_bounds__(kG64Threads, 4) gemm_update_f64_kernel(double* C, int ldc,
+                                                                          const double* __restrict__ A, int lda,
+                                                                          const double* __restrict__ B, int ldb,
+                                                                          int m, int nc, int k) {
   extern __shared__ __align__(16) double g64_smem[];
-  double* sA = g64_smem;                                // [stages][128][18]
-  double* sB = g64_smem + kG64Stages * kG64StageA;     // [stages][16][128]
+  double* sA = g64_smem;                                // [stages][64][18]
+  double* sB = g64_smem + kG64Stages * kG64StageA;     // [stages][16][64]
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int row0 = blockIdx.y * kG64BM, col0 = blockIdx.x * kG64BN;
   const int steps = (k + kG64BK - 1) / kG64BK;
@@ -1021,7 +1032,7 @@ __global__ void __launch_bounds__(256, 1) gemm_update_f64_kernel(double* C, int 
     double* b = sB + slot * kG64StageB;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int q = tid + 256 * i;
+      const int q = tid + kG64Threads * i;
       const int r = q >> 3, c2 = (q & 7) * 2;
       const int gr = row0 + r, gk = kk0 + c2;
       const int bytes = gr < m ? 8 * max(0, min(2, k - gk)) : 0;
@@ -1030,8 +1041,8 @@ __global__ void __launch_bounds__(256, 1) gemm_update_f64_kernel(double* C, int 
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int q = tid + 256 * i;
-      const int r = q >> 6, c2 = (q & 63) * 2;
+      const int q = tid + kG64Threads * i;
+      const int r = q >> 5, c2 = (q & 31) * 2;
       const int gk = kk0 + r, gc = col0 + c2;
       const int bytes = gk < k ? 8 * max(0, min(2, nc - gc)) : 0;
       const double* src = bytes ? B + (long long)gk * ldb + gc : B;
@@ -1039,81 +1050,76 @@ __global__ void __launch_bounds__(256, 1) gemm_update_f64_kernel(double* C, int 
     }
   };
 
-  // the accumulators start as this thread's 8 x 8 block of C (loaded while
-  // the operand pipeline fills) and the products are subtracted one by one,
-  // so the tile's C traffic overlaps its loads instead of following the MMAs
-  double acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = row0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = col0 + h * 64 + tx * 4;
-      const double* cp = C + (long long)r * ldc + c;
-      if (r < m && c + 3 < nc) {
-        const double2 v0 = *reinterpret_cast<const double2*>(cp);
-        const double2 v1 = *reinterpret_cast<const double2*>(cp + 2);
-        acc[i][h * 4 + 0] = v0.x;
-        acc[i][h * 4 + 1] = v0.y;
-        acc[i][h * 4 + 2] = v1.x;
-        acc[i][h * 4 + 3] = v1.y;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][h * 4 + j] = (r < m && c + j < nc) ? cp[j] : 0.0;
-      }
-    }
-  }
-
 #pragma unroll
   for (int s = 0; s < kG64Stages - 1; ++s) {
     if (s < steps) load_step(s, s);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
+
+  // the accumulators start as this thread's 8 x 4 block of C (loaded while
+  // the operand pipeline fills) and the products are subtracted one by one,
+  // so the tile's C traffic overlaps its loads instead of following the MMAs
+  const int c = col0 + tx * 4;
+  const bool whole = c + 3 < nc;
+  double acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = row0 + ty + 8 * i;
+    const double* cp = C + (long long)r * ldc + c;
+    if (r < m && whole) {
+      const double2 v0 = *reinterpret_cast<const double2*>(cp);
+      const double2 v1 = *reinterpret_cast<const double2*>(cp + 2);
+      acc[i][0] = v0.x;
+      acc[i][1] = v0.y;
+      acc[i][2] = v1.x;
+      acc[i][3] = v1.y;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = (r < m && c + j < nc) ? cp[j] : 0.0;
+    }
+  }
+
   for (int t = 0; t < steps; ++t) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kG64Stages - 2) : "memory");
     __syncthreads();  // step t landed for every thread; slot (t - 1) % stages is free
     if (t + kG64Stages - 1 < steps) load_step(t + kG64Stages - 1, (t + kG64Stages - 1) % kG64Stages);
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const double* a = sA + (t % kG64Stages) * kG64StageA;
-    const double* b = sB + (t % kG64Stages) * kG64StageB;
-#pragma unroll 8
-    for (int kk = 0; kk < kG64BK; ++kk) {
-      double av[8], bv[8];
+    const double* a = sA + (t % kG64Stages) * kG64StageA + ty * kG64ALd;
+    const double* b = sB + (t % kG64Stages) * kG64StageB + tx * 4;
+#pragma unroll 4
+    for (int kk = 0; kk < kG64BK; kk += 2) {
+      double2 av[8];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        av[i] = a[(ty * 4 + i) * kG64ALd + kk];
-        av[4 + i] = a[(64 + ty * 4 + i) * kG64ALd + kk];
+      for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const double2*>(a + 8 * i * kG64ALd + kk);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 b0 = *reinterpret_cast<const double2*>(b + (kk + h) * kG64BN);
+        const double2 b1 = *reinterpret_cast<const double2*>(b + (kk + h) * kG64BN + 2);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const double x = h ? -av[i].y : -av[i].x;
+          acc[i][0] = fma(x, b0.x, acc[i][0]);
+          acc[i][1] = fma(x, b0.y, acc[i][1]);
+          acc[i][2] = fma(x, b1.x, acc[i][2]);
+          acc[i][3] = fma(x, b1.y, acc[i][3]);
+        }
       }
-      const double2 b0 = *reinterpret_cast<const double2*>(b + kk * kG64BN + tx * 4);
-      const double2 b1 = *reinterpret_cast<const double2*>(b + kk * kG64BN + tx * 4 + 2);
-      const double2 b2 = *reinterpret_cast<const double2*>(b + kk * kG64BN + 64 + tx * 4);
-      const double2 b3 = *reinterpret_cast<const double2*>(b + kk * kG64BN + 64 + tx * 4 + 2);
-      bv[0] = b0.x, bv[1] = b0.y, bv[2] = b1.x, bv[3] = b1.y;
-      bv[4] = b2.x, bv[5] = b2.y, bv[6] = b3.x, bv[7] = b3.y;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(-av[i], bv[j], acc[i][j]);
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int r = row0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4);
+    const int r = row0 + ty + 8 * i;
     if (r >= m) continue;
+    double* cp = C + (long long)r * ldc + c;
+    if (whole) {
+      *reinterpret_cast<double2*>(cp) = make_double2(acc[i][0], acc[i][1]);
+      *reinterpret_cast<double2*>(cp + 2) = make_double2(acc[i][2], acc[i][3]);
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int c = col0 + h * 64 + tx * 4;
-      double* cp = C + (long long)r * ldc + c;
-      if (c + 3 < nc) {
-        *reinterpret_cast<double2*>(cp) = make_double2(acc[i][h * 4 + 0], acc[i][h * 4 + 1]);
-        *reinterpret_cast<double2*>(cp + 2) = make_double2(acc[i][h * 4 + 2], acc[i][h * 4 + 3]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (c + j < nc) cp[j] = acc[i][h * 4 + j];
-      }
+      for (int j = 0; j < 4; ++j)
+        if (c + j < nc) cp[j] = acc[i][j];
     }
   }
 }
@@ -1153,38 +1159,43 @@ __global__ void __launch_bounds__(kFinishThreads) lu_finish_kernel(const T* LU, 
     perm[k] = at;
     return;
   }
-  constexpr int kLd = kTriB + 16 / sizeof(T);
-  __shared__ __align__(16) T M[kTriB * kLd];  // M[s][r] = entry (r, s) of the block; rows reversed for U
+  // step s of the elimination: row s from its diagonal on, M[s][d] = entry
+  // (s + d, s) of L, or of U reversed in both directions (lower triangular too)
+  __shared__ __align__(16) T M[kTriB * kTriB];
   __shared__ T Rcp[kTriB];
   const int I = blockIdx.x >> 1, r0 = I * kTriB, nb = min(kTriB, n - r0);
   const bool upper = blockIdx.x & 1;
-  // U reversed in both directions is lower triangular too: step s of the
-  // elimination is row 63 - s of U
-#pragma unroll 16
-  for (int i = 0; i < kTriB; ++i) {
-    const T x = i < nb && tid < nb ? LU[(long long)(r0 + i) * n + r0 + tid] : (T)(i == tid);
-    M[upper ? (kTriB - 1 - tid) * kLd + kTriB - 1 - i : tid * kLd + i] = x;
+#pragma unroll 1
+  for (int i0 = 0; i0 < kTriB; i0 += 32) {
+    T t[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      t[i] = i0 + i < nb && tid < nb ? LU[(long long)(r0 + i0 + i) * n + r0 + tid] : (T)(i0 + i == tid);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      const int s = upper ? kTriB - 1 - tid : tid, d = upper ? tid - i0 - i : i0 + i - tid;
+      if (d >= 0) M[s * kTriB + d] = t[i];
+    }
   }
   __syncthreads();
-  if (upper) {
-    Rcp[tid] = tsp_rcp(M[tid * kLd + tid]);
-    __syncthreads();
-  }
+  Rcp[tid] = tsp_rcp(M[tid * kTriB]);
+  __syncthreads();
   T v[kTriB];
 #pragma unroll
   for (int i = 0; i < kTriB; ++i) v[i] = (T)(i == tid);
   T* out = (upper ? dinv_u : dinv_l) + (long long)I * kTriB * kTriB;
+  T u8[8];
+  tsp_ld8<T>(M, u8);
 #pragma unroll 1
-  for (int c0 = 0; c0 < kTriB; c0 += 8) {
+  for (int s = 0; s < kTriB; ++s) {
+    const T* u = M + s * kTriB;
+    const T x = upper ? tsp_quotient<T>(v[0], u8[0], Rcp[s]) : v[0];
+    out[upper ? (kTriB - 1 - s) * kTriB + kTriB - 1 - tid : s * kTriB + tid] = x;
+    T first[8];
+    tsp_ld8<T>(s + 1 < kTriB ? u + kTriB : u, first);
+    tsp_step<T>(v, x, u, u8, s);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int s = c0 + k;
-      const T* u = M + s * kLd + c0;
-      const T x = upper ? tsp_quotient<T>(v[k], u[k], Rcp[s]) : v[k];
-      tsp_axpy<T>(v, x, u, c0, k + 1);
-      out[upper ? (kTriB - 1 - s) * kTriB + kTriB - 1 - tid : s * kTriB + tid] = x;
-    }
-    tsp_shift8<T>(v);
+    for (int t = 0; t < 8; ++t) u8[t] = first[t];
   }
 }
 
@@ -1335,11 +1346,7 @@ Error lu_factor_impl(T* A, int n, LuUpdate upd, LuWork* w, cudaStream_t st) {
     // panel; else the cooperative kernel
     const bool tsp = w->tournament && launch_panel_tsp<T>(A, n, k0, kb, ipiv, w->moves, err, w->local_pivot, st);
     if (tsp) {
-      const int ctas = ceil_div(rest, kApplyThreads), left = ceil_div(k0, kApplyThreads);
-      if (2 * ctas + left > 0) {
-        lu_apply_kernel<T><<<2 * ctas + left, kApplyThreads, 0, st>>>(A, n, n, k0, w->moves, ctas, ctas, ut, kLuNB);
-        UVLM_LAUNCH_CHECK();
-      }
+      UVLM_TRY(launch_apply<T>(A, n, k0, w->moves, ut, st));
     } else {
       if (!launch_panel_cluster<T>(A, n, k0, kb, P, ipiv, err, st)) {
         void* args[] = {&A, &lda, &nn, &kk0, &kkb, &ipiv, &cv, &cr, &cd, &dd, &bar, &err, &rr};
@@ -1701,7 +1708,7 @@ Error gemm_update_f64(double* C, int ldc, const double* A, int lda, const double
                                     (int)kG64Smem) == cudaSuccess;
       })) {
     dim3 grid(ceil_div(nc, kG64BN), ceil_div(m, kG64BM));
-    gemm_update_f64_kernel<<<grid, 256, kG64Smem, st>>>(C, ldc, A, lda, B, ldb, m, nc, k);
+    gemm_update_f64_kernel<<<grid, kG64Threads, kG64Smem, st>>>(C, ldc, A, lda, B, ldb, m, nc, k);
     UVLM_LAUNCH_CHECK();
     return ok();
   }
