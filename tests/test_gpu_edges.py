@@ -146,3 +146,30 @@ def test_lu_of_a_general_matrix_at_its_block_edges(n):
     L = np.tril(LU, -1).astype(np.float64) + np.eye(n)
     err = np.max(np.abs(PA - L @ np.triu(LU).astype(np.float64))) / np.max(np.abs(A32))
     assert err <= n ** (5 / 3) * np.finfo(np.float32).eps
+
+
+@pytest.mark.parametrize("n,nt", [(0, 5), (1, 1), (31, 127), (32, 128), (33, 129), (1025, 300), (70, 160000)])
+@pytest.mark.parametrize("chordwise", [False, True])
+def test_ring_velocities_at_tile_and_split_edges(n, nt, chordwise):
+    """AoS rings against the reference's segment formula (src/vortex.cpp:24-38) in NumPy, a few targets on nodes.  The
+    points are in general position at distances above 1e-3 of the segments, where the formula loses at most 1e-9."""
+    from uvlm_b200 import rings as R
+
+    rng = np.random.default_rng(1000 * n + nt)
+    r = rng.uniform(-1, 1, (n, 1, 3)) + np.array([[0, 0, 0], [0.3, 0, 0], [0.3, 0.4, 0.1], [0, 0.4, 0]])
+    g = rng.standard_normal(n)
+    x = rng.uniform(-1.5, 1.5, (nt, 3))
+    if n:
+        x[:: max(nt // 7, 1)] = r[rng.integers(0, n, len(x[:: max(nt // 7, 1)])), 2]
+    got = R.InducedVelocity(x, r, g, chordwise=chordwise)
+    check = np.unique(np.linspace(0, nt - 1, 257).astype(int))
+    ref = np.zeros((len(check), 3))
+    for i, t in enumerate(x[check]):
+        for k in (0, 2) if chordwise else range(4):  # nodes[k + 1] -> nodes[k]
+            r1, r2 = t - r[:, (k + 1) % 4], t - r[:, k]
+            d = np.cross(r1, r2)
+            d2, n1, n2 = (d * d).sum(1), np.linalg.norm(r1, axis=1), np.linalg.norm(r2, axis=1)
+            ok = (d2 >= 1e-10) & (n1 >= 1e-10) & (n2 >= 1e-10)
+            f = ((r1 - r2)[ok] * (r1[ok] / n1[ok, None] - r2[ok] / n2[ok, None])).sum(1) / d2[ok]
+            ref[i] += ((g[ok] * f / (4 * np.pi))[:, None] * d[ok]).sum(0)
+    assert np.max(np.abs(got[check] - ref), initial=0) <= 1e-9 * max(np.max(np.abs(ref)), 1)

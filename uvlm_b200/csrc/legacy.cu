@@ -145,30 +145,6 @@ __global__ void __launch_bounds__(kSumThreads) sum4_kernel(const double* __restr
   }
 }
 
-// Velocity induced by AoS rings at device targets (FP64), SoA -> AoS.
-Error rings_velocity(const double* d_rings, const double* d_gamma, long long n_rings, int chordwise_only,
-                     const double* d_targets, long long nt, double* d_out, Scratch& S) {
-  double *pos, *gam, *vx, *vy, *vz;
-  UVLM_TRY(S.get(&vx, nt));
-  UVLM_TRY(S.get(&vy, nt));
-  UVLM_TRY(S.get(&vz, nt));
-  if (n_rings > 0) {
-    UVLM_TRY(S.get(&pos, 12 * n_rings));
-    UVLM_TRY(S.get(&gam, n_rings));
-    rings_to_sheets<<<gfor(n_rings), 256>>>(d_rings, d_gamma, n_rings, pos, gam);
-    UVLM_LAUNCH_CHECK();
-    SheetView v{pos, 2, 0, gam, 1, 0, (int)n_rings, 2, 1, chordwise_only ? 1 : 0};
-    UVLM_TRY(velocity_at(&v, 1, kNBodyFP64, d_targets, nt, vx, vy, vz, S));
-  } else {
-    UVLM_CUDA_TRY(cudaMemset(vx, 0, 8 * nt));
-    UVLM_CUDA_TRY(cudaMemset(vy, 0, 8 * nt));
-    UVLM_CUDA_TRY(cudaMemset(vz, 0, 8 * nt));
-  }
-  soa_to_aos<<<gfor(nt), 256>>>(vx, vy, vz, nt, d_out, nullptr, nullptr, 1.0);
-  UVLM_LAUNCH_CHECK();
-  return ok();
-}
-
 }  // namespace
 
 extern "C" {
@@ -231,14 +207,14 @@ int uvlm_rings_load_katz_plotkin(const double* rings, const double* gamma, const
       UVLM_TRY(S.up(&dw, wake_rings, (size_t)(12 * n_wake)));
       UVLM_TRY(S.up(&dwg, wake_gamma, (size_t)n_wake));
       UVLM_TRY(S.get(&uw, (size_t)(3 * n)));
-      UVLM_TRY(rings_velocity(dw, dwg, n_wake, 0, cen, n, uw, S));
+      UVLM_TRY(rings_at(dw, dwg, n_wake, false, cen, n, nullptr, nullptr, 1.0, uw, S));
     }
     if (n_bound > 0) {  // InducedVelocityByChordwiseBound (uvlm_vortex_ring.h:80-83)
       double *db, *dbg;
       UVLM_TRY(S.up(&db, bound_rings, (size_t)(12 * n_bound)));
       UVLM_TRY(S.up(&dbg, bound_gamma, (size_t)n_bound));
       UVLM_TRY(S.get(&ubc, (size_t)(3 * n)));
-      UVLM_TRY(rings_velocity(db, dbg, n_bound, 1, cen, n, ubc, S));
+      UVLM_TRY(rings_at(db, dbg, n_bound, true, cen, n, nullptr, nullptr, 1.0, ubc, S));
     }
     katz_plotkin_kernel<<<gfor(n), 256>>>(dr, dg, dgp, (int)rows, (int)cols, *kin,
                                           mk(freestream[0], freestream[1], freestream[2]), rho, t, dt, uw, ubc,
@@ -284,7 +260,7 @@ int uvlm_rings_load_joukowski(const double* rings, const double* rings0, const d
       UVLM_TRY(S.up(&dv, vortices, (size_t)(12 * n_vortices)));
       UVLM_TRY(S.up(&dvg, vortex_gamma, (size_t)n_vortices));
     }
-    UVLM_TRY(rings_velocity(dv, dvg, n_vortices, 0, mid, 4 * n, u, S));
+    UVLM_TRY(rings_at(dv, dvg, n_vortices, false, mid, 4 * n, nullptr, nullptr, 1.0, u, S));
     joukowski_kernel<<<gfor(n), 256>>>(dr, dr0, dg, dgp, (int)rows, (int)cols, *kin,
                                        mk(freestream[0], freestream[1], freestream[2]), rho, t, dt, u, terms);
     UVLM_LAUNCH_CHECK();

@@ -1041,4 +1041,118 @@ Error nbody_batch_eval(NBodyPrec prec, const NBodyBatchInput* d_in, int n, const
   }
 }
 
+// ------------------------------------------------------------- AoS rings
+// Rings that share nothing with each other (the legacy loop's containers): a
+// thread keeps one target and walks rings from shared memory, four node
+// quantities and four segments each.  Bound: the FP64 pipe, about 165
+// operations per ring and target against 13 16-byte shared-memory reads; the
+// ring range is split so that about eight CTAs per SM have work (pieces of at
+// least kRingTile rings) and the pieces' sums are added in order.  As 1 x 1
+// sheets through the strip walkers there was a far-field test for every four
+// nodes: a wake advection call with 1088 rings and 3840 targets took 267 us
+// (with records, layouts and partial sums in kernels of their own), now 162.
+namespace {
+constexpr int kRingThreads = 128, kRingTile = 32;
+
+struct alignas(16) RingRec {
+  double p[12];   // nodes
+  double r0[12];  // node k + 1 - node k
+  double g, pad;  // circulation of the walk n0 -> n1 -> n2 -> n3, over 4 pi
+};
+
+template <bool CHORDWISE>
+__global__ void __launch_bounds__(kRingThreads, 4)
+    rings_kernel(const double* __restrict__ rings, const double* __restrict__ gamma, long long n_rings,
+                 long long per_split, const double* __restrict__ targets, long long nt, double* __restrict__ partial) {
+  __shared__ RingRec sm[kRingTile];
+  const long long t = blockIdx.x * (long long)kRingThreads + threadIdx.x;
+  const double* x = targets + 3 * (t < nt ? t : nt - 1);
+  const double tx = x[0], ty = x[1], tz = x[2];
+  const long long begin = blockIdx.y * per_split, end = min(n_rings, begin + per_split);
+  double vx = 0, vy = 0, vz = 0;
+  for (long long k0 = begin; k0 < end; k0 += kRingTile) {
+    const int cnt = (int)min((long long)kRingTile, end - k0);
+    __syncthreads();
+    for (int q = threadIdx.x; q < cnt * 12; q += kRingThreads) {
+      const int r = q / 12, c = q - 12 * r;
+      const double* src = rings + 12 * (k0 + r);
+      const double a = src[c], b = src[c < 9 ? c + 3 : c - 9];
+      sm[r].p[c] = a;
+      sm[r].r0[c] = b - a;
+    }
+    if (threadIdx.x < cnt) sm[threadIdx.x].g = -gamma[k0 + threadIdx.x] * (1.0 / (4.0 * kPi));
+    __syncthreads();
+#pragma unroll 1
+    for (int r = 0; r < cnt; ++r) {
+      const RingRec& rec = sm[r];
+      NodeV<double> n[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        n[k].rx = tx - rec.p[3 * k];
+        n[k].ry = ty - rec.p[3 * k + 1];
+        n[k].rz = tz - rec.p[3 * k + 2];
+        const double q = n[k].rx * n[k].rx + n[k].ry * n[k].ry + n[k].rz * n[k].rz;
+        n[k].n = q >= kCutR2 ? q * nb_rsqrt(q) : 0.0;
+      }
+      const double g = rec.g;
+#pragma unroll
+      for (int k = 0; k < 4; k += CHORDWISE ? 2 : 1)
+        seg<double>(SegV<double>{rec.r0[3 * k], rec.r0[3 * k + 1], rec.r0[3 * k + 2]}, n[k], n[(k + 1) & 3], g, vx, vy,
+                    vz);
+    }
+  }
+  if (t < nt) {
+    double* o = partial + 3 * ((long long)blockIdx.y * nt + t);
+    o[0] = vx;
+    o[1] = vy;
+    o[2] = vz;
+  }
+}
+
+__global__ void rings_sum_kernel(const double* __restrict__ partial, int splits, long long n3,
+                                 const double* __restrict__ add3, const double* base, double scale, double* out) {
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n3;
+       q += (long long)gridDim.x * blockDim.x) {
+    double v = 0;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) v += partial[s * n3 + q];
+    if (add3) v += add3[q % 3];
+    out[q] = base ? base[q] + v * scale : v * scale;
+  }
+}
+
+// Splits of the ring range: about eight CTAs per SM, pieces of at least one tile.
+int rings_splits(long long n_rings, long long n_targets, int num_sms) {
+  const long long tiles = ceil_div(n_targets, kRingThreads);
+  const long long want = std::max<long long>((8LL * num_sms + tiles - 1) / tiles, 1);
+  return (int)std::min<long long>(want, std::max<long long>(ceil_div(n_rings, kRingTile), n_rings > 0));
+}
+
+}  // namespace
+
+long long rings_partial_size(long long n_rings, long long n_targets, int num_sms) {
+  return 3 * n_targets * rings_splits(n_rings, n_targets, num_sms);
+}
+
+Error rings_eval(const double* rings, const double* gamma, long long n_rings, bool chordwise_only,
+                 const double* targets, long long n_targets, const double* add3, const double* base, double scale,
+                 double* partial, double* out, int num_sms, cudaStream_t st) {
+  if (n_targets <= 0) return ok();
+  int splits = 0;
+  if (n_rings > 0) {
+    splits = rings_splits(n_rings, n_targets, num_sms);
+    const long long per = (n_rings + splits - 1) / splits;
+    const dim3 grid(ceil_div(n_targets, kRingThreads), splits);
+    if (chordwise_only)
+      rings_kernel<true><<<grid, kRingThreads, 0, st>>>(rings, gamma, n_rings, per, targets, n_targets, partial);
+    else
+      rings_kernel<false><<<grid, kRingThreads, 0, st>>>(rings, gamma, n_rings, per, targets, n_targets, partial);
+    UVLM_LAUNCH_CHECK();
+  }
+  const int blocks = (int)std::min<long long>((3 * n_targets + 255) / 256, 65535);
+  rings_sum_kernel<<<blocks, 256, 0, st>>>(partial, splits, 3 * n_targets, add3, base, scale, out);
+  UVLM_LAUNCH_CHECK();
+  return ok();
+}
+
 }  // namespace uvlm

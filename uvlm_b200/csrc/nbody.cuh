@@ -370,6 +370,16 @@ Error nbody_eval(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
                  long long n_targets, double* vx, double* vy, double* vz,
                  NBodyWork* work, int variant, int num_sms, cudaStream_t st);
 
+// out[t] = base[t] + (velocity induced at target t by AoS rings + add3) scale
+// in FP64 (base and add3 may be NULL; targets, base and out are AoS, and base
+// may be targets).  Ring k has nodes n0 .. n3 and circulation gamma[k], positive
+// along nodes[k + 1] -> nodes[k] (src/vortex.h:132-140).  chordwise_only: only the
+// segments n0-n1 and n2-n3.  partial: rings_partial_size() doubles.
+long long rings_partial_size(long long n_rings, long long n_targets, int num_sms);
+Error rings_eval(const double* rings, const double* gamma, long long n_rings, bool chordwise_only,
+                 const double* targets, long long n_targets, const double* add3, const double* base, double scale,
+                 double* partial, double* out, int num_sms, cudaStream_t st);
+
 // Algorithmic unique-segment count of a set of blocks (for the roofline).
 long long nbody_unique_segments(const SourceBlock* blocks, int n_blocks);
 

@@ -122,21 +122,11 @@ Error solve_rings(const double* bound_rings, const double* bound_rings0, int64_t
   UVLM_TRY(S.get(&tmp, (size_t)n));
   UVLM_TRY(launch_assemble_rings(dr, n, A, cen, nrm, 0));
   if (!drop_wake_term && n_wake > 0) {
-    double *dw, *dg, *pos, *gam, *vx, *vy, *vz;
+    double *dw, *dg;
     UVLM_TRY(S.up(&dw, wake_rings, (size_t)12 * n_wake));
     UVLM_TRY(S.up(&dg, wake_gamma, (size_t)n_wake));
-    UVLM_TRY(S.get(&pos, (size_t)12 * n_wake));
-    UVLM_TRY(S.get(&gam, (size_t)n_wake));
-    UVLM_TRY(S.get(&vx, n));
-    UVLM_TRY(S.get(&vy, n));
-    UVLM_TRY(S.get(&vz, n));
     UVLM_TRY(S.get(&wv, (size_t)3 * n));
-    rings_to_sheets<<<gfor(n_wake), 256>>>(dw, dg, n_wake, pos, gam);
-    UVLM_LAUNCH_CHECK();
-    SheetView v{pos, 2, 0, gam, 1, 0, (int)n_wake, 2, 1};
-    UVLM_TRY(velocity_at(&v, 1, kNBodyFP64, cen, n, vx, vy, vz, S));
-    soa_to_aos<<<gfor(n), 256>>>(vx, vy, vz, n, wv, nullptr, nullptr, 1.0);
-    UVLM_LAUNCH_CHECK();
+    UVLM_TRY(rings_at(dw, dg, n_wake, false, cen, n, nullptr, nullptr, 1.0, wv, S));
   }
   UVLM_TRY(launch_legacy_rhs(dk, dko, dr0, n, cen, nrm, freestream, t, wv, b, 0));
   LuWork lu;
@@ -321,28 +311,14 @@ int uvlm_rings_induced_velocity(const double* rings, const double* gammas, int64
   if (n_targets == 0) return UVLM_OK;
   Scratch S;
   auto run = [&]() -> Error {
-    double *dr, *dg, *pos, *gam, *dt, *vx, *vy, *vz, *dout;
+    double *dr = nullptr, *dg = nullptr, *dt, *dout;
     UVLM_TRY(S.up(&dt, targets, (size_t)(3 * n_targets)));
-    UVLM_TRY(S.get(&vx, n_targets));
-    UVLM_TRY(S.get(&vy, n_targets));
-    UVLM_TRY(S.get(&vz, n_targets));
     UVLM_TRY(S.get(&dout, 3 * n_targets));
     if (n_rings > 0) {
       UVLM_TRY(S.up(&dr, rings, (size_t)(12 * n_rings)));
       UVLM_TRY(S.up(&dg, gammas, (size_t)n_rings));
-      UVLM_TRY(S.get(&pos, 12 * n_rings));
-      UVLM_TRY(S.get(&gam, n_rings));
-      rings_to_sheets<<<gfor(n_rings), 256>>>(dr, dg, n_rings, pos, gam);
-      UVLM_LAUNCH_CHECK();
-      SheetView v{pos, 2, 0, gam, 1, 0, (int)n_rings, 2, 1, chordwise_only ? 1 : 0};
-      UVLM_TRY(velocity_at(&v, 1, kNBodyFP64, dt, n_targets, vx, vy, vz, S));
-    } else {
-      UVLM_CUDA_TRY(cudaMemset(vx, 0, 8 * n_targets));
-      UVLM_CUDA_TRY(cudaMemset(vy, 0, 8 * n_targets));
-      UVLM_CUDA_TRY(cudaMemset(vz, 0, 8 * n_targets));
     }
-    soa_to_aos<<<gfor(n_targets), 256>>>(vx, vy, vz, n_targets, dout, nullptr, nullptr, 1.0);
-    UVLM_LAUNCH_CHECK();
+    UVLM_TRY(rings_at(dr, dg, n_rings, chordwise_only != 0, dt, n_targets, nullptr, nullptr, 1.0, dout, S));
     UVLM_CUDA_TRY(cudaMemcpy(out, dout, sizeof(double) * 3 * n_targets, cudaMemcpyDeviceToHost));
     return ok();
   };
@@ -358,31 +334,16 @@ int uvlm_rings_advect(const double* vortex_rings, const double* vortex_gamma, in
   Scratch S;
   auto run = [&]() -> Error {
     const long long nt = 4 * n_wake;
-    double *dw, *vx, *vy, *vz, *dfs, *dr, *dg, *pos, *gam;
+    double *dw, *dfs, *dr = nullptr, *dg = nullptr, *dout;
     UVLM_TRY(S.up(&dw, wake_rings, (size_t)(12 * n_wake)));
     UVLM_TRY(S.up(&dfs, freestream, 3));
-    UVLM_TRY(S.get(&vx, nt));
-    UVLM_TRY(S.get(&vy, nt));
-    UVLM_TRY(S.get(&vz, nt));
+    UVLM_TRY(S.get(&dout, 3 * nt));
     if (n_vortex > 0) {
       UVLM_TRY(S.up(&dr, vortex_rings, (size_t)(12 * n_vortex)));
       UVLM_TRY(S.up(&dg, vortex_gamma, (size_t)n_vortex));
-      UVLM_TRY(S.get(&pos, 12 * n_vortex));
-      UVLM_TRY(S.get(&gam, n_vortex));
-      rings_to_sheets<<<gfor(n_vortex), 256>>>(dr, dg, n_vortex, pos, gam);
-      UVLM_LAUNCH_CHECK();
-      SheetView v{pos, 2, 0, gam, 1, 0, (int)n_vortex, 2, 1};
-      UVLM_TRY(velocity_at(&v, 1, kNBodyFP64, dw, nt, vx, vy, vz, S));
-    } else {
-      UVLM_CUDA_TRY(cudaMemset(vx, 0, 8 * nt));
-      UVLM_CUDA_TRY(cudaMemset(vy, 0, 8 * nt));
-      UVLM_CUDA_TRY(cudaMemset(vz, 0, 8 * nt));
     }
     // node += (induced + freestream) * dt  (src/shed.inl:8-19)
-    double* dout;
-    UVLM_TRY(S.get(&dout, 3 * nt));
-    soa_to_aos<<<gfor(nt), 256>>>(vx, vy, vz, nt, dout, dfs, dw, dt);
-    UVLM_LAUNCH_CHECK();
+    UVLM_TRY(rings_at(dr, dg, n_vortex, false, dw, nt, dfs, dw, dt, dout, S));
     UVLM_CUDA_TRY(cudaMemcpy(wake_rings, dout, sizeof(double) * 3 * nt, cudaMemcpyDeviceToHost));
     return ok();
   };
@@ -537,7 +498,7 @@ int uvlm_rings_lamb_vector(const double* panels, const double* panel_gamma, cons
     return report(fail(kErrInvalid, "invalid argument"));
   Scratch S;
   auto run = [&]() -> Error {
-    double *dp, *dg, *dv, *df, *dt, *vx, *vy, *vz, *du, *dout;
+    double *dp, *dg, *dv, *df, *dt, *du, *dout;
     UVLM_TRY(S.get(&dout, 3));
     const long long nt = 4 * n_panels;
     if (n_panels > 0) {
@@ -546,30 +507,16 @@ int uvlm_rings_lamb_vector(const double* panels, const double* panel_gamma, cons
       UVLM_TRY(S.up(&dv, node_velocities, (size_t)(12 * n_panels)));
       UVLM_TRY(S.up(&df, freestreams, (size_t)(3 * n_panels)));
       UVLM_TRY(S.get(&dt, 3 * nt));
-      UVLM_TRY(S.get(&vx, nt));
-      UVLM_TRY(S.get(&vy, nt));
-      UVLM_TRY(S.get(&vz, nt));
       UVLM_TRY(S.get(&du, 3 * nt));
       lamb_midpoints_kernel<<<gfor(nt), 256>>>(dp, n_panels, dt);
       UVLM_LAUNCH_CHECK();
+      // velocity of every vortex ring at the midpoints (InducedVelocityByVortices)
+      double *dr = nullptr, *drg = nullptr;
       if (n_vortices > 0) {
-        // velocity of every vortex ring at the midpoints (InducedVelocityByVortices)
-        double *dr, *drg, *pos, *gam;
         UVLM_TRY(S.up(&dr, vortices, (size_t)(12 * n_vortices)));
         UVLM_TRY(S.up(&drg, vortex_gamma, (size_t)n_vortices));
-        UVLM_TRY(S.get(&pos, 12 * n_vortices));
-        UVLM_TRY(S.get(&gam, n_vortices));
-        rings_to_sheets<<<gfor(n_vortices), 256>>>(dr, drg, n_vortices, pos, gam);
-        UVLM_LAUNCH_CHECK();
-        SheetView v{pos, 2, 0, gam, 1, 0, (int)n_vortices, 2, 1, 0};
-        UVLM_TRY(velocity_at(&v, 1, kNBodyFP64, dt, nt, vx, vy, vz, S));
-      } else {
-        UVLM_CUDA_TRY(cudaMemset(vx, 0, 8 * nt));
-        UVLM_CUDA_TRY(cudaMemset(vy, 0, 8 * nt));
-        UVLM_CUDA_TRY(cudaMemset(vz, 0, 8 * nt));
       }
-      soa_to_aos<<<gfor(nt), 256>>>(vx, vy, vz, nt, du, nullptr, nullptr, 1.0);
-      UVLM_LAUNCH_CHECK();
+      UVLM_TRY(rings_at(dr, drg, n_vortices, false, dt, nt, nullptr, nullptr, 1.0, du, S));
     } else {
       dp = dg = dv = df = du = nullptr;
     }

@@ -1,6 +1,6 @@
 // refapi_util.cuh -- helpers shared by the context-free C-ABI entry points
-// (refapi.cu, legacy.cu): AoS/SoA conversion, AoS
-// rings as 1 x 1 sheets, the FP64/FP32 N-body at arbitrary targets and a
+// (refapi.cu, legacy.cu): AoS/SoA conversion, the
+// FP64/FP32 N-body of sheets and of AoS rings at arbitrary targets and a
 // fixed-order block sum.
 #pragma once
 
@@ -42,19 +42,6 @@ __global__ void soa_to_aos(const double* x, const double* y, const double* z, lo
       double u = v[d] + (add3 ? add3[d] : 0.0);
       a[3 * k + d] = base ? base[3 * k + d] + u * scale : u;
     }
-  }
-}
-// AoS ring k (nodes n0..n3) -> 1 x 1 sheet k with p(0,0)=n0, p(0,1)=n1,
-// p(1,1)=n2, p(1,0)=n3 and circulation -g: the sheet walks n0->n1->n2->n3,
-// the AoS ring nodes[k+1]->nodes[k] (src/vortex.h:132-140).
-__global__ void rings_to_sheets(const double* rings, const double* g, long long n, double* pos, double* gam) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const double* r = rings + 12 * k;
-    double* p = pos + 12 * k;
-    const int map[4] = {0, 1, 3, 2};  // sheet order (0,0),(0,1),(1,0),(1,1)
-    for (int q = 0; q < 4; ++q)
-      for (int d = 0; d < 3; ++d) p[3 * q + d] = r[3 * map[q] + d];
-    gam[k] = -g[k];
   }
 }
 constexpr int kSumThreads = 256;
@@ -105,6 +92,18 @@ Error velocity_at(const SheetView* views, int nv, NBodyPrec prec, const double* 
   aos_to_soa<<<gfor(nt), 256>>>(d_targets_aos, nt, tx, ty, tz);
   UVLM_LAUNCH_CHECK();
   return velocity_soa(views, nv, prec, tx, ty, tz, nt, vx, vy, vz, S);
+}
+
+// out = base + (velocity induced by AoS rings at AoS targets + add3) scale, all
+// on the device, FP64 (base and add3 may be NULL).
+Error rings_at(const double* d_rings, const double* d_gamma, long long n_rings, bool chordwise_only,
+               const double* d_targets, long long nt, const double* add3, const double* base, double scale,
+               double* d_out, Scratch& S) {
+  double* partial = nullptr;
+  const int n_sms = sms();
+  UVLM_TRY(S.get(&partial, rings_partial_size(n_rings, nt, n_sms)));
+  return rings_eval(d_rings, d_gamma, n_rings, chordwise_only, d_targets, nt, add3, base, scale, partial, d_out, n_sms,
+                    0);
 }
 
 }  // namespace
