@@ -343,31 +343,31 @@ bool launch_panel_cluster(T* A, int n, int k0, int kb, int P, int* ipiv, int* er
 // (gathered from A, which the tournament does not modify) and keeping the 64
 // rows picked, in a 4-ary tree over the cluster (the partners' lists are read
 // through distributed shared memory).  The root's factorisation is the
-// panel's top block L11\U11 in the root's pivot order.  The chosen rows are
-// then brought to the top (LAPACK-style swap sequence in ipiv, replayed by
-// every CTA for its own rows), and every other row r gets L21(r) from
-// l U11 = a(r) (forward substitution on its original row).  The remaining
-// columns are swapped by laswp and updated as before.  The pivots differ from
+// panel's top block L11\U11 in the root's pivot order, and the root writes it,
+// the rows it displaces and the swap sequence (LAPACK-style, in ipiv).  L21, the
+// other columns' row moves and U12 follow in lu_apply_kernel.  The pivots differ from
 // column-by-column partial pivoting only where the candidates' magnitudes are
 // close; the factorisation is of the same quality for the influence matrices
 // of the path (and it backs a GMRES solve with FP64 residuals in the mixed
 // form).
 //
-// Each factorisation keeps one row per thread in registers.  Column loop:
-// blocks of 8 columns unrolled (compile-time register indices), a run-time
-// loop over the blocks, and the row shifted left by 8 columns after each
-// block (v[k] is column c0 + k), which keeps the code small and the row in
-// registers.  Per column: a block argmax of (|a|, row id) packed into one
-// 64-bit key (two warp max-reductions per level; ties go to the smaller row
-// id, NaN counts as largest, a finished row has key 0 and never wins; for
-// FP64 the 13 lowest mantissa bits make way for the id, so values within
-// 2^-39 of each other count as tied); the pivot row's owner publishes its
-// U part in shared memory; every other live row stores its multiplier in its
+// Each factorisation keeps one row per thread in registers, left-aligned (v[j]
+// is column c + j at step c), so that one short body serves all steps.  Per
+// column: a block argmax of (|a|, row id) packed into one 64-bit key (two warp
+// max-reductions per level; ties go to the smaller row id, NaN counts as
+// largest, a finished row has key 0 and never wins; for FP64 the 13 lowest
+// mantissa bits make way for the id, so values within 2^-39 of each other count
+// as tied); the pivot row's owner publishes its U part and its reciprocal in
+// shared memory; every other live row stores its multiplier in its
 // shared-memory row of L (Lrow) and eliminates against the pivot row.  Two
 // block barriers per column: a published row from one lane (one warp) costs
-// less than every warp's candidate row before a single barrier.  Two lanes per
-// row (16 warps, half rows, each lane reading half of the pivot row) measured
-// 5 % (FP32) and 12 % (FP64) slower per panel than one lane per row.
+// less than every warp's candidate row before a single barrier.
+// Bound: the serial chain of a step, about 900 cycles of an FP64 step of 256
+// rows (330 the elimination, limited by the shared-memory reads of the pivot
+// row, 150 its publication, 100 quotients and reciprocals, the rest key
+// reductions and barriers).  Panel of 2304 rows, FP64: 186 -> 115 us with L21
+// out of the cluster, rows read along the warps, one body for all steps and
+// the reciprocals formed before the pivot is known.
 constexpr int kTspRows = 256;  // rows per CTA = threads per CTA
 constexpr int kTspMaxCtas = 16;
 constexpr int kTspMaxRows = kTspRows * kTspMaxCtas;
@@ -470,17 +470,24 @@ __device__ __forceinline__ void tsp_st8(T* p, const T (&o)[8]) {
   }
 }
 
-// x / piv from r = 1 / piv: a product and one correction by its residual,
-// where r is far enough from the ends of the range for both; else a division.
-__device__ __forceinline__ float tsp_rcp(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double tsp_rcp(double x) { return __drcp_rn(x); }
+// 1 / x, or 0 where it is too near the ends of the range for tsp_quotient.
+__device__ __forceinline__ float tsp_rcp(float x) {
+  const float r = __frcp_rn(x);
+  return fabsf(r) < 0x1p+100f && fabsf(r) > 0x1p-100f ? r : 0.f;
+}
+__device__ __forceinline__ double tsp_rcp(double x) {
+  const double r = __drcp_rn(x);
+  return fabs(r) < 0x1p+900 && fabs(r) > 0x1p-900 ? r : 0.0;
+}
 
+// x / piv from r = tsp_rcp(piv): a product and one correction by its residual,
+// or a division where r is 0; 0 for a zero pivot.
 template <class T>
 __device__ __forceinline__ T tsp_quotient(T x, T piv, T r) {
-  constexpr T big = sizeof(T) == 8 ? (T)0x1p+900 : (T)0x1p+100f;
-  if (!(fabs(r) < big && fabs(r) > (T)1 / big)) return x / piv;
   const T q = x * r;
-  return fma(fma(-q, piv, x), r, q);
+  T l = fma(fma(-q, piv, x), r, q);
+  if (r == (T)0) l = piv == (T)0 ? (T)0 : x / piv;
+  return l;
 }
 
 // One step of an elimination on a row kept left-aligned in registers: v[j] is
@@ -513,16 +520,13 @@ __device__ __forceinline__ void tsp_step(T (&v)[kLuNB], T l, const T* u, const T
 // Partial-pivoting elimination of the R <= 256 rows held by threads
 // 0 .. R-1 (v, original id myid).  Picks min(64, R) pivot rows: their ids go
 // to out[] in pivot order, the owning threads to sc.pivrow[]; step c leaves
-// the pivot row's U part in Top[c] (columns c .. 63) and every other row's
+// the pivot row's U part in Top[c] (column c + j at [j]) and every other row's
 // multiplier in Lrow[thread][c].  Per column: the per-warp keys (of the
 // step's parity: a slow reader of step c may still read them while a fast
 // warp writes those of step c + 1) and a barrier; the block key; the owner
-// publishes its row and a barrier; the others eliminate.  (Deferring all but
-// the next column's update past the next argmax barrier measured 7-11 %
-// slower per step; blocking by 8 columns with the update right of the block
-// applied once per block measured the same as this.)  The operations on each row are those of a
-// column-by-column factorisation, in the same order.  Every thread of the
-// CTA calls it.
+// publishes its row and a barrier; the others eliminate.  The operations on
+// each row are those of a column-by-column factorisation, in the same order.
+// Every thread of the CTA calls it.
 template <class T>
 __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T* Lrow, T* Rcp, TspScratch& sc,
                           int* out) {
@@ -554,20 +558,20 @@ __device__ int tsp_factor(T (&v)[kLuNB], bool alive, int myid, int R, T* Top, T*
       sc.pivrow[c] = tid;
       Rcp[c] = r;
 #pragma unroll
-      for (int jc = 0; jc < 8; ++jc)
-        if (c + 8 * jc < kLuNB) {
-          T o[8];
+      for (int jc = 0; jc < 8; ++jc) {
+        if (jc == 4 && c >= kLuNB / 2) break;  // dead values from here on
+        T o[8];
 #pragma unroll
-          for (int t = 0; t < 8; ++t) o[t] = v[8 * jc + t];
-          tsp_st8<T>(u + 8 * jc, o);
-        }
+        for (int t = 0; t < 8; ++t) o[t] = v[8 * jc + t];
+        tsp_st8<T>(u + 8 * jc, o);
+      }
       alive = false;
     }
     __syncthreads();
     if (alive) {
       T u8[8];
       tsp_ld8<T>(u, u8);
-      const T l = u8[0] == (T)0 ? (T)0 : tsp_quotient<T>(v[0], u8[0], Rcp[c]);
+      const T l = tsp_quotient<T>(v[0], u8[0], Rcp[c]);
       lrow[c] = l;
       tsp_step<T>(v, l, u, u8, c);
     }
@@ -684,11 +688,11 @@ __global__ void __launch_bounds__(kTspRows, 1) lu_panel_tsp_kernel(T* A, int lda
 // moves: for i < 64 the old row of new row i, a row below the top block that a
 // top row moves to (or -1), and that top row, relative to k0.  The row and
 // column solves are the same elimination of 64 values in registers against
-// the rows of U11 or the columns of L11 in shared memory, eight columns
-// unrolled in a run-time loop.  In the panel's cluster the rows' part kept
-// only its <= 16 SMs busy, 256 rows each (20 us a panel), and a fully
-// unrolled triangular solve per column (a kernel of its own) spent 20 us a
-// panel on fetching its instructions: APPLY_FIGURES.
+// the rows of U11 or the columns of L11 in shared memory (tsp_step).  Bound:
+// the serial chain of 64 steps (about 270 cycles each for a lone warp) and three
+// round trips to memory; 22 us per panel at n = 2304 in FP64, where the swaps
+// (8 us), a triangular solve of its own (20 us) and the rows' part inside the
+// panel's cluster (20 us on its <= 16 SMs) took 48.
 constexpr int kApplyThreads = 64;
 
 template <class T>
@@ -740,7 +744,7 @@ __global__ void __launch_bounds__(kApplyThreads) lu_apply_kernel(T* A, int lda, 
 #pragma unroll 1
     for (int c = 0; c < kLuNB; ++c) {
       const T* u = M + c * kLuNB;
-      const T l = u8[0] == (T)0 ? (T)0 : tsp_quotient<T>(v[0], u8[0], Rcp[c]);  // 0: the factor is singular
+      const T l = tsp_quotient<T>(v[0], u8[0], Rcp[c]);  // 0: the factor is singular
       x[c] = l;
       T first[8];
       tsp_ld8<T>(c + 1 < kLuNB ? u + kLuNB : u, first);
@@ -860,7 +864,8 @@ bool launch_panel_tsp(T* A, int n, int k0, int kb, int* ipiv, int* moves, int* e
   return true;
 }
 
-// Row swaps of one panel applied to the columns outside the panel.
+// Row swaps of one panel applied to the columns outside the panel (after a
+// panel that is not a tournament's).
 template <class T>
 __global__ void laswp_kernel(T* A, int lda, int n, int k0, int kb, const int* __restrict__ ipiv) {
   const int other = n - kb;
@@ -879,7 +884,8 @@ __global__ void laswp_kernel(T* A, int lda, int n, int k0, int kb, const int* __
   }
 }
 
-// U12 = L11^-1 A12 (unit lower L11), one thread per column.  Optionally also
+// U12 = L11^-1 A12 (unit lower L11) after a panel that is not a tournament's
+// (lu_apply_kernel does it otherwise), one thread per column.  Optionally also
 // writes U12 transposed into ut ([col - (k0+kb)][k], leading dim ldut).
 // Columns per CTA of the TRSM (one column per thread; L11 staged once per
 // CTA).  32-column CTAs, which spread a panel's columns over more SMs, took
@@ -995,12 +1001,13 @@ __global__ void __launch_bounds__(256) gemm_update_kernel(T* C, int ldc, const T
 }
 
 // FP64 trailing update C -= A B of the plain form's LU (K = the panel width):
-// 128 x 128 output tiles, 256 threads each holding an 8 x 8 register block
-// (rows ty*4 + i and 64 + ty*4 + i, columns tx*4 + j and 64 + tx*4 + j), K
-// in steps of 16 through a three-stage cp.async pipeline.  Each entry of C
+// 64 x 64 output tiles, 128 threads each holding an 8 x 4 register block (rows
+// ty + 8 i, columns tx*4 + j), K in steps of 16 through a three-stage cp.async pipeline.  Each entry of C
 // has its products subtracted one by one in k order (FMA), so the rounding
 // differs from gemm_update_kernel's (which sums the products, then subtracts
-// once) at the level of FP64 rounding.  The 16-byte copies need 16-byte
+// once) at the level of FP64 rounding.  Bound: the FP64 pipe (four CTAs per SM).
+// Trailing blocks of 2240 / 1088 / 128 rows: 60 / 24 / 20 us with 128 x 128
+// tiles (a nearly empty last wave, or one tile's own time), 51 / 17 / 10 now.  The 16-byte copies need 16-byte
 // aligned rows: even leading dimensions and aligned bases.
 constexpr int kG64BM = 64, kG64BN = 64, kG64BK = 16, kG64Stages = 3, kG64Threads = 128;
 constexpr int kG64ALd = kG64BK + 2;  // 16-byte rows of the A tile that start four banks apart
@@ -1133,9 +1140,9 @@ __global__ void __launch_bounds__(kG64Threads, 4) gemm_update_f64_kernel(double*
 // against the block in shared memory; blocks past the matrix are padded with
 // the identity).  perm[k] is found by walking the swaps back from position k:
 // swap j <= k moves row p_j >= j to position j, so only p_j == position
-// matters; four compares per 16-byte read, independent for every k (one
-// chain of n dependent swaps took 81 us at n = 2304, the inverses from global
-// memory 108: FINISH_FIGURES).
+// matters; four compares per 16-byte read, independent for every k.  n = 2304
+// in FP64: 43 us; one chain of n dependent swaps took 81 us, inverses formed
+// in global memory 108.
 constexpr int kFinishThreads = kTriB;
 
 template <class T>

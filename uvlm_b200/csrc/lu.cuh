@@ -13,11 +13,12 @@
 //   1. lu_panel   -- one thread-block cluster (<= 16 CTAs of 256 rows): the
 //                    pivot rows chosen by a tournament (each CTA factors its
 //                    rows, candidate sets merged in a 4-ary tree through
-//                    distributed shared memory), then L21 by substitution;
+//                    distributed shared memory);
 //                    else a cluster with one barrier per column; else one
 //                    cooperative kernel with a bounded grid barrier per column;
-//   2. laswp      -- the panel's row swaps applied to the other columns;
-//   3. trsm       -- U12 = L11^-1 A12;
+//   2. lu_apply   -- after a tournament, L21 of the rows below, the row moves of
+//                    the other columns and U12 = L11^-1 A12, in one launch; else
+//   3. laswp, trsm -- the row swaps and U12;
 //   4. update     -- A22 -= L21 U12: FP64 SIMT GEMM (plain form) or a tcgen05
 //                    tensor-core GEMM in TF32 / BF16 with FP32 accumulation
 //                    (mixed form, lu_tc.cu).
