@@ -74,3 +74,35 @@ def test_strengths_scale_exactly(precision):
     # circulations so small that their squares leave the FP32 range
     small = U.InducedVelocity(t, pos, gamma * 2.0 ** -60, precision) * 2.0 ** 60
     np.testing.assert_allclose(small, v, rtol=0, atol=(1e-12 if precision == "fp64" else 2e-5) * np.max(np.abs(v)))
+
+
+@pytest.mark.parametrize("n", [2048, 8191, 8193, 20011, 33000])
+@pytest.mark.parametrize("kind", ["box", "line", "one", "odd"])
+def test_point_sets_that_are_ordered_first(n, kind):
+    """Point sets large enough to be put in the order of a space-filling curve against the same points in pieces that are
+    evaluated as given: spread in a box, along a line, all in one place, with a few that are not finite.  Tolerances of
+    the other N-body tests between two evaluations (FP64 1e-12 of max |v|; FP32 4e-5 of the local velocity + 2e-6 of
+    max |v|, twice a single one's)."""
+    import uvlm_b200 as U
+
+    pos, gamma = _sheet(1, 70, 64, seed=n, wobble=0.0)  # 9104 segments
+    rng = np.random.default_rng(n)
+    x = rng.uniform([-1, -1, -1], [12, 5, 1], (n, 3))
+    if kind == "line":
+        x = np.outer(rng.uniform(0.1, 30, n), [1.0, 0.0, 0.0]) + [0.0, 0.333, 0.77]
+    if kind == "one":
+        x[:] = x[0]
+    odd = np.zeros(n, bool)
+    if kind == "odd":
+        odd[rng.integers(0, n, 9)] = True
+        x[odd] = rng.choice([np.nan, np.inf, -np.inf, 1e300], (odd.sum(), 3))
+    for precision, piece in (("fp64", 1000), ("mixed", 1000)):
+        got = U.InducedVelocity(x, pos, gamma, precision=precision)
+        ref = np.concatenate([U.InducedVelocity(x[i:i + piece], pos, gamma, precision=precision)
+                              for i in range(0, n, piece)])
+        got, ref = got[~odd], ref[~odd]
+        assert np.all(np.isfinite(got))
+        scale, mag = np.max(np.abs(ref)), np.linalg.norm(ref, axis=1)
+        bound = 1e-12 * scale if precision == "fp64" else 4e-5 * mag + 2e-6 * scale
+        assert np.all(np.abs(got - ref).max(axis=1) <= bound)
+    np.testing.assert_array_equal(U.InducedVelocity(x, pos, gamma), U.InducedVelocity(x, pos, gamma))

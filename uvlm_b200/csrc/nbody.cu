@@ -1,6 +1,9 @@
 // nbody.cu -- strip-tiled Biot-Savart N-body (FP32 hi/lo and FP64 forms).
 #include <algorithm>
+#include <climits>
 #include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "device_once.h"
 #include "nbody.cuh"
@@ -365,20 +368,24 @@ __device__ __forceinline__ void full_column2(const RecF* col, const Tgt<float> (
   }
 }
 
+// A strip of n_cols node columns, rows padded with zero records.  (Padding the
+// columns of narrow strips as well, or walking them unpacked, took up to twice
+// the time: FP32, 60,000 points, 20 x 20 rings, 122 -> 96 us.)
 template <int H>
-__device__ __forceinline__ void walk_full_strip2(const RecF* sm, bool last_h, const Tgt<float> (&tg)[2],
-                                                 float (&acc)[2][3]) {
+__device__ __forceinline__ void walk_cols2(const RecF* sm, int n_cols, bool last_h, const Tgt<float> (&tg)[2],
+                                           float (&acc)[2][3]) {
   Node2 prev[H];
   SegV<float> ps0[H];
   float pgS[H];
   float2 a2[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  // a strip has at least two node columns
   full_column2<H, true, true>(sm, tg, prev, ps0, pgS, a2);
 #pragma unroll 2
-  for (int j = 1; j < kStripCols; ++j) full_column2<H, false, true>(sm + j, tg, prev, ps0, pgS, a2);
+  for (int j = 1; j < n_cols - 1; ++j) full_column2<H, false, true>(sm + j, tg, prev, ps0, pgS, a2);
   if (last_h)
-    full_column2<H, false, true>(sm + kStripCols, tg, prev, ps0, pgS, a2);
+    full_column2<H, false, true>(sm + n_cols - 1, tg, prev, ps0, pgS, a2);
   else
-    full_column2<H, false, false>(sm + kStripCols, tg, prev, ps0, pgS, a2);
+    full_column2<H, false, false>(sm + n_cols - 1, tg, prev, ps0, pgS, a2);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     acc[0][c] += a2[c].x;
@@ -467,7 +474,7 @@ namespace {
 
 // Strips [s_begin, s_end) of B for the thread's targets, double-buffered
 // through shared memory; FP32 partial sums per strip, FP64 across strips.
-// PK: 0 generic walkers, 1 packed FP32x2 walker on full strips.
+// PK: 0 generic walkers, 1 packed FP32x2 walker.
 template <class T, class Rec, int H, int TPT, int BLOCK, bool PAD, int PK>
 __device__ __forceinline__ void eval_strips(const Blocks& B, long long s_begin, long long s_end,
                                             const Rec* __restrict__ rec, Rec* buf0, Rec* buf1,
@@ -499,7 +506,7 @@ __device__ __forceinline__ void eval_strips(const Blocks& B, long long s_begin, 
 #pragma unroll
     for (int q = 0; q < TPT; ++q) acc[q][0] = acc[q][1] = acc[q][2] = (T)0;
     if constexpr (PAD && PK == 1 && sizeof(T) == 4 && TPT == 2) {
-      walk_full_strip2<H>(cur, si.last_h, tg, acc);
+      walk_cols2<H>(cur, si.n_cols, si.last_h, tg, acc);
     } else if constexpr (PAD)
       walk_full_strip<T, Rec, H, TPT>(cur, si.last_h, tg, acc);
     else
@@ -663,18 +670,19 @@ constexpr int kBatchBlock = 128;
 constexpr int kBatchTptF = 2, kBatchTptD = 1, kBatchHD = 2, kBatchMinB = 3;
 
 __global__ void reduce_partials_kernel(const double* __restrict__ partial, int splits, long long n, double* vx,
-                                       double* vy, double* vz) {
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    double x = 0, y = 0, z = 0;
-    for (int s = 0; s < splits; ++s) {
-      const double* p = partial + (long long)s * 3 * n;
-      x += p[t];
-      y += p[n + t];
-      z += p[2 * n + t];
-    }
-    vx[t] = x;
-    vy[t] = y;
-    vz[t] = z;
+                                       double* vy, double* vz, double* aos, const int* __restrict__ perm) {
+  const long long n3 = 3 * n;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n3;
+       q += (long long)gridDim.x * blockDim.x) {
+    double v = 0;
+#pragma unroll 8
+    for (int s = 0; s < splits; ++s) v += partial[s * n3 + q];
+    const int c = (q >= n) + (q >= 2 * n);
+    const long long t = q - c * n;
+    if (aos)
+      aos[3 * (perm ? (long long)perm[t] : t) + c] = v;
+    else
+      (c == 0 ? vx : c == 1 ? vy : vz)[t] = v;
   }
 }
 
@@ -683,7 +691,7 @@ struct Variant {
   const char* name;
   int prec;  // NBodyPrec
   int H, TPT, BLOCK, MINB;
-  int packed;  // 1: FP32x2 walker for full strips (FP32, TPT = 2); 2: the far-field walkers over sheet parts
+  int packed;  // 1: FP32x2 near walker (FP32, TPT = 2); 2: the far-field walkers over sheet parts
 };
 
 // Tile shapes: H owned node rows per strip (packed = 2: rows per lane of a
@@ -788,8 +796,8 @@ Error set_smem_once(PerDeviceOnce& once, const void* kern, size_t smem) {
 Error reduce_partials(const NBodyWork* work, long long splits, long long n_targets, double* vx, double* vy, double* vz,
                       int num_sms, cudaStream_t st) {
   const int rb = 256;
-  const int rg = (int)std::min<long long>((n_targets + rb - 1) / rb, (long long)num_sms * 8);
-  reduce_partials_kernel<<<rg, rb, 0, st>>>(work->partial, (int)splits, n_targets, vx, vy, vz);
+  const int rg = (int)std::min<long long>((3 * n_targets + rb - 1) / rb, (long long)num_sms * 8);
+  reduce_partials_kernel<<<rg, rb, 0, st>>>(work->partial, (int)splits, n_targets, vx, vy, vz, work->aos, work->perm);
   UVLM_LAUNCH_CHECK();
   return ok();
 }
@@ -806,8 +814,11 @@ Error launch_variant(const SourceBlock* blocks, int n_blocks, const double* tx, 
                      int num_sms, cudaStream_t st) {
   Blocks B{};
   const long long n_strips = fill_blocks(B, blocks, n_blocks, H);
-  const bool pad = use_padded(B);
-  auto kern = pad ? nbody_kernel<T, Rec, H, TPT, BLOCK, MINB, true, PK> : nbody_kernel<T, Rec, H, TPT, BLOCK, MINB, false, PK>;
+  // the packed walker takes strips of any width, the generic one padded strips only where most are full
+  const bool pad = PK == 1 || use_padded(B);
+  auto kern = nbody_kernel<T, Rec, H, TPT, BLOCK, MINB, true, PK>;
+  if constexpr (PK != 1)
+    if (!pad) kern = nbody_kernel<T, Rec, H, TPT, BLOCK, MINB, false, PK>;
   const size_t smem = 2 * sizeof(Rec) * (H + 1) * (kStripCols + 1);
   static PerDeviceOnce attr_once[2];
   UVLM_TRY(set_smem_once(attr_once[pad ? 1 : 0], (const void*)kern, smem));
@@ -1039,6 +1050,319 @@ Error nbody_batch_eval(NBodyPrec prec, const NBodyBatchInput* d_in, int n, const
     case 2: return run(batch_eval<float, RecF, kBatchTileH[2], kBatchTptF>, grids.tiles[2]);
     default: return run(batch_eval<float, RecF, kBatchTileH[0], kBatchTptF>, grids.tiles[0]);
   }
+}
+
+// ------------------------------------------------------ arbitrary points
+// The far walkers decide per warp, so their speed depends on how close together
+// the targets of a warp lie; points that a program hands over in any order are
+// first put in the order of a space-filling curve.  Twelve bits: each halves the
+// longest edge of the cells (an elongated wake gets most of them along its
+// length), the bits of a point's cell in that order are its key, and a stable
+// counting sort in two passes of six bits orders the keys, so that the order,
+// and with it every rounding, is the same in every run.
+//
+// One cluster of 8 CTAs does all of it in one launch: histograms per warp, their
+// sums over the CTAs through distributed shared memory.  Every warp owns a
+// contiguous range of the points and ranks 32 of them at a time.
+// FP64, 9001 shuffled points around 3 x 61 x 47 rings: 554 -> 409 us with the
+// ordering (about 12 us); FP32, 32768 points, 400 x 128 rings: 4369 -> 2570.
+constexpr int kOrderCtas = 8, kOrderThreads = 1024, kOrderWarps = kOrderThreads / 32;
+constexpr int kOrderBits = 12, kOrderDigit = 6, kOrderBins = 1 << kOrderDigit;
+
+namespace {
+struct OrderSmem {
+  int hist[kOrderWarps][kOrderBins];  // counts per warp, then each warp's next position
+  int total[kOrderBins];              // counts of this CTA
+  int wsum[2];
+  int lo[3], hi[3];                   // bounding box as ordered integers
+  float scale[3], org[3];
+  int bits[3];
+  unsigned dims;                      // two bits per key bit: the dimension it halves
+};
+
+__device__ __forceinline__ int ordered_int(float x) {
+  const int b = __float_as_int(x);
+  return b >= 0 ? b : b ^ 0x7fffffff;
+}
+__device__ __forceinline__ float ordered_float(int b) { return __int_as_float(b >= 0 ? b : b ^ 0x7fffffff); }
+
+// Lanes whose point has this lane's digit (points past the end: digit -1).
+__device__ __forceinline__ void order_count(OrderSmem& sm, int warp, int digit) {
+  const unsigned same = __match_any_sync(0xffffffffu, digit);
+  if (digit >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1) sm.hist[warp][digit] += __popc(same);
+  __syncwarp();
+}
+__device__ __forceinline__ int order_place(OrderSmem& sm, int warp, int digit) {
+  const int lane = threadIdx.x & 31;
+  const unsigned same = __match_any_sync(0xffffffffu, digit);
+  const int at = digit >= 0 ? sm.hist[warp][digit] + __popc(same & ((1u << lane) - 1)) : 0;
+  __syncwarp();
+  if (digit >= 0 && lane == __ffs(same) - 1) sm.hist[warp][digit] += __popc(same);
+  __syncwarp();
+  return at;
+}
+
+// Turns the warps' counts into their first positions.  Every thread of the
+// cluster calls it; the counts of this CTA are complete for the calling warp only.
+__device__ __forceinline__ void order_scan(cooperative_groups::cluster_group& cl, OrderSmem& sm) {
+  const int tid = threadIdx.x, rank = (int)cl.block_rank();
+  __syncthreads();
+  if (tid < kOrderBins) {
+    int s = 0;
+    for (int w = 0; w < kOrderWarps; ++w) {
+      const int c = sm.hist[w][tid];
+      sm.hist[w][tid] = s;
+      s += c;
+    }
+    sm.total[tid] = s;
+  }
+  cl.sync();
+  int first = 0;
+  if (tid < kOrderBins) {
+    int all = 0;
+#pragma unroll
+    for (int c = 0; c < kOrderCtas; ++c) {
+      const int v = *cl.map_shared_rank(&sm.total[tid], c);
+      all += v;
+      first += c < rank ? v : 0;
+    }
+    int scan = all;  // inclusive over the bins of the warp
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, scan, off);
+      if ((tid & 31) >= off) scan += v;
+    }
+    if ((tid & 31) == 31) sm.wsum[tid >> 5] = scan;
+    first += scan - all;
+  }
+  __syncthreads();
+  if (tid < kOrderBins) {
+    if (tid >= 32) first += sm.wsum[0];
+    for (int w = 0; w < kOrderWarps; ++w) sm.hist[w][tid] += first;
+  }
+  __syncthreads();
+}
+
+__global__ void __cluster_dims__(kOrderCtas, 1, 1) __launch_bounds__(kOrderThreads)
+    order_points_kernel(const double* __restrict__ x, int n, unsigned short* keys, int* first_order, int* perm,
+                        double* __restrict__ tx, double* __restrict__ ty, double* __restrict__ tz) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ OrderSmem sm;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int per_warp = (int)(((long long)n + 32 * kOrderCtas * kOrderWarps - 1) / (32 * kOrderCtas * kOrderWarps)) * 32;
+  const long long begin = (long long)per_warp * ((int)cl.block_rank() * kOrderWarps + warp);
+  const int i0 = (int)min((long long)n, begin), i1 = (int)min((long long)n, begin + per_warp);
+  constexpr int kBatch = 4;  // rows of 32 points whose loads are issued together
+
+  // ---- bounding box of the finite points
+  if (tid < 3) {
+    sm.lo[tid] = INT_MAX;
+    sm.hi[tid] = INT_MIN;
+  }
+  for (int q = tid; q < kOrderWarps * kOrderBins; q += kOrderThreads) (&sm.hist[0][0])[q] = 0;
+  __syncthreads();
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+#pragma unroll 4
+  for (int i = i0 + lane; i < i1; i += 32) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const float f = (float)x[3LL * i + d];
+      if (fabsf(f) < 1e30f) {
+        lo[d] = min(lo[d], ordered_int(f));
+        hi[d] = max(hi[d], ordered_int(f));
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = __reduce_min_sync(0xffffffffu, lo[d]);
+    hi[d] = __reduce_max_sync(0xffffffffu, hi[d]);
+    if (lane == 0) {
+      atomicMin(&sm.lo[d], lo[d]);
+      atomicMax(&sm.hi[d], hi[d]);
+    }
+  }
+  cl.sync();
+  if (warp == 0) {
+    float edge[3], org[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const int l = lane < kOrderCtas ? *cl.map_shared_rank(&sm.lo[d], lane) : INT_MAX;
+      const int h = lane < kOrderCtas ? *cl.map_shared_rank(&sm.hi[d], lane) : INT_MIN;
+      const int L = __reduce_min_sync(0xffffffffu, l), H = __reduce_max_sync(0xffffffffu, h);
+      org[d] = L <= H ? ordered_float(L) : 0.f;
+      edge[d] = L <= H ? ordered_float(H) - org[d] : 0.f;
+    }
+    if (lane == 0) {
+      const float whole[3] = {edge[0], edge[1], edge[2]};
+      int bits[3] = {0, 0, 0};
+      unsigned dims = 0;
+      for (int b = 0; b < kOrderBits; ++b) {
+        const int d = edge[0] >= edge[1] && edge[0] >= edge[2] ? 0 : (edge[1] >= edge[2] ? 1 : 2);
+        edge[d] *= 0.5f;
+        bits[d] += 1;
+        dims |= (unsigned)d << (2 * b);
+      }
+      sm.dims = dims;
+      for (int d = 0; d < 3; ++d) {
+        sm.bits[d] = bits[d];
+        sm.org[d] = org[d];
+        sm.scale[d] = whole[d] > 0.f ? (float)(1 << bits[d]) / whole[d] : 0.f;
+      }
+    }
+  }
+  __syncthreads();
+  const unsigned dims = sm.dims;
+  auto key_of = [&](const double (&p)[3]) {
+    int q[3], left[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      left[d] = sm.bits[d];
+      q[d] = min(max((int)(((float)p[d] - sm.org[d]) * sm.scale[d]), 0), (1 << left[d]) - 1);
+    }
+    int key = 0;
+#pragma unroll
+    for (int b = 0; b < kOrderBits; ++b) {
+      const int d = dims >> (2 * b) & 3;
+      const int l = --(d == 0 ? left[0] : d == 1 ? left[1] : left[2]);
+      key = key << 1 | ((d == 0 ? q[0] : d == 1 ? q[1] : q[2]) >> l & 1);
+    }
+    return key;
+  };
+
+  // ---- pass 1: the keys' low digits, in the given order
+  for (int r = i0; r < i1; r += 32 * kBatch) {
+    double p[kBatch][3];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) p[b][d] = r + 32 * b + lane < i1 ? x[3LL * (r + 32 * b + lane) + d] : 0.0;
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      if (r + 32 * b >= i1) break;
+      const bool in = r + 32 * b + lane < i1;
+      const int key = key_of(p[b]);
+      if (in) keys[r + 32 * b + lane] = (unsigned short)key;
+      order_count(sm, warp, in ? key & (kOrderBins - 1) : -1);
+    }
+  }
+  order_scan(cl, sm);
+  unsigned short* keys2 = keys + n;
+  for (int r = i0; r < i1; r += 32 * kBatch) {
+    int key[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) key[b] = r + 32 * b + lane < i1 ? keys[r + 32 * b + lane] : -1;
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      if (r + 32 * b >= i1) break;
+      const int at = order_place(sm, warp, key[b] >= 0 ? key[b] & (kOrderBins - 1) : -1);
+      if (key[b] >= 0) {
+        keys2[at] = (unsigned short)key[b];
+        first_order[at] = r + 32 * b + lane;
+      }
+    }
+  }
+  cl.sync();  // the first order is complete, and the positions are no longer read
+
+  // ---- pass 2: the high digits, in the first order
+  for (int q = tid; q < kOrderWarps * kOrderBins; q += kOrderThreads) (&sm.hist[0][0])[q] = 0;
+  __syncthreads();
+  for (int r = i0; r < i1; r += 32 * kBatch) {
+    int key[kBatch];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) key[b] = r + 32 * b + lane < i1 ? (int)__ldcg(keys2 + r + 32 * b + lane) : -1;
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      if (r + 32 * b >= i1) break;
+      order_count(sm, warp, key[b] >= 0 ? key[b] >> kOrderDigit : -1);
+    }
+  }
+  order_scan(cl, sm);
+  for (int r = i0; r < i1; r += 32 * kBatch) {
+    int key[kBatch], id[kBatch];
+    double p[kBatch][3];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int i = r + 32 * b + lane;
+      key[b] = i < i1 ? (int)__ldcg(keys2 + i) : -1;
+      id[b] = i < i1 ? __ldcg(first_order + i) : 0;
+    }
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) p[b][d] = x[3LL * id[b] + d];
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      if (r + 32 * b >= i1) break;
+      const int at = order_place(sm, warp, key[b] >= 0 ? key[b] >> kOrderDigit : -1);
+      if (key[b] >= 0) {
+        perm[at] = id[b];
+        tx[at] = p[b][0];
+        ty[at] = p[b][1];
+        tz[at] = p[b][2];
+      }
+    }
+  }
+  cl.sync();  // no CTA leaves while its counts may be read
+}
+
+__global__ void split_points_kernel(const double* __restrict__ a, long long n, double* __restrict__ x,
+                                    double* __restrict__ y, double* __restrict__ z) {
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < 3 * n;
+       q += (long long)gridDim.x * blockDim.x) {
+    const long long t = q / 3;
+    const int c = (int)(q - 3 * t);
+    (c == 0 ? x : c == 1 ? y : z)[t] = a[q];
+  }
+}
+}  // namespace
+
+size_t nbody_order_bytes(long long n_targets) { return (size_t)n_targets * 12 + 16; }
+
+// The rule, from shuffled points in and around wakes of 30 to 50,000 segments.
+// FP64: the far walkers for any set, in order from 2^24 pairs and 800 segments
+// per target on (below, the ordering costs more than it gives: 12 x 16 rings and
+// 60,000 points, 144 us as given, 180 in order; 60 x 60 and 3000, 116 and 106).
+// FP32: in order from 2^27 pairs and 2000 segments on (3 x 61 x 47 rings and 9001
+// points, 325 us as given, 227 in order).  Below, the far walkers' set-up and
+// their divergence outweigh their cheaper pairs, and the near walker takes every
+// pair (4500 points: 183 us far as given, 144 in order, 132 near), with fewer rows
+// per strip where strips are few (400 points, 50 x 50 rings: 34 us, 38 otherwise).
+constexpr int kNearVariantF32 = 13, kNearVariantSmallF32 = 14;  // fp32_h3_t2_b128_x2, fp32_h2_t2_b128_x2
+
+Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec, const double* targets,
+                        long long n_targets, double* out, NBodyWork* work, double* soa, void* order, int num_sms,
+                        cudaStream_t st) {
+  if (n_targets <= 0) return ok();
+  const long long segs = nbody_unique_segments(blocks, n_blocks);
+  if (segs == 0) {
+    UVLM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * 3 * n_targets, st));
+    return ok();
+  }
+  double *tx = soa, *ty = soa + n_targets, *tz = soa + 2 * n_targets;
+  const bool f32 = prec == kNBodyFP32;
+  const bool sort = n_targets < (1 << 30) && segs >= (f32 ? 2000 : 800) &&
+                    segs >= (1LL << (f32 ? 27 : 24)) / n_targets;
+  NBodyWork w = *work;
+  w.aos = out;
+  w.perm = nullptr;
+  if (sort) {
+    int* first = reinterpret_cast<int*>(order);
+    int* perm = first + n_targets;
+    unsigned short* keys = reinterpret_cast<unsigned short*>(perm + n_targets);
+    order_points_kernel<<<kOrderCtas, kOrderThreads, 0, st>>>(targets, (int)n_targets, keys, first, perm, tx, ty, tz);
+    w.perm = perm;
+  } else {
+    const int blocks_n = (int)std::min<long long>((3 * n_targets + 255) / 256, (long long)num_sms * 8);
+    split_points_kernel<<<blocks_n, 256, 0, st>>>(targets, n_targets, tx, ty, tz);
+  }
+  UVLM_LAUNCH_CHECK();
+  const int variant = !f32 ? kDefaultVariantF64
+                      : sort ? kDefaultVariantF32
+                      : segs >= (1LL << 24) / n_targets ? kNearVariantF32 : kNearVariantSmallF32;
+  return nbody_eval(blocks, n_blocks, prec, tx, ty, tz, n_targets, nullptr, nullptr, nullptr, &w, variant, num_sms,
+                    st);
 }
 
 // ------------------------------------------------------------- AoS rings

@@ -89,6 +89,10 @@ struct NBodyWork {
   bool near64 = false;
   void* records64 = nullptr;  // RecD array, same indices as records
   long long records64_cap = 0;
+  // where set, the velocity of target t goes to aos[3 perm[t]] (perm NULL: 3 t)
+  // instead of vx, vy, vz
+  double* aos = nullptr;
+  const int* perm = nullptr;
 };
 
 // ------------------------------------------------------------ record build
@@ -369,6 +373,13 @@ Error nbody_eval(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
                  const double* tx, const double* ty, const double* tz,
                  long long n_targets, double* vx, double* vy, double* vz,
                  NBodyWork* work, int variant, int num_sms, cudaStream_t st);
+
+// The same at arbitrary AoS targets, AoS velocities.  soa: 3 n_targets doubles;
+// order: nbody_order_bytes(n_targets) bytes.
+size_t nbody_order_bytes(long long n_targets);
+Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec, const double* targets,
+                        long long n_targets, double* out, NBodyWork* work, double* soa, void* order, int num_sms,
+                        cudaStream_t st);
 
 // out[t] = base[t] + (velocity induced at target t by AoS rings + add3) scale
 // in FP64 (base and add3 may be NULL; targets, base and out are AoS, and base

@@ -6,8 +6,8 @@
 // all device memory themselves and hand out only buffers they own.  This entry
 // point computes the same velocities as uvlm_sheet_induced_velocity, but its
 // inputs and outputs are device pointers owned by the caller and all of its
-// scratch (the source records, the per-split partial sums and the SoA
-// target/velocity vectors) lives in one file-scope device array of
+// scratch (the source records, the per-split partial sums, the targets by
+// component and their order) lives in one file-scope device array of
 // kNoAllocScratchBytes (32 MiB).  Every GPU that loads this library holds that
 // array until the process exits.
 //
@@ -59,24 +59,7 @@ Error scratch_address(void** out) {
   return ok();
 }
 
-__global__ void noalloc_aos_to_soa(const double* a, long long n, double* x, double* y, double* z) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    x[k] = a[3 * k];
-    y[k] = a[3 * k + 1];
-    z[k] = a[3 * k + 2];
-  }
-}
-
-__global__ void noalloc_soa_to_aos(const double* x, const double* y, const double* z, long long n, double* a) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    a[3 * k] = x[k];
-    a[3 * k + 1] = y[k];
-    a[3 * k + 2] = z[k];
-  }
-}
-
 inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
-inline int grid1d(long long n) { return (int)std::min<long long>(std::max<long long>((n + 255) / 256, 1), 4096); }
 
 Error run_noalloc(const double* pos, const double* gamma, int64_t num, int64_t grows, int64_t gcols,
                   const double* targets, int64_t n_targets, double* out, int32_t precision, cudaStream_t st) {
@@ -114,20 +97,14 @@ Error run_noalloc(const double* pos, const double* gamma, int64_t num, int64_t g
   void* base = nullptr;
   UVLM_TRY(scratch_address(&base));
   unsigned char* p = static_cast<unsigned char*>(base);
-  double* tx = reinterpret_cast<double*>(p);
-  double* ty = reinterpret_cast<double*>(p + vec_bytes);
-  double* tz = reinterpret_cast<double*>(p + 2 * vec_bytes);
-  double* vx = reinterpret_cast<double*>(p + 3 * vec_bytes);
-  double* vy = reinterpret_cast<double*>(p + 4 * vec_bytes);
-  double* vz = reinterpret_cast<double*>(p + 5 * vec_bytes);
+  double* soa = reinterpret_cast<double*>(p);  // three vectors, and the order in the place of three more
+  void* order = p + 3 * vec_bytes;
   NBodyWork w;
   w.records = p + 6 * vec_bytes;
   w.records_cap = (long long)rec_bytes;
   w.partial = reinterpret_cast<double*>(p + fixed);
   w.partial_cap = (long long)((kNoAllocScratchBytes - fixed) / sizeof(double));
   w.max_splits = (long long)((kNoAllocScratchBytes - fixed) / one_split);
-  noalloc_aos_to_soa<<<grid1d(n_targets), 256, 0, st>>>(targets, n_targets, tx, ty, tz);
-  UVLM_LAUNCH_CHECK();
   if (has_rings) {
     SheetView v{pos, (int)grows + 1, 0, gamma, (int)grows, 0, (int)num, (int)grows + 1, (int)gcols};
     SourceBlock blk;
@@ -135,13 +112,10 @@ Error run_noalloc(const double* pos, const double* gamma, int64_t num, int64_t g
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    UVLM_TRY(nbody_eval(&blk, 1, prec, tx, ty, tz, n_targets, vx, vy, vz, &w,
-                        prec == kNBodyFP32 ? kDefaultVariantF32 : kDefaultVariantF64, sms, st));
+    UVLM_TRY(nbody_eval_points(&blk, 1, prec, targets, n_targets, out, &w, soa, order, sms, st));
   } else {
-    UVLM_CUDA_TRY(cudaMemsetAsync(vx, 0, 3 * vec_bytes, st));
+    UVLM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)n_targets, st));
   }
-  noalloc_soa_to_aos<<<grid1d(n_targets), 256, 0, st>>>(vx, vy, vz, n_targets, out);
-  UVLM_LAUNCH_CHECK();
   return ok();
 }
 

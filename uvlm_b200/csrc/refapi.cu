@@ -161,27 +161,18 @@ int uvlm_sheet_induced_velocity(const double* pos, const double* gamma, int64_t 
   if (n_targets == 0) return UVLM_OK;
   Scratch S;
   const NBodyPrec prec = precision == UVLM_PRECISION_MIXED ? kNBodyFP32 : kNBodyFP64;
-  double *dp, *dg, *dt, *vx, *vy, *vz, *dout;
+  double *dp, *dg, *dt, *dout;
   Error e;
   auto run = [&]() -> Error {
     UVLM_TRY(S.up(&dp, pos, (size_t)(num * (grows + 1) * (gcols + 1) * 3)));
     UVLM_TRY(S.up(&dg, gamma, (size_t)(num * grows * gcols)));
     UVLM_TRY(S.up(&dt, targets, (size_t)(3 * n_targets)));
-    UVLM_TRY(S.get(&vx, n_targets));
-    UVLM_TRY(S.get(&vy, n_targets));
-    UVLM_TRY(S.get(&vz, n_targets));
     UVLM_TRY(S.get(&dout, 3 * n_targets));
     SheetView v{dp, (int)grows + 1, 0, dg, (int)grows, 0, (int)num, (int)grows + 1, (int)gcols};
-    const int nv = (grows > 0 && gcols > 0 && num > 0) ? 1 : 0;
-    if (nv)
-      UVLM_TRY(velocity_at(&v, nv, prec, dt, n_targets, vx, vy, vz, S));
-    else {
-      UVLM_CUDA_TRY(cudaMemset(vx, 0, 8 * n_targets));
-      UVLM_CUDA_TRY(cudaMemset(vy, 0, 8 * n_targets));
-      UVLM_CUDA_TRY(cudaMemset(vz, 0, 8 * n_targets));
-    }
-    soa_to_aos<<<gfor(n_targets), 256>>>(vx, vy, vz, n_targets, dout, nullptr, nullptr, 1.0);
-    UVLM_LAUNCH_CHECK();
+    if (grows > 0 && gcols > 0 && num > 0)
+      UVLM_TRY(velocity_at(&v, 1, prec, dt, n_targets, dout, S));
+    else
+      UVLM_CUDA_TRY(cudaMemset(dout, 0, sizeof(double) * 3 * n_targets));
     UVLM_CUDA_TRY(cudaMemcpy(out, dout, sizeof(double) * 3 * n_targets, cudaMemcpyDeviceToHost));
     return ok();
   };

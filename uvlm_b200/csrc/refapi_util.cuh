@@ -1,5 +1,5 @@
 // refapi_util.cuh -- helpers shared by the context-free C-ABI entry points
-// (refapi.cu, legacy.cu): AoS/SoA conversion, the
+// (refapi.cu, legacy.cu): the
 // FP64/FP32 N-body of sheets and of AoS rings at arbitrary targets and a
 // fixed-order block sum.
 #pragma once
@@ -26,24 +26,6 @@ int sms() {
   return v;
 }
 
-__global__ void aos_to_soa(const double* a, long long n, double* x, double* y, double* z) {
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    x[k] = a[3 * k];
-    y[k] = a[3 * k + 1];
-    z[k] = a[3 * k + 2];
-  }
-}
-__global__ void soa_to_aos(const double* x, const double* y, const double* z, long long n, double* a, const double* add3,
-                           const double* base, double scale) {
-  // a = base + (v + add3) * scale   (base/add3 may be NULL)
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    double v[3] = {x[k], y[k], z[k]};
-    for (int d = 0; d < 3; ++d) {
-      double u = v[d] + (add3 ? add3[d] : 0.0);
-      a[3 * k + d] = base ? base[3 * k + d] + u * scale : u;
-    }
-  }
-}
 constexpr int kSumThreads = 256;
 
 __device__ inline d3 block_sum3(d3 v, double* sh) {
@@ -66,32 +48,40 @@ __device__ inline d3 block_sum3(d3 v, double* sh) {
 
 inline int gfor(long long n) { return (int)std::min<long long>(std::max<long long>((n + 255) / 256, 1), 65535); }
 
-// Velocities of the sheets at SoA targets.  The partial sums get room for 64
-// splits of few target tiles; from 64 tiles on fewer splits fill the device.
+// Records of the sheets and room for the partial sums: 64 splits of few target
+// tiles; from 64 tiles on fewer splits fill the device.
+Error sources_at(const SheetView* views, int nv, NBodyPrec prec, long long nt, NBodyWork* w, SourceBlock* blocks,
+                 Scratch& S) {
+  long long recs = 0;
+  for (int i = 0; i < nv; ++i) recs += (long long)views[i].num * views[i].node_rows * (views[i].cols + 1);
+  w->records_cap = std::max<long long>(recs, 1) * (long long)(prec == kNBodyFP32 ? sizeof(RecF) : sizeof(RecD));
+  UVLM_TRY(S.get(reinterpret_cast<char**>(&w->records), (size_t)w->records_cap));
+  w->partial_cap = 3 * std::max<long long>(nt, 1) * (nt > 64 * 256 ? 24 : kMaxSplits);
+  UVLM_TRY(S.get(&w->partial, (size_t)w->partial_cap));
+  return nbody_build_sources(views, nv, prec, w, blocks, 0);
+}
+
+// Velocities of the sheets at SoA targets in the order given.
 Error velocity_soa(const SheetView* views, int nv, NBodyPrec prec, const double* tx, const double* ty,
                    const double* tz, long long nt, double* vx, double* vy, double* vz, Scratch& S) {
   NBodyWork w;
-  long long recs = 0;
-  for (int i = 0; i < nv; ++i) recs += (long long)views[i].num * views[i].node_rows * (views[i].cols + 1);
-  w.records_cap = std::max<long long>(recs, 1) * (long long)(prec == kNBodyFP32 ? sizeof(RecF) : sizeof(RecD));
-  UVLM_TRY(S.get(reinterpret_cast<char**>(&w.records), (size_t)w.records_cap));
-  w.partial_cap = 3 * std::max<long long>(nt, 1) * (nt > 64 * 256 ? 24 : kMaxSplits);
-  UVLM_TRY(S.get(&w.partial, (size_t)w.partial_cap));
   SourceBlock blocks[4];
-  UVLM_TRY(nbody_build_sources(views, nv, prec, &w, blocks, 0));
+  UVLM_TRY(sources_at(views, nv, prec, nt, &w, blocks, S));
   const int variant = prec == kNBodyFP32 ? kDefaultVariantF32 : kDefaultVariantF64;
   return nbody_eval(blocks, nv, prec, tx, ty, tz, nt, vx, vy, vz, &w, variant, sms(), 0);
 }
 
-Error velocity_at(const SheetView* views, int nv, NBodyPrec prec, const double* d_targets_aos, long long nt,
-                  double* vx, double* vy, double* vz, Scratch& S) {
-  double *tx, *ty, *tz;
-  UVLM_TRY(S.get(&tx, nt));
-  UVLM_TRY(S.get(&ty, nt));
-  UVLM_TRY(S.get(&tz, nt));
-  aos_to_soa<<<gfor(nt), 256>>>(d_targets_aos, nt, tx, ty, tz);
-  UVLM_LAUNCH_CHECK();
-  return velocity_soa(views, nv, prec, tx, ty, tz, nt, vx, vy, vz, S);
+// Velocities of the sheets at arbitrary AoS targets.
+Error velocity_at(const SheetView* views, int nv, NBodyPrec prec, const double* d_targets, long long nt,
+                  double* d_out, Scratch& S) {
+  NBodyWork w;
+  SourceBlock blocks[4];
+  double* soa;
+  char* order;
+  UVLM_TRY(S.get(&soa, 3 * nt));
+  UVLM_TRY(S.get(&order, nbody_order_bytes(nt)));
+  UVLM_TRY(sources_at(views, nv, prec, nt, &w, blocks, S));
+  return nbody_eval_points(blocks, nv, prec, d_targets, nt, d_out, &w, soa, order, sms(), 0);
 }
 
 // out = base + (velocity induced by AoS rings at AoS targets + add3) scale, all
