@@ -274,3 +274,24 @@ def test_per_case_solve_at_its_block_edges(precision):
         ref = one.Run(steps - 1, dt)
         one.close()
         assert np.max(np.abs(rows[:, k, 1:] - ref[:, 1:])) <= tol * np.max(np.abs(ref[:, 1:])), (r, c)
+
+
+@pytest.mark.parametrize("n", [2, 37, 38, 49, 50, 74, 75, 149])
+def test_solve_clusters_of_every_size_give_the_same_loads(n):
+    """Batches whose cases are solved by clusters of 4, 3, 2 and 1 CTAs (as many as run all cases at once): copies of one
+    case, N = 90 (rows that leave remainders in every CTA's share), against a batch of one, to the mixed tolerance."""
+    import uvlm_b200 as U
+    from uvlm_b200.batch import BatchSimulator
+
+    def loads(copies):
+        sim = BatchSimulator(precision="mixed", max_steps=5, nbody_tile=0)
+        m = U.Morphing().set_alpha(0.05).set_plug(0.1, 1.0).set_twist(0.1, 1.0, math.pi / 2)
+        for _ in range(copies):
+            sim.add_case(m, 1.0, 4.0, 9, 10, 0.15)
+        sim.run(5)
+        rows = sim.loads()
+        sim.close()
+        return rows[:, :, 1:]
+
+    one, many = loads(1), loads(n)
+    assert np.max(np.abs(many - one)) <= 1e-6 * np.max(np.abs(one))

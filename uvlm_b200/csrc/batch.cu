@@ -29,6 +29,8 @@
 #include <string>
 #include <vector>
 
+#include <cooperative_groups.h>
+
 #include "../../include/uvlm_b200.h"
 #include "bs_math.cuh"
 #include "host_lattice.h"
@@ -689,6 +691,16 @@ constexpr double kStaleContraction = 0.5;
 // that does not reach the tolerance, or a sweep contracts the residual by less
 // than kStaleContraction, is the FP32 copy of the current A factored again
 // (each case decides for itself; refac counts the factorisations).
+//
+// Mixed form, batches of fewer cases than SMs: a case is a cluster of up to
+// kSolveCluster CTAs.  The first does all of the above; the others help with the
+// residuals, each for its share of the rows of A, which one SM would stream at
+// 100 GB/s (8 MB for 1024 rings): they wait for a command, read x from the first
+// CTA's shared memory and write their part of r there.  A row's sum is the same
+// whoever forms it.  Bound: the chain of block rows of the two triangular solves
+// of a sweep.  40 cases of up to 1024 rings, a step with two
+// sweeps: 1.33 -> 1.20 ms.
+constexpr int kSolveCluster = 4;
 template <class T>
 __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BCase* __restrict__ cs, double* A64, float* F32,
                                                                 int* perm_all, double* dinv_all, const double* rhs, double* gamma,
@@ -698,10 +710,14 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
                                                                 int* sweeps_out, double* res_out, int* status,
                                                                 const int* __restrict__ order) {
   constexpr int NT = SolveCfg<T>::kThreads;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int helpers = (int)cl.num_blocks() - 1, rank = (int)cl.block_rank();
   extern __shared__ __align__(16) double sm[];
-  // CTA i takes the i-th largest case: with more cases than SMs the largest
+  __shared__ int go;  // the first CTA's command: residual rows, or done
+  // cluster i takes the i-th largest case: with more cases than SMs the largest
   // start first instead of forming the launch's last wave
-  const int ci = order[blockIdx.x];
+  const int ci = order[blockIdx.x / (helpers + 1)];
   const BCase& b = cs[ci];
   const int N = b.N;
   double* x = sm;
@@ -721,12 +737,12 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
     for (int i = threadIdx.x; i < N; i += NT) bn += bb[i] * bb[i];
     bn = sqrt(cta_sum<NT>(bn));
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // r = b - A x (FP64), returns ||r|| / ||b|| (same value in every thread)
-    auto residual = [&]() -> double {
+    // this CTA's rows of r = b - A x (FP64) into `to`
+    auto residual_rows = [&](double* to) {
       // four rows per warp at a time, so that enough loads of A are in
       // flight for one SM to stream the matrix
-      constexpr int kW = NT / 32;
-      for (int i0 = wid; i0 < N; i0 += 4 * kW) {
+      const int kW = (helpers + 1) * (NT / 32);
+      for (int i0 = rank * (NT / 32) + wid; i0 < N; i0 += 4 * kW) {
         const double* a0 = A + (long long)i0 * N;
         const bool v1 = i0 + kW < N, v2 = i0 + 2 * kW < N, v3 = i0 + 3 * kW < N;
         const double* a1 = v1 ? a0 + (long long)kW * N : a0;
@@ -750,12 +766,35 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
           c3 += __shfl_down_sync(0xffffffffu, c3, off);
         }
         if (lane == 0) {
-          r[i0] = bb[i0] - c0;
-          if (v1) r[i0 + kW] = bb[i0 + kW] - c1;
-          if (v2) r[i0 + 2 * kW] = bb[i0 + 2 * kW] - c2;
-          if (v3) r[i0 + 3 * kW] = bb[i0 + 3 * kW] - c3;
+          to[i0] = bb[i0] - c0;
+          if (v1) to[i0 + kW] = bb[i0 + kW] - c1;
+          if (v2) to[i0 + 2 * kW] = bb[i0 + 2 * kW] - c2;
+          if (v3) to[i0 + 3 * kW] = bb[i0 + 3 * kW] - c3;
         }
       }
+    };
+    if (rank > 0) {
+      double* r0 = cl.map_shared_rank(r, 0);
+      const double* x0 = cl.map_shared_rank(x, 0);
+      while (true) {
+        cl.sync();  // a command; x is final
+        if (!*cl.map_shared_rank(&go, 0)) break;
+        for (int i = threadIdx.x; i < N; i += NT) x[i] = x0[i];
+        __syncthreads();
+        residual_rows(r0);
+        cl.sync();  // r is complete
+      }
+      cl.sync();  // the command is read: the first CTA may leave
+      return;
+    }
+    // r = b - A x, returns ||r|| / ||b|| (same value in every thread)
+    auto residual = [&]() -> double {
+      if (helpers) {
+        if (threadIdx.x == 0) go = 1;
+        cl.sync();
+      }
+      residual_rows(r);
+      if (helpers) cl.sync();
       __syncthreads();
       double rn = 0;
       for (int i = threadIdx.x; i < N; i += NT) rn += r[i] * r[i];
@@ -811,6 +850,11 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
       }
     }
     if (threadIdx.x == 0 && !(rel <= tol)) status[3] = 1;
+    if (helpers) {
+      if (threadIdx.x == 0) go = 0;
+      cl.sync();
+      cl.sync();
+    }
   } else {
     cta_lu_factor<T>(A, N, perm, status, panel, map, map + N);
     if (threadIdx.x == 0) atomicAdd(refac, 1ull);
@@ -1006,6 +1050,21 @@ struct uvlm_batch {
   uvlm_batch_config cfg{};
   std::string err;
   int n = 0, cap = 0, num_sms = 148, grid = 0;
+  int solve_ctas = 1;  // CTAs per case of the mixed form's solve
+  // Launch of the mixed form's solve; `attr` has to outlive it.
+  cudaLaunchConfig_t solve_launch(cudaLaunchAttribute* attr, cudaStream_t st) const {
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(n * solve_ctas);
+    lc.blockDim = dim3(SolveCfg<float>::kThreads);
+    lc.dynamicSmemBytes = solve_smem_bytes<float>(max_N);
+    lc.stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = solve_ctas;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    lc.attrs = attr;
+    lc.numAttrs = 1;
+    return lc;
+  }
   NBodyBatchGrids nb_grids;
   int64_t steps_done = 0;
   std::vector<BCase> hc;
@@ -1253,6 +1312,18 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   else
     UVLM_CUDA_TRY(cudaFuncSetAttribute(b_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)solve_smem_bytes<double>(max_N)));
+  if (mixed()) {
+    // as many CTAs per case as run all cases at once
+    for (solve_ctas = kSolveCluster; solve_ctas > 1; --solve_ctas) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t lc = solve_launch(&attr, 0);
+      int clusters = 0;
+      if (solve_ctas * n <= num_sms &&
+          cudaOccupancyMaxActiveClusters(&clusters, b_solve_kernel<float>, &lc) == cudaSuccess && clusters >= n)
+        break;
+      cudaGetLastError();
+    }
+  }
   nb_grids = nbody_batch_grids(prec(), num_sms);
   grid = num_sms * 8;
   return ok();
@@ -1351,11 +1422,15 @@ Error uvlm_batch::enqueue_step() {
   b_rhs_kernel<<<grid, 256, 0, st>>>(d_cases, P, n, d_vx, d_vy, d_vz, d_uls, d_normal, d_rhs);
   UVLM_LAUNCH_CHECK();
   // solve
-  if (mixed())
-    b_solve_kernel<float><<<n, SolveCfg<float>::kThreads, solve_smem_bytes<float>(max_N), st>>>(
-        d_cases, d_A64, d_F32, d_perm, d_dinv, d_rhs, d_gamma, d_gamma_hist, d_step, cfg.refine_max_iter,
-        cfg.refine_tol, cfg.stale_factors, d_has_factor, d_refac, d_sweeps, d_res, d_status, d_solve_order);
-  else
+  if (mixed()) {
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t lc = solve_launch(&attr, st);
+    UVLM_CUDA_TRY(cudaLaunchKernelEx(&lc, b_solve_kernel<float>, (const BCase*)d_cases, d_A64, d_F32, d_perm, d_dinv,
+                                     (const double*)d_rhs, d_gamma, (const double*)d_gamma_hist,
+                                     (const long long*)d_step, (int)cfg.refine_max_iter, (double)cfg.refine_tol,
+                                     (int)cfg.stale_factors, d_has_factor, d_refac, d_sweeps, d_res, d_status,
+                                     (const int*)d_solve_order));
+  } else
     b_solve_kernel<double><<<n, SolveCfg<double>::kThreads, solve_smem_bytes<double>(max_N), st>>>(
         d_cases, d_A64, d_F32, d_perm, nullptr, d_rhs, d_gamma, d_gamma_hist, d_step, 0, 0.0, 0, d_has_factor,
         d_refac, d_sweeps, d_res, d_status, d_solve_order);
