@@ -539,8 +539,8 @@ __device__ void cta_lu_factor(T* A, int N, int* perm_out, int* status, T* P, int
 }
 
 // Inverses of the 32 x 32 diagonal blocks of L and of U, one warp per block,
-// one column of the inverse per lane; D[2 b + (U)][l][q] = inverse[q][l], so
-// that a lane per row reads them in order.  FP64 although the factors are FP32:
+// one column of the inverse per lane, stored by rows in D[2 b + (U)].  FP64 although
+// the factors are FP32:
 // rounded to FP32 they cost some cases a third refinement sweep.  Rows past N
 // act as the identity.
 template <class T>
@@ -573,22 +573,80 @@ __device__ void cta_diag_inverses(const T* LU, int N, double* D) {
     }
     double* d = D + (long long)k * B * B;
 #pragma unroll
-    for (int i = 0; i < B; ++i) d[lane * B + i] = x[i];
+    for (int i = 0; i < B; ++i) d[i * B + lane] = x[i];
   }
   __syncthreads();
 }
 
 // y <- (LU)^-1 y in place (y in shared memory, already permuted, FP64
 // arithmetic), block row by block row: every warp forms the products of two or
-// four rows with the part of y that is known, along the rows (coalesced pairs; a
-// thread per row touched a line per value, and one thread replayed the row
-// exchanges before each solve: a step's solve launch with its two sweeps and
-// three FP64 residuals went from 2.07 to 0.72 ms), then one warp solves the 32 x 32 diagonal block: with the
-// block's inverse (D, FP32 factors) or by substitution (FP64 factors).
+// four rows with the part of y that is known, along the rows (a thread per row
+// touched a line per value), then the 32 x 32 diagonal block is applied.
+//
+// FP32 factors, with the inverses of the diagonal blocks (D): bound by the chain of
+// block rows, a round trip to L2 or two and two barriers each, so 16 loads a lane
+// are in flight and the inverse is read ahead of the products and applied by all
+// warps.  256 cases, a step with its two sweeps: 3.71 ms with one warp for it and
+// half the loads, 3.52 now (40 cases 1.21 and 1.12).
+__device__ void cta_lu_solve_f32(const float* LU, int N, const double* D, double* y) {
+  constexpr int kW = SolveCfg<float>::kThreads / 32, B = kSolveBlock, kR = B / kW;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __shared__ double t[B];
+  // block row J0 with the known columns [a, b): the diagonal block's inverse is
+  // read ahead of the products, and its product spread over the warps too
+  auto block = [&](int J0, bool upper, int a, int b) {
+    constexpr int U = 8;
+    const int nb = min(B, N - J0);
+    const double* d = D + (long long)(2 * (J0 / B) + (upper ? 1 : 0)) * B * B;
+    double dv[kR], s[kR];
+    const float* row[kR];
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+      dv[k] = d[(wid + k * kW) * B + lane];
+      row[k] = LU + (long long)(J0 + min(wid + k * kW, nb - 1)) * N;
+      s[k] = 0.0;
+    }
+#pragma unroll 1
+    for (int j0 = a + 2 * lane; j0 < b; j0 += 64 * U) {  // N, a and b are even
+      float2 v[kR][U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < kR; ++k)
+          v[k][u] = j0 + 64 * u < b ? *reinterpret_cast<const float2*>(row[k] + j0 + 64 * u) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (j0 + 64 * u >= b) break;
+        const double2 yj = *reinterpret_cast<const double2*>(y + j0 + 64 * u);
+#pragma unroll
+        for (int k = 0; k < kR; ++k) s[k] += (double)v[k][u].x * yj.x + (double)v[k][u].y * yj.y;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+      for (int off = 16; off; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+      const int r = wid + k * kW;
+      if (lane == 0) t[r] = r < nb ? y[J0 + r] - s[k] : 0.0;
+    }
+    __syncthreads();
+    const double v = t[lane];
+#pragma unroll
+    for (int k = 0; k < kR; ++k) {
+      s[k] = dv[k] * v;
+      for (int off = 16; off; off >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], off);
+      const int r = wid + k * kW;
+      if (lane == 0 && r < nb) y[J0 + r] = s[k];
+    }
+    __syncthreads();
+  };
+  for (int J0 = 0; J0 < N; J0 += B) block(J0, false, 0, J0);
+  for (int J0 = (N - 1) / B * B; J0 >= 0; J0 -= B) block(J0, true, min(J0 + B, N), N);
+}
+
+// FP64 factors: one warp solves the diagonal block by substitution.
 template <class T>
-__device__ void cta_lu_solve(const T* LU, int N, const double* D, double* y) {
+__device__ void cta_lu_solve(const T* LU, int N, double* y) {
   constexpr int NT = SolveCfg<T>::kThreads, kW = NT / 32, B = kSolveBlock, kR = B / kW;
-  using V2 = typename std::conditional<sizeof(T) == 4, float2, double2>::type;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   // y[J0 + r] -= sum over columns [a, b) for the block's rows
   auto products = [&](int J0, int nb, int a, int b) {
@@ -605,8 +663,8 @@ __device__ void cta_lu_solve(const T* LU, int N, const double* D, double* y) {
       const double y0 = y[j], y1 = j + 1 < b ? y[j + 1] : 0.0;
 #pragma unroll
       for (int k = 0; k < kR; ++k) {
-        const V2 v = *reinterpret_cast<const V2*>(row[k] + j);
-        s[k] += (double)v.x * y0 + (double)v.y * y1;
+        const double2 v = *reinterpret_cast<const double2*>(row[k] + j);
+        s[k] += v.x * y0 + v.y * y1;
       }
     }
 #pragma unroll
@@ -618,30 +676,22 @@ __device__ void cta_lu_solve(const T* LU, int N, const double* D, double* y) {
   auto diagonal = [&](int J0, int nb, bool upper) {
     if (wid == 0) {
       double v = lane < nb ? y[J0 + lane] : 0.0;
-      if constexpr (sizeof(T) == 4) {
-        const double* d = D + (long long)(2 * (J0 / B) + (upper ? 1 : 0)) * B * B + lane;
-        double s = 0.0;
+      T a[B];
 #pragma unroll
-        for (int l = 0; l < B; ++l) s += d[l * B] * __shfl_sync(0xffffffffu, v, l);
-        v = s;
+      for (int l = 0; l < B; ++l)
+        a[l] = lane < nb && l < nb ? LU[(long long)(J0 + lane) * N + J0 + l] : (T)(l == lane ? 1 : 0);
+      if (!upper) {
+#pragma unroll
+        for (int l = 0; l < B; ++l) {
+          const double xl = __shfl_sync(0xffffffffu, v, l);
+          if (lane > l) v -= a[l] * xl;
+        }
       } else {
-        T a[B];
 #pragma unroll
-        for (int l = 0; l < B; ++l)
-          a[l] = lane < nb && l < nb ? LU[(long long)(J0 + lane) * N + J0 + l] : (T)(l == lane ? 1 : 0);
-        if (!upper) {
-#pragma unroll
-          for (int l = 0; l < B; ++l) {
-            const double xl = __shfl_sync(0xffffffffu, v, l);
-            if (lane > l) v -= a[l] * xl;
-          }
-        } else {
-#pragma unroll
-          for (int l = B - 1; l >= 0; --l) {
-            if (lane == l) v /= a[l];
-            const double xl = __shfl_sync(0xffffffffu, v, l);
-            if (lane < l) v -= a[l] * xl;
-          }
+        for (int l = B - 1; l >= 0; --l) {
+          if (lane == l) v /= a[l];
+          const double xl = __shfl_sync(0xffffffffu, v, l);
+          if (lane < l) v -= a[l] * xl;
         }
       }
       if (lane < nb) y[J0 + lane] = v;
@@ -699,7 +749,7 @@ constexpr double kStaleContraction = 0.5;
 // CTA's shared memory and write their part of r there.  A row's sum is the same
 // whoever forms it.  Bound: the chain of block rows of the two triangular solves
 // of a sweep.  40 cases of up to 1024 rings, a step with two
-// sweeps: 1.33 -> 1.20 ms.
+// sweeps: 1.33 -> 1.20 ms with helpers, 1.12 with the solves as they are now.
 constexpr int kSolveCluster = 4;
 template <class T>
 __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BCase* __restrict__ cs, double* A64, float* F32,
@@ -804,7 +854,7 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
     auto sweep = [&]() {
       for (int i = threadIdx.x; i < N; i += NT) y[i] = r[perm[i]];
       __syncthreads();
-      cta_lu_solve<T>(LU, N, dinv, y);
+      cta_lu_solve_f32(LU, N, dinv, y);
       for (int i = threadIdx.x; i < N; i += NT) x[i] += y[i];
       __syncthreads();
     };
@@ -838,7 +888,7 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
       }
       for (int i = threadIdx.x; i < N; i += NT) y[i] = bb[perm[i]];
       __syncthreads();
-      cta_lu_solve<T>(LU, N, dinv, y);
+      cta_lu_solve_f32(LU, N, dinv, y);
       for (int i = threadIdx.x; i < N; i += NT) x[i] = y[i];
       __syncthreads();
       sweeps = 0;
@@ -861,7 +911,7 @@ __global__ void __launch_bounds__(SolveCfg<T>::kThreads) b_solve_kernel(const BC
     __syncthreads();
     for (int i = threadIdx.x; i < N; i += NT) x[i] = bb[perm[i]];
     __syncthreads();
-    cta_lu_solve<T>(A, N, nullptr, x);
+    cta_lu_solve<T>(A, N, x);
   }
   bool finite = true;
   for (int i = threadIdx.x; i < N; i += NT) {
