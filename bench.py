@@ -53,10 +53,10 @@ FLOP_PER_PAIR = 59
 # leading CPU_LU_N^2 block, each scaled to the whole step.
 CPU_STRIDE, CPU_LU_N = 32, 2048
 # DRAM bytes of one advection launch of the N-body kernel at the held wake,
-# from an ncu capture of the packed FP32x2 tile with the far-field walker
-# (bench.py --profile): about the algorithmic bytes (56,115 source records x
-# 64 B + targets + outputs).
-NBODY_TRAFFIC = {"heave_pitch": 4899072}
+# from an ncu capture of the FP32x2 walkers over sheet parts (bench.py
+# --profile): about the algorithmic bytes (56,115 source records x 64 B +
+# targets + outputs).
+NBODY_TRAFFIC = {"heave_pitch": 4921600}
 
 
 def variant_index(name):
@@ -707,7 +707,7 @@ def run_ours(args, rank, world, local_rank):
             "plain_fp64_stage_ms": {"kin_shed": stage64[0], "assembly": stage64[1], "rhs": stage64[2],
                                     "solve": stage64[3], "loads": stage64[4], "advect": stage64[5],
                                     "total": stage64[7]},
-            "roofline": {"bound": "fp32_simt", "kernel": "nbody_kernel (every N-body launch of a step: RHS, "
+            "roofline": {"bound": "fp32_simt", "kernel": "nbody_parts_kernel (every N-body launch of a step: RHS, "
                                                               f"loads, {wl.advection} advection)",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": "FP32 FMA probe on this GPU, the larger of scalar FFMA and packed FP32x2 "
@@ -718,7 +718,7 @@ def run_ours(args, rank, world, local_rank):
                          "traffic": NBODY_TRAFFIC.get(wl.name),
                          "traffic_unit": "DRAM bytes per advection launch (ncu dram__bytes_read.sum + "
                                          "dram__bytes_write.sum, one launch at the held wake)"},
-            "plain_fp64_roofline": {"bound": "fp64_simt", "kernel": "nbody_kernel<double> (every N-body launch "
+            "plain_fp64_roofline": {"bound": "fp64_simt", "kernel": "nbody_parts_kernel<double> (every N-body launch "
                                                                      "of a plain FP64 step)",
                                     "achieved": achieved64, "peak": pk64.value, "unit": "TFLOP/s",
                                     "frac": achieved64 / pk64.value,
