@@ -106,3 +106,38 @@ def test_point_sets_that_are_ordered_first(n, kind):
         bound = 1e-12 * scale if precision == "fp64" else 4e-5 * mag + 2e-6 * scale
         assert np.all(np.abs(got - ref).max(axis=1) <= bound)
     np.testing.assert_array_equal(U.InducedVelocity(x, pos, gamma), U.InducedVelocity(x, pos, gamma))
+
+
+# ---------------------------------------------------------------- ends of the range
+def _lattice():
+    pos, gamma = _sheet(1, 9, 40, seed=11, wobble=0.003)
+    return pos, gamma, _targets(pos, seed=12)
+
+
+DISTANCES = [1e9, 1e20, 1e78, 1e100, 1e153, 1e154, 1e155, 1e250]
+
+
+def _far_points(distance, n=64):
+    d = np.random.default_rng(1).standard_normal((n, 3))
+    return d / np.linalg.norm(d, axis=1)[:, None] * distance
+
+
+def _far_limit(gamma, distance):
+    """Bound of the velocity at a distance: every segment is shorter than 1."""
+    return np.abs(gamma).sum() / distance * min(1e3 / distance, 1.0)
+
+
+@pytest.mark.parametrize("distance", DISTANCES)
+def test_near_walkers_and_rings_give_no_velocity_far_away(distance):
+    """Points so far away that products of distances leave the FP64 range: rings, and a sheet of circulations below
+    1e-13, which the near walkers take."""
+    import uvlm_b200 as U
+    from uvlm_b200 import rings as R
+
+    pos, gamma, _ = _lattice()
+    gamma = gamma * 1e-14
+    far = _far_points(distance)
+    n = pos[0]
+    ring = np.stack([n[:-1, :-1], n[:-1, 1:], n[1:, 1:], n[1:, :-1]], 2).reshape(-1, 4, 3)
+    for got in (U.InducedVelocity(far, pos, gamma), R.InducedVelocity(far, ring, gamma.reshape(-1))):
+        assert np.all(np.isfinite(got)) and np.max(np.abs(got)) <= _far_limit(gamma, distance)

@@ -91,7 +91,7 @@ __device__ __forceinline__ float nb_rcp(float x) {
 // remainder is below 2^-56.  Five and three FP64 operations, without the
 // special cases of the library functions: the arguments are squared distances
 // and denominators that the callers' cuts keep away from 0 (what a zero gives
-// is dropped by a select).
+// is dropped by a select), and what an infinite one gives (a NaN) is dropped too.
 __device__ __forceinline__ double nb_rsqrt(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -172,7 +172,11 @@ __device__ __forceinline__ void seg(const SegV<T>& r0, const NodeV<T>& a, const 
   const T num = (a.n + b.n) * (beyond ? (T)1 : nn - dot12);
   const T den = nn * (beyond ? nn + dot12 : d2);
   T k = g * num * nb_rcp(den);
-  k = (d2 >= (T)kCutD2 && nn > (T)0) ? k : (T)0;
+  bool keep = d2 >= (T)kCutD2 && nn > (T)0;
+  // an infinite denominator (|r| above about 1e77): the velocity underflows,
+  // and nb_rcp has no answer
+  if constexpr (sizeof(T) == 8) keep = keep && __double2hiint(den) != 0x7ff00000;
+  k = keep ? k : (T)0;
   vx += k * dx;
   vy += k * dy;
   vz += k * dz;
