@@ -141,3 +141,104 @@ def test_near_walkers_and_rings_give_no_velocity_far_away(distance):
     ring = np.stack([n[:-1, :-1], n[:-1, 1:], n[1:, 1:], n[1:, :-1]], 2).reshape(-1, 4, 3)
     for got in (U.InducedVelocity(far, pos, gamma), R.InducedVelocity(far, ring, gamma.reshape(-1))):
         assert np.all(np.isfinite(got)) and np.max(np.abs(got)) <= _far_limit(gamma, distance)
+
+
+# ---------------------------------------------------------------- pinned tiles
+def _velocity(pos, gamma, wing, wing_gamma, targets, variant, near_fp64=(), precision="mixed", max_wake_rows=64):
+    """Velocities of a wing and a wake sheet set (the same column count, even) by one pinned tile."""
+    import uvlm_b200 as U
+
+    num, rows, cols = gamma.shape
+    sim = U.SimpleSimulator(precision=precision, nbody_variant=variant, near_fp64=near_fp64 if precision == "mixed"
+                            else None, max_wake_rows=max(max_wake_rows, rows + 2))
+    for _ in range(num):
+        sim.AddWing(U.RectGenerator(), U.Morphing(), 1.0, 4.0, wing_gamma.shape[1], cols)
+    sim.set_forward_flight([-1.0, 0.0, 0.0])
+    sim.set_advection("euler")
+    sim.begin()
+    sim.set_state(rows, wing, pos, wing_gamma, wing_gamma, gamma)
+    out = sim.Velocity(targets, include_freestream=False)
+    sim.close()
+    return out
+
+
+def _variants():
+    import uvlm_b200 as U
+
+    names = [U.lib().uvlm_nbody_variant_name(i).decode() for i in range(64)]
+    return {name: i for i, name in enumerate(names) if name != "?"}
+
+
+PART_TILES = ["fp32_h2_t2_b128_x2f", "fp32_h3_t2_b128_x2f", "fp32_h4_t2_b128_x2f"]
+
+
+@pytest.mark.parametrize("distance", DISTANCES)
+def test_part_walkers_give_no_fp64_velocity_far_away(distance):
+    """The same by the part walkers, alone and beside points that are near and keep their velocities."""
+    import uvlm_b200 as U
+
+    pos, gamma, near = _lattice()
+    far, limit = _far_points(distance), _far_limit(gamma, distance)
+    got = U.InducedVelocity(far, pos, gamma)
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got)) <= limit
+    mixed = np.empty((128, 3))
+    mixed[0::2], mixed[1::2] = far, near[:64]
+    got = U.InducedVelocity(mixed, pos, gamma)
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got[0::2])) <= limit
+    ref = U.InducedVelocity(near, pos, gamma)[:64]
+    assert np.max(np.abs(got[1::2] - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("tile", PART_TILES)
+@pytest.mark.parametrize("distance", [1e6, 1e12, 1e18, 1e21, 1e30])
+def test_part_walkers_give_no_fp32_velocity_far_away(tile, distance):
+    """The same in FP32, whose squares of distances leave the range from 1e19 on."""
+    pos, gamma, near = _lattice()
+    wing, wing_gamma = pos[:, :2] - [0.31, 0.0, 0.0], np.ones((1, 1, 40))
+    x = np.empty((128, 3))
+    x[0::2], x[1::2] = _far_points(distance), near[:64]
+    got = _velocity(pos, gamma, wing, wing_gamma, x, _variants()[tile])
+    assert np.all(np.isfinite(got)) and np.max(np.abs(got[0::2])) <= _far_limit(gamma, distance)
+
+
+@pytest.mark.parametrize("exponent", [40, 66, 100, 160])
+def test_fp64_sheets_of_any_size(exponent):
+    """A lattice and its points scaled by a power of two (on nodes, near and far; not along the extension of segments,
+    where the oracle itself cancels once its absolute cut-off is out of reach): the oracle's velocities, to 1e-12 of
+    max |v|, where coordinates, their squares and the bounds of a part leave the FP32 range."""
+    import pyoracle as o
+
+    import uvlm_b200 as U
+
+    pos, gamma, t = _lattice()
+    t, s = t[:364], 2.0 ** exponent
+    ref = o.sheet_induced_velocity(pos * s, gamma, t * s)
+    got = U.InducedVelocity(t * s, pos * s, gamma)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("exponent", [-400, 60, 130, 520])
+def test_fp64_strengths_of_any_size(exponent):
+    """Circulations scaled by a power of two: the velocities scaled by it, to 1e-12 of max |v|."""
+    import uvlm_b200 as U
+
+    pos, gamma, t = _lattice()
+    ref = U.InducedVelocity(t, pos, gamma)
+    got = U.InducedVelocity(t, pos, gamma * 2.0 ** exponent) * 2.0 ** -exponent
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("tile", PART_TILES)
+def test_part_walkers_scale_with_the_strengths(tile):
+    """As test_strengths_scale_exactly, by the FP32 part walkers: powers of two scale exactly, and circulations whose
+    squares leave the FP32 range on either side give the same velocities to the rounding of another walker (2e-5 of
+    max |v|)."""
+    pos, gamma, t = _lattice()
+    wing, wing_gamma = _sheet(1, 2, 40, seed=8, wobble=0.0)
+    wing = wing - [0.31, 0.0, 0.0]
+    v = {e: _velocity(pos, gamma * 2.0 ** e, wing, wing_gamma * 2.0 ** e, t, _variants()[tile]) * 2.0 ** -e
+         for e in (0, -20, 10, -60, 75)}
+    for e in (-20, 10):
+        np.testing.assert_array_equal(v[e], v[0])
+    for e in (-60, 75):
+        np.testing.assert_allclose(v[e], v[0], rtol=0, atol=2e-5 * np.max(np.abs(v[0])))

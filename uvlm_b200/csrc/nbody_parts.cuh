@@ -413,14 +413,18 @@ __device__ __forceinline__ void parts_prepare(PartsSmem<T, Rec, h, BLOCK>& sm, i
   }
 }
 
+constexpr float kPartsReach2 = 1e30f;  // square of the distance from which on the near walkers take every pair
+
 // The tests of one part for this warp's targets; ts receives the walker's
 // target coordinates.  Bit 0: far; bit 1: chordwise pairs may be cut; bit 2:
 // spanwise pairs may be cut; bit 3: at least middle; bit 4: strengths that the
 // pairwise cut-off test can square.  Warp-uniform.  longest: the part's longest
 // segment.  The FP32 roundings of
 // the projections stay below 1e-6 (|x - O| + rho), which the test gives away.
-// A part of vanishing strengths (|2 g| < 1e-13 everywhere, where the squares
-// of that test would leave the FP32 range) is left to the near walker.
+// Left to the near walkers, which have no such limits: a part of strengths whose
+// squares would leave the FP32 range (|2 g| < 1e-13 everywhere, or above 1e15),
+// and pairs at or above a distance of 1e15, whose squares and their products do
+// (a part's radius and longest segment are then below that too).
 template <class T, class Rec, int h, int BLOCK, int TPT>
 __device__ __forceinline__ unsigned parts_test(const PartsSmem<T, Rec, h, BLOCK>& sm, int p, int wpp,
                                                const Tgt<T> (&tg)[TPT], typename LaneOf<T>::V (&ts)[TPT][3],
@@ -446,7 +450,7 @@ __device__ __forceinline__ unsigned parts_test(const PartsSmem<T, Rec, h, BLOCK>
   const float aH = 0.999f * __uint_as_float(y.z), aS = 0.999f * __uint_as_float(y.w);
   const float lim2 = 1.000002f * (rho + nb_sqrt(__uint_as_float(l2))) + 1e-3f;
   const float lim = sizeof(T) == 8 ? lim2 : 2.000001f * rho + 1e-3f;
-  const bool strong = gm == 0.f || gm >= 1e-13f;
+  const bool strong = gm == 0.f || (gm >= 1e-13f && gm <= 1e15f);
   bool far = strong, mid = strong, freeH = true, freeS = true;
 #pragma unroll
   for (int q = 0; q < TPT; ++q) {
@@ -457,8 +461,8 @@ __device__ __forceinline__ unsigned parts_test(const PartsSmem<T, Rec, h, BLOCK>
 #pragma unroll
     for (int d = 0; d < 3; ++d) ts[q][d] = v_dup(w[d]);
     const float t2 = dot3(l, l);
-    far = far && t2 >= lim * lim;
-    mid = mid && t2 >= lim2 * lim2;
+    far = far && t2 >= lim * lim && t2 < kPartsReach2;
+    mid = mid && t2 >= lim2 * lim2 && t2 < kPartsReach2;
     const float reach = nb_sqrt(t2) + rho;
     const float tH = nb_sqrt(across2(l, uH, dot3(l, uH))), tS = nb_sqrt(across2(l, uS, dot3(l, uS)));
     freeH = freeH && aH * (tH - pH - 1e-6f * reach) - eH * reach > 1.1e-5f;
@@ -652,7 +656,8 @@ __device__ __forceinline__ bool block_mid(const Slot<typename LaneOf<T>::V>* loc
   for (int q = 0; q < TPT; ++q) {
     const float t[3] = {(float)(v_first(ts[q][0]) + o[0]), (float)(v_first(ts[q][1]) + o[1]),
                         (float)(v_first(ts[q][2]) + o[2])};
-    mid = mid && dot3(t, t) >= lim * lim;
+    const float t2 = dot3(t, t);
+    mid = mid && t2 >= lim * lim && t2 < kPartsReach2;
   }
   return __all_sync(0xffffffffu, mid);
 }
