@@ -242,3 +242,38 @@ def test_part_walkers_scale_with_the_strengths(tile):
         np.testing.assert_array_equal(v[e], v[0])
     for e in (-60, 75):
         np.testing.assert_allclose(v[e], v[0], rtol=0, atol=2e-5 * np.max(np.abs(v[0])))
+
+
+@pytest.mark.parametrize("tile,h", [("fp32_h2_t2_b128_x2f", 2), ("fp32_h3_t2_b128_x2f", 3), ("fp32_h4_t2_b128_x2f", 4)])
+def test_fp32_sums_are_short_on_narrow_sheets(tile, h):
+    """FP32 sums go to FP64 after h node rows of one sheet.  A wake of 8 columns whose spanwise segments all add up the
+    same way over 210 rows at a time, seen from far away, so that the rounding of the sums outweighs that of the terms;
+    all coordinates are multiples of 2^-18 below 32, so that positions relative to any node are exact in FP32.
+
+    Bound: adding the k-th of n = 8 h terms of size t to a sum rounds by at most u k t, uniformly distributed (variance
+    a third of the square), so a sum gathers (u t)^2 n^3 / 9 and all N terms N n^2 / 9; the terms themselves are taken
+    to be off by 4 u each at random.  Twice the root of the sum of both."""
+    import pyoracle as o
+
+    rows, cols, n_t = 2100, 8, 256
+    rng = np.random.default_rng(h)
+    i, j = np.meshgrid(np.arange(rows + 1), np.arange(cols + 1), indexing="ij")
+    pos = np.stack([2.0 ** -17 * i, 0.125 * j, 0.0 * i], -1)[None]
+    up = np.where((np.arange(rows) // 210) % 2 == 0, 1.0, -1.0) * rng.uniform(0.5, 1.5, rows)
+    gamma = np.repeat(np.cumsum(up)[:, None], cols, 1)[None]
+    wing, wing_gamma = pos[:, :2] - [1.0, 0.0, 0.0], np.zeros((1, 1, cols))
+    d = rng.standard_normal((n_t, 3)) * [1.0, 0.3, 1.0]
+    targets = d / np.linalg.norm(d, axis=1)[:, None] * rng.uniform(20, 25, (n_t, 1))
+    targets = np.round(targets * 2.0 ** 18) * 2.0 ** -18
+    ref = o.sheet_induced_velocity(pos, gamma, targets)
+    copies = 141
+    got = _velocity(pos, gamma, wing, wing_gamma, np.tile(targets, (copies, 1)), _variants()[tile],
+                    max_wake_rows=copies * n_t // (cols + 1) + 1)
+    got = got.reshape(copies, n_t, 3)
+    assert np.all(got == got[0])
+    t = 0.125 / (4 * np.pi * np.linalg.norm(targets, axis=1)[:, None] ** 2)
+    rms = np.sqrt(np.mean(np.sum(((got[0] - ref) / t) ** 2, axis=1)))  # in mean terms of one segment
+    u, terms = 2.0 ** -24, rows * cols
+    bound = 2 * u * np.sqrt(terms * ((cols * h) ** 2 / 9 + 16))
+    print(f"{tile}: rms error {rms / u:.0f} u terms, bound {bound / u:.0f}")
+    assert rms <= bound
