@@ -173,3 +173,32 @@ def test_ring_velocities_at_tile_and_split_edges(n, nt, chordwise):
             f = ((r1 - r2)[ok] * (r1[ok] / n1[ok, None] - r2[ok] / n2[ok, None])).sum(1) / d2[ok]
             ref[i] += ((g[ok] * f / (4 * np.pi))[:, None] * d[ok]).sum(0)
     assert np.max(np.abs(got[check] - ref), initial=0) <= 1e-9 * max(np.max(np.abs(ref)), 1)
+
+
+def test_ring_velocities_round_once_per_ring():
+    """A running sum over rings rounds once per ring: 1000 rings whose velocities add up, more targets than one split
+    of the rings needs.  Bound: one rounding of the sum per ring, uniform over a unit in the last place (variance a
+    twelfth of its square), against an 80-bit evaluation; the segments' own roundings are a tenth of that.  1.5 times
+    the root of the sum."""
+    from uvlm_b200 import rings as R
+
+    rng = np.random.default_rng(8)
+    n, nt, L = 1000, 256, np.longdouble
+    base = np.array([[0, 0, 0], [1, 0, 0], [1, 1, 0], [0, 1, 0]], float)
+    r = base + 0.05 * rng.standard_normal((n, 4, 3))
+    g = rng.uniform(0.5, 1.5, n)
+    x = np.array([0.5, 0.5, 0.0]) + rng.uniform(-0.8, 0.8, (nt, 3)) + np.array([0, 0, 2.5]) * rng.choice([-1, 1], (nt, 1))
+    got = R.InducedVelocity(np.tile(x, (600, 1)), r, g).reshape(600, nt, 3)
+    assert np.all(got == got[0])
+    run, var = np.zeros((nt, 3), L), np.zeros((nt, 3))
+    pi = L("3.14159265358979323846264338327950288")
+    for k in range(n):
+        p = r[k].astype(L)
+        for s in range(4):  # nodes[s + 1] -> nodes[s]
+            r1, r2 = x.astype(L) - p[(s + 1) % 4], x.astype(L) - p[s]
+            n1, n2 = np.sqrt((r1 * r1).sum(1)), np.sqrt((r2 * r2).sum(1))
+            f = (n1 + n2) / (n1 * n2 * (n1 * n2 + (r1 * r2).sum(1)))
+            run += (g[k] * f / (4 * pi))[:, None] * np.cross(r1, r2)
+        var += np.spacing(np.abs(run).astype(float)) ** 2 / 12
+    rms = float(np.sqrt(np.mean((got[0] - run) ** 2)))
+    assert rms <= 1.5 * np.sqrt(np.mean(var))

@@ -1379,6 +1379,9 @@ Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
 // sheets through the strip walkers there was a far-field test for every four
 // nodes: a wake advection call with 1088 rings and 3840 targets took 267 us
 // (with records, layouts and partial sums in kernels of their own), now 162.
+// A ring's segments are summed on their own: they nearly cancel, and added to
+// the sum one by one, each rounds at the sum's magnitude (error against 80-bit
+// arithmetic, 1000 rings: 1.7e-15, 7.7e-16 now).
 namespace {
 constexpr int kRingThreads = 128, kRingTile = 32;
 
@@ -1423,10 +1426,14 @@ __global__ void __launch_bounds__(kRingThreads, 4)
         n[k].n = q >= kCutR2 ? q * nb_rsqrt(q) : 0.0;
       }
       const double g = rec.g;
+      double rx = 0, ry = 0, rz = 0;
 #pragma unroll
       for (int k = 0; k < 4; k += CHORDWISE ? 2 : 1)
-        seg<double>(SegV<double>{rec.r0[3 * k], rec.r0[3 * k + 1], rec.r0[3 * k + 2]}, n[k], n[(k + 1) & 3], g, vx, vy,
-                    vz);
+        seg<double>(SegV<double>{rec.r0[3 * k], rec.r0[3 * k + 1], rec.r0[3 * k + 2]}, n[k], n[(k + 1) & 3], g, rx, ry,
+                    rz);
+      vx += rx;
+      vy += ry;
+      vz += rz;
     }
   }
   if (t < nt) {
