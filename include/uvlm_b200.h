@@ -254,6 +254,16 @@ int uvlm_measure_fp32_peak(int32_t device, double* tflops);
 /* Measured FP64 FMA throughput (TFLOP/s): the denominator of the plain FP64
  * form's N-body roofline. */
 int uvlm_measure_fp64_peak(int32_t device, double* tflops);
+/* The arithmetic that the kernels form in steps of their own, for checks of its
+ * accuracy: out[k] (host arrays) of x[k], and of y[k] for the quotients.  No
+ * counterpart in the reference. */
+enum {
+  UVLM_ARITH_RSQRT = 0,        /* 1 / sqrt(x), FP64 N-body */
+  UVLM_ARITH_RECIPROCAL = 1,   /* 1 / x, FP64 N-body */
+  UVLM_ARITH_QUOTIENT = 2,     /* x / y, FP64 LU */
+  UVLM_ARITH_QUOTIENT_F32 = 3  /* x / y rounded to FP32, FP32 LU */
+};
+int uvlm_check_arithmetic(int32_t kind, const double* x, const double* y, int64_t n, double* out);
 /* Every bounded device-side wait of the library (the triangular solves'
  * block-row flags, the cooperative grid barrier, the tensor-core kernels'
  * mbarriers) gives up after `cycles` SM clock cycles on `device` (0 restores

@@ -480,8 +480,10 @@ __device__ __forceinline__ double tsp_rcp(double x) {
   return fabs(r) < 0x1p+900 && fabs(r) > 0x1p-900 ? r : 0.0;
 }
 
-// x / piv from r = tsp_rcp(piv): a product and one correction by its residual,
-// or a division where r is 0; 0 for a zero pivot.
+// x / piv from r = tsp_rcp(piv): a product and one correction by its residual
+// (P. W. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990), which rounds as the division does with a
+// correctly rounded r; or a division where r is 0; 0 for a zero pivot.
 template <class T>
 __device__ __forceinline__ T tsp_quotient(T x, T piv, T r) {
   const T q = x * r;
@@ -1730,6 +1732,26 @@ Error gemm_update_f32_simt(float* C, int ldc, const float* A, int lda, const flo
   if (m <= 0 || nc <= 0 || k <= 0) return ok();
   dim3 grid(ceil_div(nc, 64), ceil_div(m, 64));
   gemm_update_kernel<float><<<grid, 256, 0, st>>>(C, ldc, A, lda, B, ldb, m, nc, k);
+  UVLM_LAUNCH_CHECK();
+  return ok();
+}
+
+namespace {
+template <class T>
+__global__ void quotient_kernel(const double* __restrict__ x, const double* __restrict__ y, long long n,
+                                double* __restrict__ out) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+    out[k] = (double)tsp_quotient<T>((T)x[k], (T)y[k], tsp_rcp((T)y[k]));
+}
+}  // namespace
+
+Error lu_quotients(bool f32, const double* x, const double* y, long long n, double* out, cudaStream_t st) {
+  if (n <= 0) return ok();
+  const unsigned grid = (unsigned)std::min<long long>((n + 255) / 256, 4096);
+  if (f32)
+    quotient_kernel<float><<<grid, 256, 0, st>>>(x, y, n, out);
+  else
+    quotient_kernel<double><<<grid, 256, 0, st>>>(x, y, n, out);
   UVLM_LAUNCH_CHECK();
   return ok();
 }

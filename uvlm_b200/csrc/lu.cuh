@@ -103,6 +103,9 @@ Error gemm_update_f32_simt(float* C, int ldc, const float* A, int lda, const flo
 Error gemm_update_tc(float* C, int ldc, const float* A, int lda, const float* Bt, int ldbt, int m, int nc, int k,
                      LuUpdate kind, LuWork* w, cudaStream_t st);
 bool gemm_tc_available();
+// out[k] = x[k] / y[k] as the eliminations form it (FP64, or both rounded to
+// FP32); device arrays.
+Error lu_quotients(bool f32, const double* x, const double* y, long long n, double* out, cudaStream_t st);
 // The bounded-wait limit of this unit's kernels (0 = default), and a check
 // that a wait on a flag nothing sets gives up after `cycles` (restores the
 // default limit afterwards).

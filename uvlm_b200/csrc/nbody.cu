@@ -85,10 +85,13 @@ __device__ __forceinline__ float nb_rcp(float x) {
 }
 
 // FP64 1/sqrt(x) and 1/x from the hardware's approximations (PTX rsqrt.approx
-// / rcp.approx .ftz.f64, relative error about 2^-20) by one step of third
-// order each: with e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 +
-// 3 e^2/8 + O(e^3)); with e = 1 - x y, 1/x = y (1 + e + e^2 + O(e^3)).  The
-// remainder is below 2^-56.  Five and three FP64 operations, without the
+// / rcp.approx .ftz.f64, relative error about 2^-20) by one step of a
+// third-order (Householder) iteration each, the series of the exact correction
+// cut after its second term: with e = 1 - x y^2, 1/sqrt(x) = y (1 - e)^(-1/2) =
+// y (1 + e/2 + 3 e^2/8 + O(e^3)); with e = 1 - x y, 1/x = y (1 + e + e^2 +
+// O(e^3)).  Measured over 4 million arguments of all exponents against 80-bit
+// arithmetic: 1/sqrt(x) below 0.993 ulp, 0.331 rms; 1/x below 0.507, 0.289 rms.
+// Five and three FP64 operations, without the
 // special cases of the library functions: the arguments are squared distances
 // and denominators that the callers' cuts keep away from 0 (what a zero gives
 // is dropped by a select), and what an infinite one gives (a NaN) is dropped too.
@@ -1054,6 +1057,20 @@ Error nbody_batch_eval(NBodyPrec prec, const NBodyBatchInput* d_in, int n, const
     case 2: return run(batch_eval<float, RecF, kBatchTileH[2], kBatchTptF>, grids.tiles[2]);
     default: return run(batch_eval<float, RecF, kBatchTileH[0], kBatchTptF>, grids.tiles[0]);
   }
+}
+
+namespace {
+__global__ void arithmetic_kernel(bool recip, const double* __restrict__ x, long long n, double* __restrict__ out) {
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+    out[k] = recip ? nb_rcp(x[k]) : nb_rsqrt(x[k]);
+}
+}  // namespace
+
+Error nbody_arithmetic(bool recip, const double* x, long long n, double* out, cudaStream_t st) {
+  if (n <= 0) return ok();
+  arithmetic_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 4096), 256, 0, st>>>(recip, x, n, out);
+  UVLM_LAUNCH_CHECK();
+  return ok();
 }
 
 // ------------------------------------------------------ arbitrary points

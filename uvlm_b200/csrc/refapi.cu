@@ -412,6 +412,27 @@ int uvlm_lu_factor_f32(const float* A, int64_t n, int32_t update, float* LU, int
   return report(run());
 }
 
+int uvlm_check_arithmetic(int32_t kind, const double* x, const double* y, int64_t n, double* out) {
+  const bool quotient = kind == UVLM_ARITH_QUOTIENT || kind == UVLM_ARITH_QUOTIENT_F32;
+  if (kind < UVLM_ARITH_RSQRT || kind > UVLM_ARITH_QUOTIENT_F32 || n < 0 || (n && (!x || !out || (quotient && !y))))
+    return report(fail(kErrInvalid, "invalid argument"));
+  if (n == 0) return UVLM_OK;
+  Scratch S;
+  auto run = [&]() -> Error {
+    double *dx, *dy = nullptr, *dout;
+    UVLM_TRY(S.up(&dx, x, (size_t)n));
+    if (quotient) UVLM_TRY(S.up(&dy, y, (size_t)n));
+    UVLM_TRY(S.get(&dout, (size_t)n));
+    if (quotient)
+      UVLM_TRY(lu_quotients(kind == UVLM_ARITH_QUOTIENT_F32, dx, dy, n, dout, 0));
+    else
+      UVLM_TRY(nbody_arithmetic(kind == UVLM_ARITH_RECIPROCAL, dx, n, dout, 0));
+    UVLM_CUDA_TRY(cudaMemcpy(out, dout, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    return ok();
+  };
+  return report(run());
+}
+
 int uvlm_dense_solve(const double* A, int64_t n, const double* b, double* x, int32_t method, int32_t* iters) {
   if (!A || !b || !x || n < 1 || method < 0 || method > 2) return report(fail(kErrInvalid, "invalid argument"));
   Scratch S;
