@@ -53,3 +53,32 @@ def test_threads_share_the_workspace_and_it_is_given_back():
         np.testing.assert_array_equal(a, b)
     with pytest.raises(U.UVLMError):
         U.release_workspace(63)
+
+
+def _free_bytes():
+    import torch
+
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def test_memory_kept_after_a_large_call_is_bounded_and_given_back():
+    """A call that takes over 1 GB keeps at most 256 MiB when it returns, also after several such calls at once, and
+    nothing after release_workspace (each to 32 MiB, the driver's own granularity)."""
+    import uvlm_b200 as U
+
+    pos, gamma, _ = _case(0)
+    t = np.random.default_rng(1).uniform(5, 9, (3_000_000, 3))
+    U.InducedVelocity(t[:1000], pos, gamma)  # the kernels are loaded
+    U.release_workspace()
+    before, slack = _free_bytes(), 32 << 20
+    U.InducedVelocity(t, pos, gamma)
+    assert before - _free_bytes() <= (256 << 20) + slack
+    threads = [threading.Thread(target=lambda: U.InducedVelocity(t[:1_000_000], pos, gamma)) for _ in range(4)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert before - _free_bytes() <= (256 << 20) + slack
+    U.InducedVelocity(t[:100_000], pos, gamma)
+    U.release_workspace()
+    assert before - _free_bytes() <= slack

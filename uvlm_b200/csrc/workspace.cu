@@ -9,8 +9,10 @@
 // freed by one call is handed to the next one, of any thread, in the order of
 // that stream.  The pool is the library's own (the device's default pool, which
 // the host program may use, is not touched).  It keeps at most
-// kKeptWorkspaceBytes between calls, what exceeds that goes back to the device
-// at the next synchronisation, and uvlm_release_workspace gives all of it back.
+// kKeptWorkspaceBytes between calls: a call that ends with more reserved waits
+// for the stream and trims the pool (a release threshold alone takes effect at
+// the program's next synchronisation, whenever that is; 2.0 GB stayed after 3
+// million points), and uvlm_release_workspace gives all of it back.
 #include <cuda.h>
 
 #include <mutex>
@@ -102,6 +104,25 @@ Error workspace_alloc(void** p, size_t bytes) {
 
 void workspace_free(void* p) {
   if (p) cudaFreeAsync(p, nullptr);
+}
+
+void workspace_settle() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return;
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    pool = g_pool[dev];
+  }
+  unsigned long long reserved = 0;
+  if (!pool) return;
+  if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  // of several calls at once, the last to end sees what all of them reserved
+  if (reserved > kKeptWorkspaceBytes && cudaStreamSynchronize(nullptr) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, kKeptWorkspaceBytes);
 }
 
 }  // namespace uvlm

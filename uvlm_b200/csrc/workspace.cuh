@@ -10,6 +10,8 @@ namespace uvlm {
 // Stream-ordered on the legacy default stream of the current device.
 Error workspace_alloc(void** p, size_t bytes);
 void workspace_free(void* p);
+// After a call's last workspace_free: gives back what is kept beyond the bound.
+void workspace_settle();
 // Unique id of the context current on this thread (0 if the driver entry
 // points are unavailable).  A cudaDeviceReset destroys the primary context and
 // what belongs to it; the next primary context has another id.
@@ -25,6 +27,7 @@ struct Scratch {
   Scratch& operator=(const Scratch&) = delete;
   ~Scratch() {
     for (void* q : p) workspace_free(q);
+    if (!p.empty()) workspace_settle();
   }
   Error bytes(void** out, size_t count) {
     constexpr size_t kSlab = 1u << 20;
