@@ -82,3 +82,64 @@ def test_memory_kept_after_a_large_call_is_bounded_and_given_back():
     U.InducedVelocity(t[:100_000], pos, gamma)
     U.release_workspace()
     assert before - _free_bytes() <= slack
+
+
+_DRIVER_CONTEXT = """
+import ctypes as C, sys
+import numpy as np
+cuda = C.CDLL("libcuda.so.1")
+ctx, now, dev, flags, active = C.c_void_p(), C.c_void_p(), C.c_int(), C.c_uint(), C.c_int()
+assert cuda.cuInit(0) == 0 and cuda.cuDeviceGet(C.byref(dev), 0) == 0
+assert cuda.cuCtxCreate_v2(C.byref(ctx), 0, dev) == 0
+sys.path[:0] = sys.argv[2:]
+import test_gpu_workspace as T
+import uvlm_b200 as U
+out = []
+for call in T.CALLS:
+    out.append(np.asarray(call()))
+    assert cuda.cuCtxGetCurrent(C.byref(now)) == 0 and now.value == ctx.value, "another context is current"
+U.release_workspace()
+assert cuda.cuCtxGetCurrent(C.byref(now)) == 0 and now.value == ctx.value, "another context is current"
+assert cuda.cuDevicePrimaryCtxGetState(dev, C.byref(flags), C.byref(active)) == 0 and not active.value
+np.savez(sys.argv[1], *out)
+"""
+
+
+def _gradients():
+    from uvlm_b200.warmstart import MLP
+
+    rng = np.random.default_rng(3)
+    net = MLP(seed=1)
+    return net.gradients(rng.standard_normal((100, 8)).astype(np.float32), rng.standard_normal(100).astype(np.float32))[0]
+
+
+def _call(f):
+    def run():
+        import uvlm_b200 as U
+
+        return f(U)
+
+    return run
+
+
+CALLS = [_call(lambda U: U.InducedVelocity(_case(2)[2], *_case(2)[:2])),
+         _call(lambda U: U.InducedVelocity(_case(2)[2], *_case(2)[:2], precision="mixed")),
+         _call(lambda U: U.dense_solve(np.eye(70) * 3 + np.ones((70, 70)) * 0.1, np.arange(70.0))[0]),
+         _gradients]
+
+
+def test_calls_stay_in_the_callers_context(tmp_path):
+    """A program that works in a driver context of its own: the calls give the same results there, leave it current, and
+    bring up no other context (arrays of one context cannot be read from another)."""
+    import os
+    import subprocess
+    import sys
+
+    here = os.path.dirname(os.path.abspath(__file__))
+    path = str(tmp_path / "out.npz")
+    p = subprocess.run([sys.executable, "-c", _DRIVER_CONTEXT, path, os.path.dirname(here), here], capture_output=True,
+                       text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    with np.load(path) as got:
+        for name, call in zip(got.files, CALLS):
+            np.testing.assert_array_equal(got[name], call())

@@ -12,7 +12,8 @@
 // kKeptWorkspaceBytes between calls: a call that ends with more reserved waits
 // for the stream and trims the pool (a release threshold alone takes effect at
 // the program's next synchronisation, whenever that is; 2.0 GB stayed after 3
-// million points), and uvlm_release_workspace gives all of it back.
+// million points), and uvlm_release_workspace gives all of it back.  A thread that
+// works in a driver context of its own takes its arrays from that context instead.
 #include <cuda.h>
 
 #include <mutex>
@@ -27,13 +28,45 @@ namespace {
 // The 4096 x 4096 dense solve (134 MB of matrix, 67 MB of FP32 factors) fits.
 constexpr unsigned long long kKeptWorkspaceBytes = 256ull << 20;
 
+// The driver's context calls (NULL where there is no driver).
+struct Driver {
+  CUresult (*get_current)(CUcontext*) = nullptr;
+  CUresult (*set_current)(CUcontext) = nullptr;
+  CUresult (*get_id)(CUcontext, unsigned long long*) = nullptr;
+  CUresult (*device_get)(CUdevice*, int) = nullptr;
+  CUresult (*primary_state)(CUdevice, unsigned*, int*) = nullptr;
+  CUresult (*primary_retain)(CUcontext*, CUdevice) = nullptr;
+  CUresult (*primary_release)(CUdevice) = nullptr;
+  Driver() {
+    find("cuCtxGetCurrent", get_current);
+    find("cuCtxSetCurrent", set_current);
+    find("cuCtxGetId", get_id);
+    find("cuDeviceGet", device_get);
+    find("cuDevicePrimaryCtxGetState", primary_state);
+    find("cuDevicePrimaryCtxRetain", primary_retain);
+    find("cuDevicePrimaryCtxRelease", primary_release);
+  }
+  template <class F>
+  static void find(const char* name, F& f) {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &fn, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+      f = reinterpret_cast<F>(fn);
+    else
+      cudaGetLastError();
+  }
+};
+const Driver& driver() {
+  static const Driver d;
+  return d;
+}
+
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 unsigned long long g_pool_ctx[kMaxDevices] = {};  // context the pool belongs to
 
 Error pool_of(int dev, cudaMemPool_t* out) {
   if (dev < 0 || dev >= kMaxDevices) return fail(kErrUnsupported, "device ordinal out of range");
-  UVLM_CUDA_TRY(cudaSetDevice(dev));  // makes the primary context current, also after a reset
   const unsigned long long ctx = current_context_id();
   std::lock_guard<std::mutex> lk(g_pool_mu);
   if (!g_pool[dev] || g_pool_ctx[dev] != ctx) {
@@ -59,29 +92,41 @@ Error pool_of(int dev, cudaMemPool_t* out) {
 }  // namespace
 
 unsigned long long current_context_id() {
-  using GetCurrent = CUresult (*)(CUcontext*);
-  using GetId = CUresult (*)(CUcontext, unsigned long long*);
-  static GetCurrent get_current = nullptr;
-  static GetId get_id = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_current = reinterpret_cast<GetCurrent>(fn);
-    if (cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      get_id = reinterpret_cast<GetId>(fn);
-  });
+  const Driver& d = driver();
   CUcontext ctx = nullptr;
   unsigned long long id = 0;
-  if (get_current && get_id && get_current(&ctx) == CUDA_SUCCESS && ctx) get_id(ctx, &id);
+  if (d.get_current && d.get_id && d.get_current(&ctx) == CUDA_SUCCESS && ctx) d.get_id(ctx, &id);
   return id;
 }
 
-Error workspace_alloc(void** p, size_t bytes) {
+bool workspace_in_primary_context() {
+  const Driver& d = driver();
+  int dev = 0;
+  if (!d.get_current || !d.device_get || !d.primary_state || !d.primary_retain || !d.primary_release ||
+      cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  CUcontext now = nullptr, primary = nullptr;
+  if (d.get_current(&now) != CUDA_SUCCESS) now = nullptr;
+  if (!now) return cudaSetDevice(dev) == cudaSuccess;
+  // the state first: retaining would bring up a context that the program does without
+  unsigned flags = 0;
+  int active = 0;
+  CUdevice device = 0;
+  if (d.device_get(&device, dev) != CUDA_SUCCESS || d.primary_state(device, &flags, &active) != CUDA_SUCCESS ||
+      !active || d.primary_retain(&primary, device) != CUDA_SUCCESS)
+    return false;
+  d.primary_release(device);
+  return primary == now;
+}
+
+Error workspace_alloc(void** p, size_t bytes, bool pooled) {
   *p = nullptr;
+  if (!pooled) {
+    UVLM_CUDA_TRY(cudaMalloc(p, bytes));
+    return ok();
+  }
   int dev = 0;
   UVLM_CUDA_TRY(cudaGetDevice(&dev));
   cudaMemPool_t pool = nullptr;
@@ -102,8 +147,12 @@ Error workspace_alloc(void** p, size_t bytes) {
   return ok();
 }
 
-void workspace_free(void* p) {
-  if (p) cudaFreeAsync(p, nullptr);
+void workspace_free(void* p, bool pooled) {
+  if (!p) return;
+  if (pooled)
+    cudaFreeAsync(p, nullptr);
+  else
+    cudaFree(p);
 }
 
 void workspace_settle() {
@@ -130,18 +179,31 @@ void workspace_settle() {
 extern "C" int uvlm_release_workspace(int32_t device) {
   using namespace uvlm;
   auto run = [&]() -> Error {
-    int ndev = 0, before = 0;
+    int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
       cudaGetLastError();
       return fail(kErrCuda, "no CUDA device");
     }
     if (device < 0 || device >= ndev || device >= kMaxDevices) return fail(kErrInvalid, "no such device");
-    cudaMemPool_t pool = nullptr;
+    // in the device's primary context; the caller's own is current again afterwards
+    const Driver& d = driver();
+    int before = 0;
+    CUcontext ctx = nullptr;
     UVLM_CUDA_TRY(cudaGetDevice(&before));
+    if (d.get_current) d.get_current(&ctx);
+    {
+      std::lock_guard<std::mutex> lk(g_pool_mu);
+      if (!g_pool[device]) return ok();  // nothing was ever kept
+    }
+    UVLM_CUDA_TRY(cudaSetDevice(device));
+    cudaMemPool_t pool = nullptr;
     Error e = pool_of(device, &pool);
     if (!e.code && (cudaStreamSynchronize(nullptr) != cudaSuccess || cudaMemPoolTrimTo(pool, 0) != cudaSuccess))
       e = fail(kErrCuda, "the workspace could not be released");
-    cudaSetDevice(before);
+    if (ctx && d.set_current)
+      d.set_current(ctx);
+    else
+      cudaSetDevice(before);
     return e;
   };
   const Error e = run();

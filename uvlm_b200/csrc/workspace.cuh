@@ -7,9 +7,14 @@
 
 namespace uvlm {
 
-// Stream-ordered on the legacy default stream of the current device.
-Error workspace_alloc(void** p, size_t bytes);
-void workspace_free(void* p);
+// Whether the calling thread works in its device's primary context (made current
+// if there is none), where the pool lives.  A program may have a context of its
+// own current instead: its calls stay in it and allocate there.
+bool workspace_in_primary_context();
+// pooled: from the pool, stream-ordered on the legacy default stream of the
+// current device; else from the current context.
+Error workspace_alloc(void** p, size_t bytes, bool pooled);
+void workspace_free(void* p, bool pooled);
 // After a call's last workspace_free: gives back what is kept beyond the bound.
 void workspace_settle();
 // Unique id of the context current on this thread (0 if the driver entry
@@ -19,6 +24,7 @@ unsigned long long current_context_id();
 
 // Device buffers of one call, freed at scope exit.  Small ones share slabs.
 struct Scratch {
+  const bool pooled = workspace_in_primary_context();
   std::vector<void*> p;
   char* slab = nullptr;
   size_t left = 0;
@@ -26,8 +32,8 @@ struct Scratch {
   Scratch(const Scratch&) = delete;
   Scratch& operator=(const Scratch&) = delete;
   ~Scratch() {
-    for (void* q : p) workspace_free(q);
-    if (!p.empty()) workspace_settle();
+    for (void* q : p) workspace_free(q, pooled);
+    if (pooled && !p.empty()) workspace_settle();
   }
   Error bytes(void** out, size_t count) {
     constexpr size_t kSlab = 1u << 20;
@@ -38,7 +44,7 @@ struct Scratch {
     if (need <= kSlab / 2) {
       if (need > left) {
         void* s = nullptr;
-        UVLM_TRY(workspace_alloc(&s, kSlab));
+        UVLM_TRY(workspace_alloc(&s, kSlab, pooled));
         p.push_back(s);
         slab = static_cast<char*>(s);
         left = kSlab;
@@ -48,7 +54,7 @@ struct Scratch {
       left -= need;
       return ok();
     }
-    UVLM_TRY(workspace_alloc(out, need));
+    UVLM_TRY(workspace_alloc(out, need, pooled));
     p.push_back(*out);
     return ok();
   }
