@@ -295,3 +295,34 @@ def test_solve_clusters_of_every_size_give_the_same_loads(n):
 
     one, many = loads(1), loads(n)
     assert np.max(np.abs(many - one)) <= 1e-6 * np.max(np.abs(one))
+
+
+def _small_batch(rows, cols, n, precision="mixed", use_graph=True, steps=3, tile=0):
+    import uvlm_b200 as U
+    from uvlm_b200.batch import BatchSimulator
+
+    sim = BatchSimulator(precision=precision, max_steps=steps, use_graph=use_graph,
+                         nbody_tile=tile if precision == "mixed" else -1)
+    m = U.Morphing().set_alpha(0.05).set_plug(0.1, 1.0).set_twist(0.1, 1.0, math.pi / 2)
+    for _ in range(n):
+        sim.add_case(m, 1.0, 4.0, rows, cols, 0.15)
+    return sim
+
+
+@pytest.mark.parametrize("use_graph", [True, False])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_batches_of_different_sizes_live_at_once(precision, use_graph):
+    """A batch of large cases runs after one of small cases was created: its loads are those it has alone."""
+    alone = _small_batch(16, 64, 2, precision, use_graph)
+    alone.run(3)
+    want = alone.loads()
+    alone.close()
+    large, small = _small_batch(16, 64, 2, precision, use_graph), _small_batch(4, 8, 2, precision, use_graph)
+    large.begin()
+    small.begin()
+    small.run(1)
+    large.run(3)
+    got = large.loads()
+    large.close()
+    small.close()
+    np.testing.assert_array_equal(got, want)

@@ -33,6 +33,7 @@
 
 #include "../../include/uvlm_b200.h"
 #include "bs_math.cuh"
+#include "device_once.h"
 #include "host_lattice.h"
 #include "nbody.cuh"
 #include "step_math.cuh"
@@ -303,6 +304,7 @@ struct SolveCfg {
   static constexpr int NB = sizeof(T) == 4 ? 32 : 16;
 };
 constexpr int kSolveBlock = 32;  // diagonal block of the triangular solves
+constexpr int kMaxCaseRings = 1024;
 
 // Leading dimension of the column-major panel: 16-byte aligned columns with room
 // for the rows that an update tile reads past the last one.
@@ -1096,6 +1098,25 @@ __global__ void b_step_end_kernel(long long* d_step) {
 
 using namespace uvlm;
 
+namespace {
+// Shared memory of the solve up to the largest case, once per device: the limit
+// belongs to the kernel, so one that followed each batch's own size would be
+// lowered under a live batch of larger cases.
+template <class T>
+Error allow_solve_smem(int device) {
+  static PerDeviceOnce once;
+  cudaError_t e = cudaSuccess;
+  if (!once_on_device(once, device, [&] {
+        e = cudaFuncSetAttribute(b_solve_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)solve_smem_bytes<T>(kMaxCaseRings));
+        return e == cudaSuccess;
+      }))
+    return fail(kErrCuda, std::string("batch: the solve's shared memory could not be set on this device: ") +
+                              cudaGetErrorString(e));
+  return ok();
+}
+}  // namespace
+
 struct uvlm_batch {
   uvlm_batch_config cfg{};
   std::string err;
@@ -1356,12 +1377,7 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   UVLM_CUDA_TRY(cudaMemset(d_has_factor, 0, sizeof(int) * n));
   UVLM_CUDA_TRY(cudaMemset(d_refac, 0, sizeof(unsigned long long)));
   UVLM_CUDA_TRY(cudaMemset(d_loads, 0, sizeof(double) * (size_t)cfg.max_steps * n * 3));
-  if (mixed())
-    UVLM_CUDA_TRY(cudaFuncSetAttribute(b_solve_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)solve_smem_bytes<float>(max_N)));
-  else
-    UVLM_CUDA_TRY(cudaFuncSetAttribute(b_solve_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)solve_smem_bytes<double>(max_N)));
+  UVLM_TRY(mixed() ? allow_solve_smem<float>(cfg.device) : allow_solve_smem<double>(cfg.device));
   if (mixed()) {
     // as many CTAs per case as run all cases at once
     for (solve_ctas = kSolveCluster; solve_ctas > 1; --solve_ctas) {
@@ -1566,7 +1582,7 @@ int uvlm_batch_create(const uvlm_batch_config* cfg, const uvlm_batch_case* cases
   }
   for (int c = 0; c < n_cases; ++c) {
     const uvlm_batch_case& u = cases[c];
-    if (u.rows < 1 || u.cols < 2 || (u.cols & 1) || u.rows > 64 || u.cols > 64 || u.rows * u.cols > 1024 ||
+    if (u.rows < 1 || u.cols < 2 || (u.cols & 1) || u.rows > 64 || u.cols > 64 || u.rows * u.cols > kMaxCaseRings ||
         !(u.chord > 0) ||
         !(u.span > 0) || !(u.dt > 0)) {
       set_global_error("uvlm_batch_create: every case needs 1 <= rows <= 64, even 2 <= cols <= 64, "
