@@ -202,3 +202,58 @@ def test_ring_velocities_round_once_per_ring():
         var += np.spacing(np.abs(run).astype(float)) ** 2 / 12
     rms = float(np.sqrt(np.mean((got[0] - run) ** 2)))
     assert rms <= 1.5 * np.sqrt(np.mean(var))
+
+
+def test_simulators_do_not_see_a_busy_default_stream():
+    """Batches and simulators run on streams of their own; their first arrays are there before the first step although
+    another thread keeps the default stream, which fills them, busy."""
+    import threading
+
+    import torch
+
+    import uvlm_b200 as U
+    from uvlm_b200.batch import BatchSimulator
+
+    def batch(precision, graph):
+        sim = BatchSimulator(precision=precision, max_steps=4, use_graph=graph,
+                             nbody_tile=0 if precision == "mixed" else -1)
+        for _ in range(3):
+            sim.add_case(U.Morphing().set_alpha(0.05).set_plug(0.1, 1.0), 1.0, 4.0, 4, 8, 0.15)
+        sim.run(4)
+        out = sim.loads()
+        sim.close()
+        return out
+
+    def simulator(precision):
+        sim = U.SimpleSimulator(precision=precision)
+        sim.AddWing(U.RectGenerator(), U.Morphing().set_alpha(0.05).set_plug(0.1, 1.0), 1.0, 4.0, 4, 8)
+        sim.set_forward_flight([-1.0, 0.0, 0.0])
+        sim.set_advection("euler")
+        out = sim.Run(3, 0.15)
+        gamma = sim.state()["wing_gamma"]
+        sim.close()
+        return np.concatenate([out.ravel(), gamma.ravel()])
+
+    calls = [lambda p=p, g=g: batch(p, g) for p in ("fp64", "mixed") for g in (True, False)]
+    calls += [lambda p=p: simulator(p) for p in ("fp64", "mixed")]
+    want = [call() for call in calls]
+    stop = threading.Event()
+
+    def busy():
+        done = [torch.cuda.Event() for _ in range(4)]
+        k = 0
+        while not stop.is_set():
+            done[k % 4].synchronize()  # four sleeps of about 20 ms queued at a time
+            torch.cuda._sleep(40_000_000)
+            done[k % 4].record()
+            k += 1
+
+    th = threading.Thread(target=busy)
+    th.start()
+    try:
+        got = [call() for _ in range(2) for call in calls]
+    finally:
+        stop.set()
+        th.join()
+    for a, b in zip(got, want + want):
+        np.testing.assert_array_equal(a, b)

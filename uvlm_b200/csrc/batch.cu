@@ -1392,6 +1392,8 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   }
   nb_grids = nbody_batch_grids(prec(), num_sms);
   grid = num_sms * 8;
+  // the copies and fills above are the default stream's, the steps `st`'s
+  UVLM_CUDA_TRY(cudaStreamSynchronize(nullptr));
   return ok();
 }
 

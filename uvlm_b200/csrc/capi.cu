@@ -1004,7 +1004,8 @@ int uvlm_begin(uvlm_ctx* c) {
           cudaSuccess ||
       cudaMemset(c->d_gamma, 0, sizeof(double) * c->N) != cudaSuccess ||
       cudaMemset(c->d_gamma_prev, 0, sizeof(double) * c->N) != cudaSuccess ||
-      cudaMemset(c->d_row, 0, sizeof(double) * (1 + 2 * c->num)) != cudaSuccess)
+      cudaMemset(c->d_row, 0, sizeof(double) * (1 + 2 * c->num)) != cudaSuccess ||
+      cudaStreamSynchronize(nullptr) != cudaSuccess)  // the steps run on a stream of their own
     return c->fail_with(fail(kErrCuda, "initial upload failed"));
   c->wake_start = c->PR;
   c->wake_nodes = 0;
@@ -1132,6 +1133,7 @@ int uvlm_set_state(uvlm_ctx* c, int64_t wake_rows, const double* wing_pos, const
       up(c->d_wgamma + ((size_t)n * c->PR + c->wake_start) * c->C, wake_gamma + (size_t)n * wake_rows * c->C,
          (size_t)wake_rows * c->C);
   }
+  if (!e.code && cudaStreamSynchronize(nullptr) != cudaSuccess) e = fail(kErrCuda, "state upload failed");
   c->has_vprev = false;
   c->have_factors = false;
   return c->fail_with(e);
