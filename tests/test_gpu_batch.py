@@ -326,3 +326,47 @@ def test_batches_of_different_sizes_live_at_once(precision, use_graph):
     large.close()
     small.close()
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cols", [2, 36, 64])
+def test_memory_of_a_long_batch(precision, cols):
+    """The partial sums of a batch take 1 GiB, or one set per 16 wake rows and 64 columns (at least 8 sets per case):
+    what a batch of 24 cases and 1000 steps takes on the device beside its other arrays."""
+    import torch
+
+    _small_batch(4, cols, 1, precision, steps=4).close()
+    sim = _small_batch(4, cols, 24, precision, steps=1000)
+    before = torch.cuda.mem_get_info(0)[0]
+    sim.begin()
+    used = before - torch.cuda.mem_get_info(0)[0]
+    sim.run(2)
+    sim.close()
+    nodes = 24 * 1002 * (cols + 1)
+    sets = max(8, math.ceil(1002 / 16) + 1)
+    # per node: positions, circulation, record, targets and velocities, one set of partial sums each
+    other = nodes * (24 + 8 + 96 + 24 + 24)
+    assert used <= max(1 << 30, nodes * 24 * sets) + other + (16 << 20)
+
+
+@pytest.mark.parametrize("precision,cols,steps,longest", [("fp64", 64, 56, 1000), ("fp64", 34, 80, 1000),
+                                                          ("mixed", 64, 105, 1300)])
+def test_long_batches_whose_items_take_more_than_three_strips(precision, cols, steps, longest):
+    """Batches made for wakes so long that their partial sums are bounded, once their wakes pass 24 strips, against a
+    single-case FP64 simulator, to the batch tolerances."""
+    import uvlm_b200 as U
+
+    sim = _small_batch(1, cols, 40, precision, steps=longest, tile=1)
+    sim.run(steps)
+    rows = sim.loads()
+    sim.close()
+    one = U.SimpleSimulator()
+    m = U.Morphing().set_alpha(0.05).set_plug(0.1, 1.0).set_twist(0.1, 1.0, math.pi / 2)
+    one.AddWing(U.RectGenerator(), m, 1.0, 4.0, 1, cols)
+    one.set_forward_flight([-1.0, 0.0, 0.0])
+    one.set_advection("euler")
+    ref = one.Run(steps - 1, 0.15)
+    one.close()
+    tol = 1e-9 if precision == "fp64" else 1e-6
+    for k in (0, 39):
+        assert np.max(np.abs(rows[:, k, 1:] - ref[:, 1:])) <= tol * np.max(np.abs(ref[:, 1:]))

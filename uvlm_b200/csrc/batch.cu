@@ -1309,6 +1309,7 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   want(&d_tiles, n_tiles);
   want(reinterpret_cast<char**>(&d_rec), (size_t)tot_rec * (mixed() ? sizeof(RecF) : sizeof(RecD)));
   // partial sums: the largest stage at the last step bounds every step
+  long long partial_of[2] = {0, 0};  // fine, coarse
   {
     const long long s = cfg.max_steps - 1;
     std::vector<NBodyBatchInput> in(n);
@@ -1330,10 +1331,10 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
         }
         in[c] = x;
       }
-      partial_cap = std::max(partial_cap, nbody_batch_partial_doubles(prec(), in.data(), n));
+      for (int k = 0; k < 2; ++k)
+        partial_of[k] = std::max(partial_of[k], nbody_batch_partial_doubles(prec(), in.data(), n, k == 1));
     }
   }
-  want(&d_partial, partial_cap);
   want(&d_in, n);
   want(&d_plan, n);
   want(&d_totals, 4);
@@ -1344,10 +1345,24 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
   want(&d_refac, 1);
   want(&d_res, n);
   want(&d_loads, (size_t)cfg.max_steps * n * 3);
+  want(&d_partial, 1);
 
-  size_t bytes = 0;
-  for (const auto& w : wanted) bytes += (w.second + 255) & ~(size_t)255;
-  UVLM_CUDA_TRY(cudaMalloc(&block, bytes));
+  // coarse where the fine partial sums are large, or do not fit
+  bool coarse = sizeof(double) * partial_of[0] > kBatchFineBytes;
+  auto allocate = [&]() -> cudaError_t {
+    partial_cap = partial_of[coarse];
+    wanted.back().second = sizeof(double) * (size_t)std::max(partial_cap, 1LL);
+    size_t bytes = 0;
+    for (const auto& w : wanted) bytes += (w.second + 255) & ~(size_t)255;
+    return cudaMalloc(&block, bytes);
+  };
+  cudaError_t got = allocate();
+  if (got == cudaErrorMemoryAllocation && !coarse) {
+    cudaGetLastError();
+    coarse = true;
+    got = allocate();
+  }
+  UVLM_CUDA_TRY(got);
   char* at = static_cast<char*>(block);
   for (const auto& w : wanted) {
     *w.first = at;
@@ -1391,6 +1406,7 @@ Error uvlm_batch::alloc(const uvlm_batch_case* cases) {
     }
   }
   nb_grids = nbody_batch_grids(prec(), num_sms);
+  nb_grids.coarse = coarse;
   grid = num_sms * 8;
   // the copies and fills above are the default stream's, the steps `st`'s
   UVLM_CUDA_TRY(cudaStreamSynchronize(nullptr));

@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) nbody_kernel(Blocks B, long long 
 template <int H, int TPC>
 __global__ void __launch_bounds__(256) batch_plan_kernel(const NBodyBatchInput* __restrict__ in, int n,
                                                          NBodyBatchPlan* __restrict__ plan, long long partial_cap,
-                                                         long long* totals, int* status) {
+                                                         bool coarse, long long* totals, int* status) {
   __shared__ long long sh[3][256];
   __shared__ long long carry[3];
   if (threadIdx.x < 3) carry[threadIdx.x] = 0;
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(256) batch_plan_kernel(const NBodyBatchInput* 
       p.tgt_off = x.tgt_off;
       p.n_tgt = x.n_tgt;
       p.tiles = (p.n_tgt + TPC - 1) / TPC;
-      p.splits = (p.n_strips + kBatchStripsPerItem - 1) / kBatchStripsPerItem;
+      p.splits = batch_splits(p.n_strips, x.blocks, x.n_blocks, coarse);
       v[0] = p.tiles * p.splits;
       v[1] = p.splits * 3 * p.n_tgt;
       v[2] = p.n_tgt;
@@ -982,7 +982,7 @@ const char* nbody_batch_tile_name(NBodyPrec prec, int tile) {
   return (tile >= 0 && tile < kNumBatchTilesF) ? names[tile] : "?";
 }
 
-long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in, int n) {
+long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in, int n, bool coarse) {
   // the bound of every tile the batch may run (the fewest rows per strip
   // make the most strips, hence the most source splits)
   long long worst = 0;
@@ -993,7 +993,7 @@ long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in,
     for (int c = 0; c < n; ++c) {
       PartBlocks B{};
       const long long strips = fill_parts(B, in[c].blocks, in[c].n_blocks, H, kMaxParts);
-      const long long splits = (strips + kBatchStripsPerItem - 1) / kBatchStripsPerItem;
+      const long long splits = batch_splits(strips, in[c].blocks, in[c].n_blocks, coarse);
       total += splits * 3 * in[c].n_tgt;
     }
     worst = std::max(worst, total);
@@ -1015,8 +1015,8 @@ int batch_grid_of(int num_sms) {
 template <class T, class Rec, int h, int TPT>
 Error batch_eval(const NBodyBatchInput* d_in, int n, const double* tx, const double* ty, const double* tz,
                  const void* records, double* partial, long long partial_cap, NBodyBatchPlan* d_plan,
-                 long long* d_totals, int* status, int grid, cudaStream_t st) {
-  batch_plan_kernel<h * LaneOf<T>::kLanes, kBatchBlock * TPT><<<1, 256, 0, st>>>(d_in, n, d_plan, partial_cap,
+                 long long* d_totals, int* status, bool coarse, int grid, cudaStream_t st) {
+  batch_plan_kernel<h * LaneOf<T>::kLanes, kBatchBlock * TPT><<<1, 256, 0, st>>>(d_in, n, d_plan, partial_cap, coarse,
                                                                                  d_totals, status);
   UVLM_LAUNCH_CHECK();
   batch_nbody_kernel<T, Rec, h, TPT, kBatchBlock, kBatchMinB>
@@ -1045,7 +1045,8 @@ Error nbody_batch_eval(NBodyPrec prec, const NBodyBatchInput* d_in, int n, const
                        const NBodyBatchGrids& grids, cudaStream_t st) {
   if (n <= 0) return ok();
   auto run = [&](auto eval, int grid) -> Error {
-    UVLM_TRY(eval(d_in, n, tx, ty, tz, records, partial, partial_cap, d_plan, d_totals, status, grid, st));
+    UVLM_TRY(eval(d_in, n, tx, ty, tz, records, partial, partial_cap, d_plan, d_totals, status, grids.coarse, grid,
+                  st));
     batch_reduce_kernel<<<grid, 256, 0, st>>>(d_plan, n, d_totals, partial, vx, vy, vz);
     UVLM_LAUNCH_CHECK();
     return ok();

@@ -309,10 +309,26 @@ struct SplitTable {
 // Many independent problems in one persistent launch: problem c has its own
 // source blocks (records already built) and targets [tgt_off, tgt_off+n_tgt)
 // of the shared SoA target arrays; its velocities land at the same indices.
-// Work items = (problem, target tile, source split) with at most
-// kBatchStripsPerItem strips each; every CTA strides over the items, so the
-// launch shape is fixed while the problem sizes change from step to step.
-constexpr int kBatchStripsPerItem = 3;
+// Work items = (problem, target tile, source split); every CTA strides over the
+// items, so the launch shape is fixed while the problem sizes change from step
+// to step.  A split takes kBatchStripsPerItem strips.  Each split stores a
+// partial sum per target, which on long wakes in FP64 is up to 2.6 times what
+// one split per kBatchRowsPerSplit node rows and 64 columns takes (265 MB for a
+// 64-column case of 1000 steps, 100 so): a batch whose partial sums would pass
+// kBatchFineBytes has no more than that (`coarse`; 3 cases of 300 steps then
+// take 1680 ms, 1653 else).
+constexpr int kBatchStripsPerItem = 3, kBatchRowsPerSplit = 16, kBatchManySplits = 8;
+constexpr long long kBatchFineBytes = 1LL << 30;
+__host__ __device__ inline long long batch_splits(long long strips, const SourceBlock* blocks, int n_blocks,
+                                                  bool coarse) {
+  const long long fine = (strips + kBatchStripsPerItem - 1) / kBatchStripsPerItem;
+  if (!coarse) return fine;
+  long long rows = 0;
+  for (int i = 0; i < n_blocks; ++i) rows += (long long)blocks[i].num * blocks[i].node_rows * ((blocks[i].cols + 63) / 64);
+  long long most = (rows + kBatchRowsPerSplit - 1) / kBatchRowsPerSplit;
+  if (most < kBatchManySplits) most = kBatchManySplits;
+  return fine < most ? fine : most;
+}
 
 struct NBodyBatchInput {
   SourceBlock blocks[2];
@@ -327,7 +343,7 @@ struct NBodyBatchPlan {
 };
 
 // Upper bound of the partial-sum doubles for the given inputs (host copy).
-long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in, int n);
+long long nbody_batch_partial_doubles(NBodyPrec prec, const NBodyBatchInput* in, int n, bool coarse);
 // Persistent grid sizes used by nbody_batch_eval on this device, and the
 // FP32 tile (strip height) the batch runs: tiles[t] is the grid of tile t.
 constexpr int kNumBatchTilesF = 3;
@@ -335,6 +351,7 @@ struct NBodyBatchGrids {
   int fp64 = 0;
   int tiles[kNumBatchTilesF] = {0, 0, 0};
   int tile = 0;
+  bool coarse = false;  // batch_splits
 };
 const char* nbody_batch_tile_name(NBodyPrec prec, int tile);
 NBodyBatchGrids nbody_batch_grids(NBodyPrec prec, int num_sms);
