@@ -277,3 +277,24 @@ def test_fp32_sums_are_short_on_narrow_sheets(tile, h):
     bound = 2 * u * np.sqrt(terms * ((cols * h) ** 2 / 9 + 16))
     print(f"{tile}: rms error {rms / u:.0f} u terms, bound {bound / u:.0f}")
     assert rms <= bound
+
+
+@pytest.mark.parametrize("shape,n", [((1, 1, 3), 220000), ((1, 2, 4), 95325), ((1, 2, 4), 95326), ((1, 8, 36), 3382),
+                                     ((1, 8, 36), 3383), ((1, 6, 64), 30001), ((3, 5, 9), 12345), ((1, 21, 22), 17000),
+                                     ((1, 21, 23), 17000), ((1, 15, 70), 9000)])
+def test_unordered_points_at_the_edges_of_the_tile_rule(shape, n):
+    """Point sets on both sides of 2^21 pairs and of 1000 segments, and sheets whose node rows fill strips of 2, 3 or 4
+    rows differently, against the oracle; tolerances as above."""
+    import pyoracle as o
+
+    import uvlm_b200 as U
+
+    pos, gamma = _sheet(*shape, seed=n, wobble=0.003)
+    t = _targets(pos, seed=n)
+    x = np.tile(t, (n // len(t) + 1, 1))[:n]
+    ref = o.sheet_induced_velocity(pos, gamma, t)
+    ref = np.tile(ref, (n // len(t) + 1, 1))[:n]
+    scale, mag = np.max(np.abs(ref)), np.linalg.norm(ref, axis=1)
+    assert np.max(np.abs(U.InducedVelocity(x, pos, gamma) - ref)) <= 1e-12 * scale
+    got = U.InducedVelocity(x, pos, gamma, precision="mixed")
+    assert np.all(np.abs(got - ref).max(axis=1) <= 2e-5 * mag + 1e-6 * scale)

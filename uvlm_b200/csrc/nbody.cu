@@ -769,8 +769,9 @@ SplitTable make_splits(long long tiles, long long n_strips, long long resident, 
 
 // Equal splits (the tiles that walk no parts): the number that ends first, a
 // whole number of waves of `resident` CTAs at a time, each taking its strips
-// plus about a third of one.
-long long choose_splits(long long tiles, long long n_strips, long long resident, long long most) {
+// plus about a third of one.  cost (where set): the time in strips.
+long long choose_splits(long long tiles, long long n_strips, long long resident, long long most,
+                        double* cost_out = nullptr) {
   most = std::max(1LL, std::min(most, std::min(n_strips, (long long)kMaxSplits)));
   long long best = 1;
   double best_cost = 1e300;
@@ -782,6 +783,7 @@ long long choose_splits(long long tiles, long long n_strips, long long resident,
       best = s;
     }
   }
+  if (cost_out) *cost_out = best_cost;
   return best;
 }
 
@@ -1342,16 +1344,39 @@ __global__ void split_points_kernel(const double* __restrict__ a, long long n, d
 
 size_t nbody_order_bytes(long long n_targets) { return (size_t)n_targets * 12 + 16; }
 
-// The rule, from shuffled points in and around wakes of 30 to 50,000 segments.
-// FP64: the far walkers for any set, in order from 2^24 pairs and 800 segments
-// per target on (below, the ordering costs more than it gives: 12 x 16 rings and
-// 60,000 points, 144 us as given, 180 in order; 60 x 60 and 3000, 116 and 106).
-// FP32: in order from 2^27 pairs and 2000 segments on (3 x 61 x 47 rings and 9001
-// points, 325 us as given, 227 in order).  Below, the far walkers' set-up and
-// their divergence outweigh their cheaper pairs, and the near walker takes every
-// pair (4500 points: 183 us far as given, 144 in order, 132 near), with fewer rows
-// per strip where strips are few (400 points, 50 x 50 rings: 34 us, 38 otherwise).
-constexpr int kNearVariantF32 = 13, kNearVariantSmallF32 = 14;  // fp32_h3_t2_b128_x2, fp32_h2_t2_b128_x2
+// The rule, from shuffled points in and around sheets of 22 to 50,000 segments.
+// In order, by the far walkers: FP64 from 2^24 pairs and 1000 segments per target
+// on (60 x 60 rings and 3000 points, 106 us in order; 20 x 20 and 60,000, 243 in
+// order, 224 by the near walker), FP32 from 2^27 pairs and 2000 segments on
+// (3 x 61 x 47 rings and 9001 points, 325 us as given, 227 in order).  Below,
+// points in any order leave the far walkers little and cost them their set-up
+// and divergence, and the near walkers take every pair: FP64 8 x 36 rings and
+// 200,000 points 678 us far, 516 near; but below 2^21 pairs the far walkers'
+// narrower strips fill more of the device (8 x 36 and 180 points: 27 us, 37).
+constexpr int kNearVariantF64 = 9;  // fp64_h2_t1_b128_m3
+
+// FP32 near tile for unordered points: the rows per strip whose strips end
+// first, 3 where the others gain less than 3 %.  A strip costs about its padded
+// rows and the row below: 7 node rows take 388 us in three strips of 3, 355 in two of 4
+// (250,000 points, 64 columns); few points want the most strips (400 points,
+// 50 x 50 rings: 31, 36 and 44 us with 2, 3 and 4 rows).
+int near_variant_f32(const SourceBlock* blocks, int n_blocks, long long n_targets, int num_sms) {
+  constexpr int kRows[3] = {2, 3, 4}, kVariant[3] = {14, 13, 12};  // fp32_h*_t2_b128_x2
+  const long long tiles = (n_targets + 255) / 256;
+  int best = 0;
+  double best_cost = 1e300;
+  for (int i = 0; i < 3; ++i) {
+    Blocks B{};
+    double cost = 0;
+    choose_splits(tiles, fill_blocks(B, blocks, n_blocks, kRows[i]), 3LL * num_sms, kMaxSplits, &cost);
+    cost *= (kRows[i] + 1) * (kRows[i] == 3 ? 0.97 : 1.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = i;
+    }
+  }
+  return kVariant[best];
+}
 
 Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec, const double* targets,
                         long long n_targets, double* out, NBodyWork* work, double* soa, void* order, int num_sms,
@@ -1364,7 +1389,7 @@ Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
   }
   double *tx = soa, *ty = soa + n_targets, *tz = soa + 2 * n_targets;
   const bool f32 = prec == kNBodyFP32;
-  const bool sort = n_targets < (1 << 30) && segs >= (f32 ? 2000 : 800) &&
+  const bool sort = n_targets < (1 << 30) && segs >= (f32 ? 2000 : 1000) &&
                     segs >= (1LL << (f32 ? 27 : 24)) / n_targets;
   NBodyWork w = *work;
   w.aos = out;
@@ -1380,9 +1405,9 @@ Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
     split_points_kernel<<<blocks_n, 256, 0, st>>>(targets, n_targets, tx, ty, tz);
   }
   UVLM_LAUNCH_CHECK();
-  const int variant = !f32 ? kDefaultVariantF64
-                      : sort ? kDefaultVariantF32
-                      : segs >= (1LL << 24) / n_targets ? kNearVariantF32 : kNearVariantSmallF32;
+  int variant = f32 ? kDefaultVariantF32 : kDefaultVariantF64;
+  if (!sort && f32) variant = near_variant_f32(blocks, n_blocks, n_targets, num_sms);
+  if (!sort && !f32 && segs >= (1LL << 21) / n_targets) variant = kNearVariantF64;
   return nbody_eval(blocks, n_blocks, prec, tx, ty, tz, n_targets, nullptr, nullptr, nullptr, &w, variant, num_sms,
                     st);
 }
