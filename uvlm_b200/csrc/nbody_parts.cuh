@@ -669,7 +669,10 @@ constexpr int kBlockCols = 8;  // segment columns of a block of a near part
 // bodies here, for the first, the inner and the two kinds of last column, made
 // near parts 1.3 times slower): before the first column stand nodes marked as
 // cut, and the last one's chordwise strengths are zero where it does not own
-// them.
+// them.  The body is there twice, so that a column's nodes become the previous
+// ones without copies: four wings of 16 x 64 at 300 wake rows, advection of a
+// step 27.8 -> 26.1 ms (26.8 before the parts), 32 x 128 at 400 rows 8.98 -> 8.69;
+// three times: 26.3 and 8.88; 4 rows at a time instead: 27.3 and 8.77.
 template <int HN>
 __device__ __forceinline__ void walk_near2(const RecF* base, int stride, int nr, int nc, bool last_h,
                                            const Tgt<float> (&tg)[2], float2 (&acc)[3]) {
@@ -682,7 +685,7 @@ __device__ __forceinline__ void walk_near2(const RecF* base, int stride, int nr,
     ps0[r] = SegV<float>{0.f, 0.f, 0.f};
     pgS[r] = 0.f;
   }
-#pragma unroll 1
+#pragma unroll 2
   for (int j = 0; j < nc; ++j) {
     const RecF* col = base + j;
     const float own = j < nc - 1 || last_h ? 1.f : 0.f;
