@@ -1355,27 +1355,21 @@ size_t nbody_order_bytes(long long n_targets) { return (size_t)n_targets * 12 + 
 // narrower strips fill more of the device (8 x 36 and 180 points: 27 us, 37).
 constexpr int kNearVariantF64 = 9;  // fp64_h2_t1_b128_m3
 
-// FP32 near tile for unordered points: the rows per strip whose strips end
-// first, 3 where the others gain less than 3 %.  A strip costs about its padded
-// rows and the row below: 7 node rows take 388 us in three strips of 3, 355 in two of 4
-// (250,000 points, 64 columns); few points want the most strips (400 points,
-// 50 x 50 rings: 31, 36 and 44 us with 2, 3 and 4 rows).
-int near_variant_f32(const SourceBlock* blocks, int n_blocks, long long n_targets, int num_sms) {
-  constexpr int kRows[3] = {2, 3, 4}, kVariant[3] = {14, 13, 12};  // fp32_h*_t2_b128_x2
+// FP32 near tile: the rows per strip whose strips end first, 3 where 2 gain less
+// than 3 % (4 would sum more segments in FP32).  A strip costs about its padded
+// rows and the row below: 7 node rows take 352 us in three strips of 3, 298 in
+// four of 2 (200,000 points, 64 columns); few points want the most strips (400
+// points, 50 x 50 rings: 31 and 36 us with 2 and 3 rows).
+int nbody_near_variant_f32(const SourceBlock* blocks, int n_blocks, long long n_targets, int num_sms) {
+  constexpr int kVariant[2] = {14, 13};  // fp32_h2_t2_b128_x2, fp32_h3_t2_b128_x2
   const long long tiles = (n_targets + 255) / 256;
-  int best = 0;
-  double best_cost = 1e300;
-  for (int i = 0; i < 3; ++i) {
+  double cost[2];
+  for (int i = 0; i < 2; ++i) {
     Blocks B{};
-    double cost = 0;
-    choose_splits(tiles, fill_blocks(B, blocks, n_blocks, kRows[i]), 3LL * num_sms, kMaxSplits, &cost);
-    cost *= (kRows[i] + 1) * (kRows[i] == 3 ? 0.97 : 1.0);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = i;
-    }
+    choose_splits(tiles, fill_blocks(B, blocks, n_blocks, i + 2), 3LL * num_sms, kMaxSplits, &cost[i]);
+    cost[i] *= i + 3;
   }
-  return kVariant[best];
+  return kVariant[cost[0] < 0.97 * cost[1] ? 0 : 1];
 }
 
 Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec, const double* targets,
@@ -1406,7 +1400,7 @@ Error nbody_eval_points(const SourceBlock* blocks, int n_blocks, NBodyPrec prec,
   }
   UVLM_LAUNCH_CHECK();
   int variant = f32 ? kDefaultVariantF32 : kDefaultVariantF64;
-  if (!sort && f32) variant = near_variant_f32(blocks, n_blocks, n_targets, num_sms);
+  if (!sort && f32) variant = nbody_near_variant_f32(blocks, n_blocks, n_targets, num_sms);
   if (!sort && !f32 && segs >= (1LL << 21) / n_targets) variant = kNearVariantF64;
   return nbody_eval(blocks, n_blocks, prec, tx, ty, tz, n_targets, nullptr, nullptr, nullptr, &w, variant, num_sms,
                     st);

@@ -378,6 +378,9 @@ const char* nbody_variant_name(int v);
 // on long wakes the autotuner chooses).
 constexpr int kDefaultVariantF32 = 17, kDefaultVariantF64 = 18;  // fp32_h2_t2_b128_x2f, fp64_h2_t1_b128_m3f
 
+// The FP32 near tile for an evaluation of few pairs, or of points in no order.
+int nbody_near_variant_f32(const SourceBlock* blocks, int n_blocks, long long n_targets, int num_sms);
+
 // Build the source records of `n_views` sheets into work.records (blocks are
 // appended in order) and fill blocks[].  Returns total records.
 Error nbody_build_sources(const SheetView* views, int n_views, NBodyPrec prec,
