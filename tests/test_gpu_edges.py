@@ -257,3 +257,30 @@ def test_simulators_do_not_see_a_busy_default_stream():
         th.join()
     for a, b in zip(got, want + want):
         np.testing.assert_array_equal(a, b)
+
+
+def test_small_mixed_evaluations_take_the_near_tiles():
+    """FP32 stages below 2^25 pairs run a near tile (2 or 3 rows), unless one is pinned or their near pairs are FP64; the
+    loads are those of the pinned part walker to the mixed tolerance."""
+    import uvlm_b200 as U
+
+    names = [U.lib().uvlm_nbody_variant_name(v).decode() for v in range(64)]
+    near, far = ("fp32_h2_t2_b128_x2", "fp32_h3_t2_b128_x2"), "fp32_h2_t2_b128_x2f"
+
+    def run(**kw):
+        sim = U.SimpleSimulator(precision="mixed", **kw)
+        sim.AddWing(U.RectGenerator(), U.Morphing().set_alpha(0.08).set_plug(0.1, 1.0), 1.0, 4.0, 6, 12)
+        sim.set_forward_flight([-1.0, 0.0, 0.0])
+        sim.set_advection("RK2")
+        loads = sim.Run(20, 0.12)
+        tiles = [names[v] for v in sim.stats().stage_variant[:3]]
+        sim.close()
+        return loads[:, 1:], tiles
+
+    loads, tiles = run()
+    assert tiles[0].endswith("x2f") and tiles[1] in near and tiles[2] in near, tiles
+    pinned, tiles = run(nbody_variant=names.index(far))
+    assert tiles == [far] * 3
+    _, tiles = run(near_fp64=True)
+    assert all(t.endswith("x2f") for t in tiles), tiles
+    assert np.max(np.abs(loads - pinned)) <= 1e-6 * np.max(np.abs(pinned))

@@ -111,6 +111,7 @@ struct uvlm_ctx {
                              {kDefaultVariantF32, kDefaultVariantF64},
                              {kDefaultVariantF32, kDefaultVariantF64}};
   bool stage_pinned[3][2] = {};        // the configuration chose the tile
+  int stage_ran[3] = {-1, -1, -1};      // the tile of the stage's last evaluation
   double stage_tuned_pairs[3][2] = {};  // pairs of the evaluation the tile was tuned on (0: not yet)
   // learned warm start: network (borrowed), per-step features, collected data
   uvlm_mlp* mlp = nullptr;
@@ -296,6 +297,8 @@ Error uvlm_ctx::build_sources(bool with_bound, const double* wake_pos_buf, NBody
   return nbody_build_sources(views, nv, prec, &nb, blocks, st);
 }
 
+constexpr double kNearPairs = 1 << 25;
+
 Error uvlm_ctx::eval(const SourceBlock* blocks, int nblocks, long long nt, NBodyPrec prec, int stage) {
   const double pairs = (double)nt * (double)nbody_unique_segments(blocks, nblocks);
   work_nbody += pairs;
@@ -338,10 +341,18 @@ Error uvlm_ctx::eval(const SourceBlock* blocks, int nblocks, long long nt, NBody
     UVLM_CUDA_TRY(cudaMemsetAsync(d_vz, 0, sizeof(double) * nt, st));
     return ok();
   }
-const bool rec = timing && nbev_n < kNbEvents;
+  // few FP32 pairs: the part walkers' set-up costs more than their cheaper pairs
+  // give (advection of a step, both evaluations, near and part walkers: 8 x 16
+  // and 50 wake rows 80 and 92 us, 4 x 8 x 24 and 20 rows 121 and 131; 16 x 64 and
+  // 100 rows, 98 million pairs, 353 and 319); with FP64 near pairs they stay
+  int run = chosen;
+  if (prec == kNBodyFP32 && !nb.near64 && !stage_pinned[stage][pi] && pairs < kNearPairs)
+    run = nbody_near_variant_f32(blocks, nblocks, nt, num_sms);
+  stage_ran[stage] = run;
+  const bool rec = timing && nbev_n < kNbEvents;
   if (rec) UVLM_CUDA_TRY(cudaEventRecord(nbev[2 * nbev_n], st));
   const Error e = nbody_eval(blocks, nblocks, prec, d_tx, d_ty, d_tz, nt, d_vx, d_vy, d_vz, &nb,
-                             chosen, num_sms, st);
+                             run, num_sms, st);
   if (rec) {
     UVLM_CUDA_TRY(cudaEventRecord(nbev[2 * nbev_n + 1], st));
     ++nbev_n;
@@ -694,13 +705,17 @@ Error uvlm_ctx::stage_advect(double* row) {
   last.t = t;
   last.wake_rows = wake_rings();
   {
-    const int pm = mixed() ? 0 : 1;
-    last.nbody_variant = stage_variant[kStageAdvect][pm];
-    last.stage_variant[0] = stage_variant[kStageRhs][stage_prec(UVLM_STAGE_RHS) == kNBodyFP64 ? 1 : 0];
-    last.stage_variant[1] = stage_variant[kStageLoads][stage_prec(UVLM_STAGE_LOADS) == kNBodyFP64 ? 1 : 0];
-    last.stage_variant[2] = stage_variant[kStageAdvect][stage_prec(UVLM_STAGE_ADVECT) == kNBodyFP64 ? 1 : 0];
+    // the tiles that ran; before a stage's first evaluation the one it would start with
+    auto tile = [&](int stage, int bit) {
+      return stage_ran[stage] >= 0 ? stage_ran[stage] : stage_variant[stage][stage_prec(bit) == kNBodyFP64 ? 1 : 0];
+    };
+    last.stage_variant[0] = tile(kStageRhs, UVLM_STAGE_RHS);
+    last.stage_variant[1] = tile(kStageLoads, UVLM_STAGE_LOADS);
+    last.stage_variant[2] = tile(kStageAdvect, UVLM_STAGE_ADVECT);
     last.stage_variant[3] = -1;
-    (void)pm;
+    last.nbody_variant = mixed() == (stage_prec(UVLM_STAGE_ADVECT) == kNBodyFP32)
+                             ? last.stage_variant[2]
+                             : stage_variant[kStageAdvect][mixed() ? 0 : 1];
   }
   if (timing) {
     float ms[8] = {0};
