@@ -370,3 +370,20 @@ def test_long_batches_whose_items_take_more_than_three_strips(precision, cols, s
     tol = 1e-9 if precision == "fp64" else 1e-6
     for k in (0, 39):
         assert np.max(np.abs(rows[:, k, 1:] - ref[:, 1:])) <= tol * np.max(np.abs(ref[:, 1:]))
+
+
+@pytest.mark.parametrize("n", [2, 37, 38, 49, 50, 74, 75, 149])
+def test_solve_clusters_of_every_size_give_the_same_bits(n):
+    """A residual row is the same sum whichever CTA of a cluster forms it: copies of one case, solved by clusters of 4,
+    3, 2 and 1 CTAs, against a batch of one: equal loads, sweeps and residuals, bit by bit."""
+    def run(copies):
+        sim = _small_batch(9, 10, copies, steps=5)
+        sim.run(5)
+        out = sim.loads()[:, :, 1:], *sim.solve_stats()
+        sim.close()
+        return out
+
+    (one, sweeps1, res1), (many, sweeps, res) = run(1), run(n)
+    np.testing.assert_array_equal(many, np.repeat(one, n, axis=1))
+    np.testing.assert_array_equal(sweeps, np.repeat(sweeps1, n))
+    np.testing.assert_array_equal(res, np.repeat(res1, n))

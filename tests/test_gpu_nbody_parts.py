@@ -298,3 +298,38 @@ def test_unordered_points_at_the_edges_of_the_tile_rule(shape, n):
     assert np.max(np.abs(U.InducedVelocity(x, pos, gamma) - ref)) <= 1e-12 * scale
     got = U.InducedVelocity(x, pos, gamma, precision="mixed")
     assert np.all(np.abs(got - ref).max(axis=1) <= 2e-5 * mag + 1e-6 * scale)
+
+
+PINNED = [("fp32_h2_t2_b128_x2f", ()), ("fp32_h3_t2_b128_x2f", ()), ("fp32_h4_t2_b128_x2f", ()),
+          ("fp32_h3_t2_b128_x2f", ("advect",)), ("fp64_h2_t1_b128_m3f", None), ("fp64_h3_t1_b128_m2f", None),
+          ("fp64_h2_t2_b128_f", None)]
+# (sheets, wake rows, columns, copies of the targets): remainders of 2, 4, 6 and 8 node rows and of 32 columns,
+# uneven parts, and enough targets that narrow parts share a strip (4 CTAs' worth of tiles times strips per slot)
+PINNED_SHAPES = [(1, 1, 2, 1), (5, 2, 6, 1), (2, 7, 8, 500), (1, 26, 16, 300), (1, 13, 34, 1), (2, 9, 66, 1),
+                 (1, 5, 130, 1), (1, 45, 2, 800)]
+
+
+@pytest.mark.parametrize("shape", PINNED_SHAPES)
+@pytest.mark.parametrize("tile,near", PINNED)
+def test_pinned_part_walkers_match_oracle(tile, near, shape):
+    """Every part walker at every target of _targets (nodes, all distances, both sides of the cut-off) against the
+    oracle, in both precisions, and in FP32 not the near tile's bits (the part walker has run)."""
+    import pyoracle as o
+
+    num, rows, cols, copies = shape
+    pos, gamma = _sheet(num, rows, cols, seed=rows + cols, wobble=0.004)
+    wing, wing_gamma = _sheet(num, 2, cols, seed=rows, wobble=0.002)
+    wing = wing - [0.31, 0.0, 0.0]
+    targets = _targets(pos, seed=5 + rows)
+    ref = o.sheet_induced_velocity(pos, gamma, targets) + o.sheet_induced_velocity(wing, wing_gamma, targets)
+    scale, mag = np.max(np.abs(ref)), np.linalg.norm(ref, axis=1)
+    many = np.tile(targets, (copies, 1))
+    fp64 = near is None
+    got = _velocity(pos, gamma, wing, wing_gamma, many, _variants()[tile], near or (), "fp64" if fp64 else "mixed",
+                    max_wake_rows=max(64, len(many) // (num * (cols + 1)) + 1))
+    bound = np.full(len(ref), 1e-12 * scale) if fp64 else 2e-5 * mag + 1e-6 * scale
+    err = np.abs(got.reshape(copies, -1, 3) - ref).max(axis=(0, 2))
+    assert np.all(err <= bound)
+    if not fp64:
+        plain = _velocity(pos, gamma, wing, wing_gamma, targets, _variants()["fp32_h3_t2_b128_x2"])
+        assert np.any(got[: len(ref)] != plain)

@@ -243,3 +243,20 @@ def test_mlp_gradients_at_tile_and_split_edges(n):
     g, loss = net.gradients(X, T)
     assert abs(loss - loss_ref) <= 1e-5 * abs(loss_ref)
     assert np.max(np.abs(g - g_ref)) <= 1e-4 * np.max(np.abs(g_ref))
+
+
+@pytest.mark.parametrize("n", [16, 31, 32, 33, 64, 4096])
+def test_mlp_gradients_at_inner_step_edges(n):
+    """Batches at the edges of the 32-row inner steps of the weight gradients, with the tolerances of the autograd
+    comparison."""
+    from uvlm_b200.warmstart import MLP
+
+    rng = np.random.default_rng(n)
+    net = MLP(seed=n)
+    X = rng.standard_normal((n, 8)).astype(np.float32)
+    T = (0.3 * rng.standard_normal(n)).astype(np.float32)
+    net.set_normalization(rng.standard_normal(8) * 0.1, 0.5 + rng.random(8), 0.7)
+    g_ref, loss_ref, _ = _torch_reference(net, X, T)
+    g, loss = net.gradients(X, T)
+    assert abs(loss - loss_ref) <= 1e-5 * abs(loss_ref)
+    assert np.max(np.abs(g - g_ref)) <= 1e-4 * np.max(np.abs(g_ref))
