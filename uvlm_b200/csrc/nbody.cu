@@ -720,7 +720,7 @@ constexpr Variant kVariants[] = {
     {"fp32_h4_t2_b128_x2", kNBodyFP32, 4, 2, 128, 3, 1},
     {"fp32_h3_t2_b128_x2", kNBodyFP32, 3, 2, 128, 3, 1},
     {"fp32_h2_t2_b128_x2", kNBodyFP32, 2, 2, 128, 3, 1},
-    {"fp32_h4_t2_b128_x2f", kNBodyFP32, 4, 2, 128, 3, 2},
+    {"fp32_h4_t2_b128_x2f", kNBodyFP32, 4, 2, 128, 2, 2},
     {"fp32_h3_t2_b128_x2f", kNBodyFP32, 3, 2, 128, 3, 2},
     {"fp32_h2_t2_b128_x2f", kNBodyFP32, 2, 2, 128, 3, 2},
     {"fp64_h2_t1_b128_m3f", kNBodyFP64, 2, 1, 128, 3, 2},

@@ -44,7 +44,7 @@ struct alignas(16) RecF {
   float4 hi;  // x_hi, y_hi, z_hi, gS/(4 pi)
   float4 lo;  // x_lo, y_lo, z_lo, gH/(4 pi)
   float4 sv;  // s0.x, s0.y, s0.z, h0.x
-  float4 hv;  // h0.y, h0.z, |s0|^2, |h0|^2 (squared lengths of the FP32 segment vectors)
+  float4 hv;  // h0.y, h0.z, 0, 0
 };
 struct alignas(16) RecD {
   double4 a;  // x, y, z, gS/(4 pi)
@@ -67,7 +67,6 @@ struct SheetView {
   const double* gamma;  // [n][rows_alloc][cols] with the same physical rows
   int g_rows_alloc, g_row0;
   int num, node_rows, cols;  // cols = rings per row (C)
-  int spanwise_only = 0;     // 1: chordwise strengths forced to zero
 };
 
 enum NBodyPrec { kNBodyFP64 = 0, kNBodyFP32 = 1 };
@@ -115,8 +114,7 @@ __device__ inline Rec build_record(const SheetView& v, long long k) {
   const double* p = v.pos + (((long long)n * v.rows_alloc + v.row0 + i) * C1 + j) * 3;
   const int R = v.node_rows - 1;
   const double gS = (j < v.cols) ? sheet_ring_gamma(v, n, i, j) - sheet_ring_gamma(v, n, i - 1, j) : 0.0;
-  const double gH =
-      (i < R && !v.spanwise_only) ? sheet_ring_gamma(v, n, i, j - 1) - sheet_ring_gamma(v, n, i, j) : 0.0;
+  const double gH = i < R ? sheet_ring_gamma(v, n, i, j - 1) - sheet_ring_gamma(v, n, i, j) : 0.0;
   double s0[3] = {0, 0, 0}, h0[3] = {0, 0, 0};
   if (j < v.cols)
     for (int d = 0; d < 3; ++d) s0[d] = p[3 + d] - p[d];
@@ -131,8 +129,7 @@ __device__ inline Rec build_record(const SheetView& v, long long k) {
     const float sx = (float)s0[0], sy = (float)s0[1], sz = (float)s0[2];
     const float ex = (float)h0[0], ey = (float)h0[1], ez = (float)h0[2];
     r.sv = make_float4(sx, sy, sz, ex);
-    r.hv = make_float4(ey, ez, (float)((double)sx * sx + (double)sy * sy + (double)sz * sz),
-                       (float)((double)ex * ex + (double)ey * ey + (double)ez * ez));
+    r.hv = make_float4(ey, ez, 0.f, 0.f);
   } else {
     r.a = make_double4(p[0], p[1], p[2], gS * s);
     r.b = make_double4(gH * s, s0[0], s0[1], s0[2]);
