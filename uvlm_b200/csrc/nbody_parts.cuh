@@ -40,10 +40,10 @@
 // and only the blocks that are closer still are left to the near walkers.  With
 // the near field in FP64, the pairs of every part that is not far are FP64.
 //
-// Bound: the FMA pipe (about 60 % busy in FP32) with the reciprocal unit at
-// about 45 %; 12 warps per SM.  Advection stage of an RK2 step, 52k targets x
+// Bound: the FMA pipe (65 % busy in FP32) with the reciprocal unit at 54 %; 12
+// warps per SM.  Advection stage of an RK2 step, 52k targets x
 // 111k segments, against a pairwise cut-off test and a cross product per
-// segment: FP32 10.41 -> 8.81 ms, FP64 (8 x 128 wing, 103k segments) 38.2 ->
+// segment: FP32 10.66 -> 8.69 ms, FP64 (8 x 128 wing, 103k segments) 38.2 ->
 // 20.6 ms; at a 50-row wake FP32 0.40 -> 0.40 ms, FP64 0.90 -> 0.59 ms.
 //
 // FP32: the two lanes of the sm_100 FP32x2 instructions hold two SOURCE rows
