@@ -261,7 +261,8 @@ enum {
   UVLM_ARITH_RSQRT = 0,        /* 1 / sqrt(x), FP64 N-body */
   UVLM_ARITH_RECIPROCAL = 1,   /* 1 / x, FP64 N-body */
   UVLM_ARITH_QUOTIENT = 2,     /* x / y, FP64 LU */
-  UVLM_ARITH_QUOTIENT_F32 = 3  /* x / y rounded to FP32, FP32 LU */
+  UVLM_ARITH_QUOTIENT_F32 = 3, /* x / y rounded to FP32, FP32 LU */
+  UVLM_ARITH_SQRT = 4          /* sqrt(x), FP64 N-body */
 };
 int uvlm_check_arithmetic(int32_t kind, const double* x, const double* y, int64_t n, double* out);
 /* Every bounded device-side wait of the library (the triangular solves'

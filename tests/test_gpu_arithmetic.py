@@ -1,10 +1,12 @@
-"""The FP64 reciprocal square root and reciprocal of the N-body kernels and the quotients of the LU against 80-bit
+"""The FP64 square root, its reciprocal and the reciprocal of the N-body kernels and the quotients of the LU against 80-bit
 arithmetic (B200).
 
 All three are formed from an approximation by steps of their own.  Bounds, in units in the last place:
   1/sqrt(x)  1.01: half a unit of the last rounding, half a unit of the rounding of x y in the residual, and the
              remainder of a third-order step from a seed of relative error 2^-20 (CUDA's rsqrt: 1);
   1/x        0.51: half a unit of the last rounding and the remainder 2^-60 (CUDA's: 0.5);
+  sqrt(x)    0.78: half a unit of the last rounding, half of the half unit of x y (it enters halved) and the
+             remainder;
   x/y        the correctly rounded quotient, as the division gives it.
 """
 import ctypes as C
@@ -15,7 +17,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 _P = C.POINTER(C.c_double)
-RSQRT, RECIPROCAL, QUOTIENT, QUOTIENT_F32 = range(4)
+RSQRT, RECIPROCAL, QUOTIENT, QUOTIENT_F32, SQRT = range(5)
 
 
 def _call(kind, x, y=None):
@@ -64,3 +66,14 @@ def test_lu_quotients(kind, dtype, low, high):
     np.testing.assert_array_equal(_call(kind, x, y).astype(dtype), x / y)
     assert np.all(_call(kind, x[:100], np.zeros(100)) == 0)
     assert np.all(np.isnan(_call(kind, x[:100], np.full(100, np.nan))))
+
+
+@pytest.mark.parametrize("low,high", [(-67, 40), (-1020, 1023)])
+def test_nbody_lengths(low, high):
+    rng = np.random.default_rng(high)
+    n = 1 << 20
+    x = _mantissas(rng, n) * 2.0 ** rng.integers(low, high, n)
+    x[:2] = 2.0 ** low, (2 - 2.0 ** -52) * 2.0 ** (high - 1)
+    ref = np.sqrt(x.astype(np.longdouble))
+    err = np.abs((_call(SQRT, x) - ref) / np.spacing(ref.astype(np.float64)))
+    assert float(err.max()) <= 0.78

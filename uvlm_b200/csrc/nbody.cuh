@@ -408,9 +408,10 @@ Error rings_eval(const double* rings, const double* gamma, long long n_rings, bo
                  const double* targets, long long n_targets, const double* add3, const double* base, double scale,
                  double* partial, double* out, int num_sms, cudaStream_t st);
 
-// out[k] = nb_rsqrt(x[k]) (recip = false) or nb_rcp(x[k]), the FP64 forms of
-// the N-body kernels; device arrays.
-Error nbody_arithmetic(bool recip, const double* x, long long n, double* out, cudaStream_t st);
+// out[k] = nb_rsqrt(x[k]), nb_rcp(x[k]) or nb_sqrt(x[k]), the FP64 forms of the
+// N-body kernels; device arrays.
+enum NBodyArith { kNBodyRsqrt, kNBodyRcp, kNBodySqrt };
+Error nbody_arithmetic(NBodyArith f, const double* x, long long n, double* out, cudaStream_t st);
 
 // Algorithmic unique-segment count of a set of blocks (for the roofline).
 long long nbody_unique_segments(const SourceBlock* blocks, int n_blocks);

@@ -414,7 +414,7 @@ int uvlm_lu_factor_f32(const float* A, int64_t n, int32_t update, float* LU, int
 
 int uvlm_check_arithmetic(int32_t kind, const double* x, const double* y, int64_t n, double* out) {
   const bool quotient = kind == UVLM_ARITH_QUOTIENT || kind == UVLM_ARITH_QUOTIENT_F32;
-  if (kind < UVLM_ARITH_RSQRT || kind > UVLM_ARITH_QUOTIENT_F32 || n < 0 || (n && (!x || !out || (quotient && !y))))
+  if (kind < UVLM_ARITH_RSQRT || kind > UVLM_ARITH_SQRT || n < 0 || (n && (!x || !out || (quotient && !y))))
     return report(fail(kErrInvalid, "invalid argument"));
   if (n == 0) return UVLM_OK;
   Scratch S;
@@ -426,7 +426,10 @@ int uvlm_check_arithmetic(int32_t kind, const double* x, const double* y, int64_
     if (quotient)
       UVLM_TRY(lu_quotients(kind == UVLM_ARITH_QUOTIENT_F32, dx, dy, n, dout, 0));
     else
-      UVLM_TRY(nbody_arithmetic(kind == UVLM_ARITH_RECIPROCAL, dx, n, dout, 0));
+      UVLM_TRY(nbody_arithmetic(kind == UVLM_ARITH_RECIPROCAL ? kNBodyRcp
+                                : kind == UVLM_ARITH_SQRT     ? kNBodySqrt
+                                                              : kNBodyRsqrt,
+                                dx, n, dout, 0));
     UVLM_CUDA_TRY(cudaMemcpy(out, dout, sizeof(double) * n, cudaMemcpyDeviceToHost));
     return ok();
   };
