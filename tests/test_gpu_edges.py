@@ -284,3 +284,39 @@ def test_small_mixed_evaluations_take_the_near_tiles():
     _, tiles = run(near_fp64=True)
     assert all(t.endswith("x2f") for t in tiles), tiles
     assert np.max(np.abs(loads - pinned)) <= 1e-6 * np.max(np.abs(pinned))
+
+
+@pytest.mark.parametrize("chordwise", [False, True])
+def test_shared_segments_of_equal_rings_cancel(chordwise):
+    """A lattice of rings of one circulation carries nothing on the segments inside it, and points 1e-4 away from
+    those see the boundary alone: both rings evaluate the segment alike.  Bound: the sum of each ring's terms, up to
+    v = g / (2 pi distance), rounds by at most half a unit each, eight terms; an evaluation from the other end would be
+    off by the length over the distance, 1e4 units."""
+    from uvlm_b200 import rings as R
+
+    rng = np.random.default_rng(4)
+    rows, cols, L = 5, 6, np.longdouble
+    i, j = np.meshgrid(np.arange(rows + 1), np.arange(cols + 1), indexing="ij")
+    p = np.stack([1.0 * i, 1.0 * j, 0 * i], -1) + 0.05 * rng.standard_normal((rows + 1, cols + 1, 3))
+    rings = np.stack([p[:-1, :-1], p[:-1, 1:], p[1:, 1:], p[1:, :-1]], 2).reshape(-1, 4, 3)
+    # inner segments along j (every ring's first and third) and, for whole rings, along i
+    a, b = [p[1:-1, :-1].reshape(-1, 3)], [p[1:-1, 1:].reshape(-1, 3)]
+    if not chordwise:
+        a, b = a + [p[:-1, 1:-1].reshape(-1, 3)], b + [p[1:, 1:-1].reshape(-1, 3)]
+    a, b = np.concatenate(a), np.concatenate(b)
+    side = np.cross(b - a, rng.standard_normal(a.shape))
+    x = a + (b - a) * rng.uniform(0.2, 0.8, (len(a), 1)) + side / np.linalg.norm(side, axis=1)[:, None] * 1e-4
+    got = R.InducedVelocity(x, rings, np.ones(len(rings)), chordwise=chordwise)
+    # the boundary, nodes[k + 1] -> nodes[k] of the rings on it
+    edges = [(p[0, k + 1], p[0, k]) for k in range(cols)] + [(p[rows, k], p[rows, k + 1]) for k in range(cols)]
+    if not chordwise:
+        edges += [(p[k, 0], p[k + 1, 0]) for k in range(rows)] + [(p[k + 1, cols], p[k, cols]) for k in range(rows)]
+    ref = np.zeros(x.shape, L)
+    for s, e in edges:
+        r1, r2 = x.astype(L) - s, x.astype(L) - e
+        n1, n2 = np.sqrt((r1 * r1).sum(1)), np.sqrt((r2 * r2).sum(1))
+        dot, d = (r1 * r2).sum(1), np.cross(r1, r2)
+        f = np.where(dot >= 0, (n1 + n2) / (n1 * n2 * (n1 * n2 + dot)), (n1 + n2) * (n1 * n2 - dot) / (n1 * n2 * (d * d).sum(1)))
+        ref += f[:, None] * d
+    ref /= 4 * L("3.14159265358979323846264338327950288")
+    assert float(np.max(np.abs(got - ref))) <= 8 * 2.0 ** -53 / (2 * np.pi * 1e-4)
